@@ -278,7 +278,7 @@ def sweep_bytes(m, modes_planes, reads_of_factor):
     return sum(reads_of_factor * m.nsolve * m.nband * 8 + 2 * 2 * P * m.nsolve * 8 for P in modes_planes)
 
 
-TILE_BYTES = 64 * 65 * 8   # one 64 x 64 band tile as stored (rows padded to 65)
+TILE_BYTES = 64 * 64 * 8   # one 64 x 64 band tile as stored
 
 
 def envelope_sweep_bytes(mesh, m, modes_planes):

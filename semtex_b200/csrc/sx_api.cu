@@ -27,8 +27,8 @@ BandSched sx_modal_s::sched(int nj) {
     if (it != sched_for.end()) {
       sc = it->second;
     } else {
-      // ranks 1..C-1 share the J-1 tiles j >= 2, so C <= J
-      sc.C = pick_cluster(nj, std::min(16, std::max(1, J)), 2, J + 2, &sc.S, forced_stages);
+      // ranks 1..C-1 share the J - 2 tiles j >= 3, so C <= J - 1
+      sc.C = pick_cluster(nj, std::min(16, std::max(1, J - 1)), J, &sc.S, forced_stages);
       sc.Q = default_lead(sc.C, J);
       sched_for[nj] = sc;
     }
@@ -724,7 +724,10 @@ extern "C" int sx_modal_autotune(sx_modal s, double *d_u, const double *d_f, con
     // (1) cluster size and ring depth, with the default leader share
     for (int S : {BAND_STAGES_MAX, 3, 2, 1})
       for (int C : {1, 2, 3, 4, 6, 8, 12, 16})
-        if (rc == SX_OK && C <= J && band_active_clusters(C, 2, J + 2, S) > 0)
+        if (rc == SX_OK && C <= J && band_active_clusters(C, J, S) > 0 &&
+            // one CTA a system has every tile on its chain: a candidate only
+            // where there are no others, or too many systems for two
+            (C > 1 || J < 3 || band_active_clusters(2, J, S) < nj))
           trial({{C, S, default_lead(C, J)}, inner0});
     // (2) the leader's share on the best of those: none, or the last of every
     // K positions for K = C + 1, C + 2, 2C
@@ -1035,7 +1038,7 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
   b->dkey.clear();
   std::vector<Job> jobs;
   std::vector<size_t> j0;
-  int maxJ = 1, maxP = 1, forced = 0, fstages = 0, flead = -1;
+  int maxJ = 1, forced = 0, fstages = 0, flead = -1;
   for (Part &q : parts) {
     j0.push_back(jobs.size());
     if (q.gd.empty()) continue;
@@ -1044,7 +1047,6 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
     for (auto &g : q.gd) {
       jobs.push_back(make_job(*q.s, g, slot, q.u, q.f, q.bc, q.stride, bcstride));
       maxJ = std::max(maxJ, jobs.back().J);
-      maxP = std::max(maxP, g.P);
       slot += g.P;
     }
     forced = std::max(forced, q.s->forced_cluster);
@@ -1059,8 +1061,8 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
   b->jobs = jobs;
   b->sc = BandSched();
   b->sc.C = forced > 0 ? forced
-                       : pick_cluster((int)jobs.size(), std::min(16, std::max(1, maxJ)), maxP <= 2 ? 2 : 8,
-                                      maxJ + 2, &b->sc.S, fstages);
+                       : pick_cluster((int)jobs.size(), std::min(16, std::max(1, maxJ - 1)), maxJ, &b->sc.S,
+                                      fstages);
   if (forced > 0 && fstages > 0) b->sc.S = fstages;
   b->sc.Q = flead >= 0 ? flead : default_lead(b->sc.C, maxJ);
   auto body = [&]() -> int {

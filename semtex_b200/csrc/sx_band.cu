@@ -1,28 +1,60 @@
-// sx_band.cu -- banded triangular solves U^T y = b, U x = y (LAPACK
-// dpbtrs "U" as called at src/field.cpp:609) on the tiled band factor.
+// sx_band.cu -- banded triangular solves (LAPACK dpbtrs "U" as called at
+// src/field.cpp:609) on the tiled band factor.
 //
-// Both sweeps are left-looking over block columns of NB rows:
-//   forward  y_k = D_k^T (b_k - sum_{j>=1} T(k,j)^T   y_{k-j})
-//   backward x_k = D_k   (y_k - sum_{j>=1} T(k+j,j)   x_{k+j})
-// with T(k,j) = U(rows of block k-j, cols of block k) and D_k = U_kk^-1.
+// The factor is held as the block LDL^T form of U^T U (sx_factor.cu): the
+// off-diagonal tiles are T(k, j) = U_bb^-1 U(rows of block b = k - j, cols of
+// block k), and D_k = U_kk^-1.  Both sweeps are left-looking over block
+// columns of NB rows and hold no diagonal solve on their chains:
+//   forward  z_k = b_k - sum_{j>=1} T(k,j)^T   z_{k-j}
+//   middle   w_k = D_k D_k^T z_k                       (independent per block)
+//   backward x_k = w_k - sum_{j>=1} T(k+j,j) x_{k+j}
 //
-// One thread-block cluster of C CTAs works on one system (all P right-hand
-// sides of the job at once).  The leader CTA (rank 0) owns the critical
-// path: the j = 1 tile (needs the block just solved) and D_k; ranks 1..C-1
-// own the older tiles j >= 2 round-robin, so they run ahead while the
-// leader finishes the previous block.  Tiles stream into each CTA through a
-// ring of 1-D TMA bulk copies (cp.async.bulk + mbarrier complete_tx).
-// Partial sums go to the leader over distributed shared memory; each solved
-// block goes to the RHS array in global memory (where it stays in L2), and
-// the leader's release at cluster scope on every rank's mbarrier for that
-// block lets the ranks fetch it from there (cp.async through L2, one block
-// per tile, issued under the previous tile's work).  Partials are combined
-// in rank order, so the result does not depend on timing.
+// One thread-block cluster of C CTAs works on one system (up to two
+// right-hand sides at once).  The block-column chain is what bounds a system:
+// nothing of step t + 1 can end before block t is known.  So the leader CTA
+// (rank 0) keeps the chain on one SM: it owns the tiles j <= 2, and a step of
+// its chain is the j = 1 tile's product, one reduction and one block barrier
+// (two forward), the j = 2 tile of the next step following off the chain.
+// Ranks 1..C-1 own the tiles j >= 3 and the D_k: what they multiply was solved
+// three steps earlier or more, which covers the way to another SM and back.  A solved block goes to every rank's window of the last blocks
+// by st.async (its mbarrier counts the bytes: no fence, no flag, no trip
+// through L2); the ranks' partial sums return to the leader the same way.
 //
-// Every wait is bounded (clock64); on timeout the kernel records
-// SX_ERR_TIMEOUT in the status word, drains its own bulk copies (bounded),
-// meets the other CTAs at a final cluster barrier and returns.
+// Tiles (32 KB, unpadded) stream into each CTA through a ring of 1-D TMA bulk
+// copies issued by a warp of their own; the eight working warps never meet
+// at a block barrier over a tile: each waits for the tile's mbarrier, reads
+// its eight rows (a warp reads 512 contiguous bytes of a row) and releases
+// the slot.  Forward, a lane keeps two columns and the warps' sums are added
+// in warp order; backward, a warp keeps eight rows and its lanes' sums are
+// added by shuffles, so the ranks run without block barriers.  Partials are
+// combined in rank order, so the result does not depend on timing.
+//
+// A tile costs an SM some 500-800 cycles: the copy writes its 32 KB into
+// shared memory, the warps read it back, and each warp reads the block it
+// multiplies, all through one 128-byte-a-cycle port.  So a block is kept in the
+// order in which a sweep's lanes read it without conflicts, and eight warps do
+// better than sixteen (each reads the whole block backward).  The leader's
+// step is two such tiles and about as long again in hand-offs.
+//
+// Measured (B200, 1965 MHz; both sweeps, the envelope's tiles twice), against
+// the previous form (y_k = D_k^T (b_k - ...) with D_k on the chain, blocks
+// fetched through L2 after a cluster-scope release, four block barriers a
+// step):
+//   32 systems, 236 block columns of 8.9 tiles   2.64 -> 0.78 ms, 5.99 TB/s
+//   12 systems, 1206 block columns of 22.5      15.85 -> 3.97 ms, 5.50 TB/s
+//   64 systems of that band                     24.9 -> 16.6 ms, 7.00 TB/s
+//   one system of the first kind                 (5.6 -> 1.47 us a block column)
+// With the leader owning j <= 3: 0.90 / 4.64 ms; with sixteen warps 0.82 /
+// 4.27 ms.  The first two are bound by the leader's chain (1.65 us a block
+// column), the third by HBM.
+//
+// Every wait is bounded (clock64).  When one runs out, the thread marks the
+// CTA as given up and goes on without waiting or sending: the control flow
+// depends on the tables alone, so every barrier is still met; the kernel
+// records SX_ERR_TIMEOUT, waits (bounded) for its own bulk copies, meets the
+// other CTAs at the final cluster barrier and returns.
 #include <algorithm>
+#include <type_traits>
 
 #include "sx_kernels.cuh"
 #include "sx_ptx.cuh"
@@ -31,7 +63,6 @@
 namespace sx {
 
 constexpr long long WAIT_LIMIT = SWEEP_WAIT_DEFAULT;  // ~2 s at 1.9 GHz
-
 
 // Cycles a wait of the sweep loop may take before the kernel gives up
 // (SX_ERR_TIMEOUT); per device, set by sx_set_wait_limit.  The drain of a
@@ -45,456 +76,540 @@ int set_sweep_wait_limit(long long cycles) {
   return SX_OK;
 }
 
-// Division by a small runtime divisor d (1 <= d <= 2^16) of n < 2^24 by one
-// 64-bit multiply: floor(n / d) = (n ceil(2^40 / d)) >> 40 exactly in that
-// range (the rounding error of the reciprocal stays below 2^-16 <= 1 / d).
-struct FastDiv {
-  unsigned long long m = 1ull << 40;
-  unsigned d = 1;
-  __host__ __device__ FastDiv() {}
-  __host__ __device__ explicit FastDiv(unsigned dv) : m(((1ull << 40) + dv - 1) / dv), d(dv) {}
-  __device__ __forceinline__ int div(int n) const { return (int)(((unsigned long long)(unsigned)n * m) >> 40); }
-  __device__ __forceinline__ int mod(int n) const { return n - div(n) * (int)d; }
-};
+namespace {
 
-struct SweepGeom {
-  int nblk, J, C, rank;
-  // Leader share: Q = 0, the leader (rank 0) owns only the j = 1 tile and
-  // D_k, and ranks 1..C-1 the tiles j >= 2 round-robin.  Q = K >= 2: the
-  // positions p = j - 2 of the tiles j >= 2 run in cycles of K whose last
-  // position is the leader's; the other positions go round-robin to ranks
-  // 1..C-1.  The leader works through its tiles of step t + 1 during step t,
-  // between its j = 1 tile and the wait for the ranks' partial sums, so they
-  // stay off the block-column chain; they are listed under step t, after
-  // the j = 1 tile and before D_k.
-  int Q;
-  FastDiv dC1, dQ, dQ1;  // divisions by C - 1, Q and Q - 1 (1 when unused)
-  // Envelope of the factor (null: the whole band): jf[k] tiles above the
-  // diagonal are non-zero in block column k, jb[k] right of it in block row
-  // k; every tile beyond them is an exact zero and is skipped.
-  const int *jf, *jb;
-  // off-diagonal tiles of step t (t < nblk: forward block t, else backward
-  // block 2 nblk - 1 - t)
-  __device__ __forceinline__ int jmax(int t) const {
-    if (t >= 2 * nblk) return 0;
-    if (t < nblk) {
-      const int b = min(J, t);
-      return jf ? max(0, min(b, __ldg(jf + t))) : b;
-    }
-    const int k = 2 * nblk - 1 - t, b = min(J, nblk - 1 - k);
-    return jb ? max(0, min(b, __ldg(jb + k))) : b;
-  }
-  // what a step's tile list depends on: its own tile count and the next
-  // step's (the leader's share of it); read once per step
-  struct Step {
-    int jm, jm1;
-  };
-  __device__ __forceinline__ Step step(int t) const { return Step{jmax(t), jmax(t + 1)}; }
-  // the leader's tiles of step t + 1, listed at step t
-  __device__ __forceinline__ int ahead_count(const Step &s) const { return dQ.div(max(s.jm1 - 1, 0)); }
-  // tiles j >= 2 of step t that are not the leader's
-  __device__ __forceinline__ int rank_positions(const Step &s) const {
-    const int npos = max(s.jm - 1, 0);
-    return Q == 0 ? npos : npos - dQ.div(npos);
-  }
-  // tiles owned by `rank` at a step; D_k is always last, on rank 0
-  __device__ __forceinline__ int count(const Step &s) const {
-    const int jm = s.jm;
-    if (C == 1) return jm + 1;
-    if (rank == 0) return (jm >= 1 ? 1 : 0) + (Q == 0 ? 0 : ahead_count(s)) + 1;
-    const int N = rank_positions(s);
-    return N > rank - 1 ? dC1.div(N - rank) + 1 : 0;
-  }
-  // j of the idx-th owned tile, in processing order: a rank's tiles j >= 2
-  // from the oldest block down; the leader's j = 1 tile, its tiles of step
-  // t + 1 from the oldest block down, then D_k (j = 0)
-  __device__ __forceinline__ int jat(const Step &s, int idx) const {
-    const int jm = s.jm;
-    if (C == 1) return idx < jm ? jm - idx : 0;
-    if (rank == 0) {
-      const int a = jm >= 1 ? 1 : 0;
-      if (idx < a) return 1;
-      if (Q == 0) return 0;
-      const int F1 = ahead_count(s), e = idx - a;
-      return e < F1 ? (F1 - 1 - e) * Q + (Q - 1) + 2 : 0;
-    }
-    const int N = rank_positions(s);
-    const int n = N > rank - 1 ? dC1.div(N - rank) + 1 : 0;
-    const int i = (rank - 1) + (n - 1 - idx) * (C - 1);
-    return (Q == 0 ? i : i + dQ1.div(i)) + 2;
-  }
-  // whether a tile j at step t is the leader's tile of step t + 1
-  __device__ __forceinline__ bool ahead(int j) const { return rank == 0 && C > 1 && Q > 0 && j >= 2; }
-};
+constexpr int SWP_WARPS = 8;                       // working warps
+constexpr int SWP_THREADS = (SWP_WARPS + 1) * 32;  // and the copying warp
+constexpr int RPW = NB / SWP_WARPS;                // rows of a tile a warp reads
+constexpr int VEC = 2 * NB;                        // a block of two right-hand sides, [row][plane]
+constexpr int LPE = SWP_WARPS * 32 / VEC;          // lanes that share an element of a block
+constexpr int RED = VEC + 2;                       // pitch of the warps' sums (lanes of an element on distinct banks)
+constexpr int NEAR = 2;                           // the leader's tiles: j <= NEAR
+constexpr int DLAG = NEAR + 1;                    // steps a D_k follows its block by, on the ranks
 
-__device__ __forceinline__ const double *tile_src(const Job &Jb, int t, int j) {
-  const int nblk = Jb.nblk;
-  const size_t J1 = Jb.J + 1;
-  if (t < nblk) {
-    const int k = t;
-    return j ? Jb.tiles + ((size_t)k * J1 + j) * TSZ : Jb.dinv + (size_t)k * TSZ;
-  }
-  const int k = 2 * nblk - 1 - t;
-  return j ? Jb.tiles + ((size_t)(k + j) * J1 + j) * TSZ : Jb.dinv + (size_t)k * TSZ;
+
+// Slots of the leader's buffer of partial sums: a rank runs at most this many
+// steps ahead of the leader.
+constexpr int DEPTH = 3;
+static_assert(NEAR + 1 == DEPTH, "the ranks' one wait a step covers their youngest tile");
+
+// Blocks in a CTA's window: every block a step multiplies (j <= J), and
+// those whose arrival a rank waits for before it reuses a partial's slot.
+__host__ __device__ __forceinline__ int window_blocks(int J) { return max(J, DEPTH) + 2; }
+
+// Doubles of the warps' sums and the leader's partial sums (see the kernel).
+__host__ __device__ __forceinline__ int red_doubles(int C) {
+  return SWP_WARPS * RED + max(SWP_WARPS * RED, DEPTH * (C - 1) * VEC);
 }
 
-// Two CTAs per SM for up to two planes (128 registers a thread), one for more.
-template <int PMAX>
-__global__ void __launch_bounds__(256, PMAX <= 2 ? 2 : 1)
+// This warp's rows of a tile, two columns a lane, and the values of the block
+// they meet: forward the rows' own, both planes side by side (the same in
+// every lane); backward the columns', plane by plane.  The window keeps each
+// sweep's blocks in the order its lanes read them.
+struct TileRegs {
+  double2 a[RPW], z[RPW];
+};
+template <bool FWD>
+__device__ __forceinline__ void tile_load(TileRegs &r, const double *T, const double *z, int w, int lane) {
+  const double2 *t2 = reinterpret_cast<const double2 *>(T) + w * RPW * (NB / 2) + lane;
+  const double2 *z2 = reinterpret_cast<const double2 *>(z) + (FWD ? w * RPW : lane);
+#pragma unroll
+  for (int i = 0; i < (FWD ? RPW : 2); i++) r.z[i] = z2[FWD ? i : i * (NB / 2)];
+#pragma unroll
+  for (int i = 0; i < RPW; i++) r.a[i] = t2[i * (NB / 2)];
+}
+// Forward: acc (two columns, two planes) += T^T z; backward: acc (the rows, two
+// planes) += this lane's columns of T times z.
+template <bool FWD>
+__device__ __forceinline__ void tile_fma(const TileRegs &r, double *acc) {
+#pragma unroll
+  for (int i = 0; i < RPW; i++) {
+    if (FWD) {
+      acc[0] = fma(r.a[i].x, r.z[i].x, acc[0]);
+      acc[1] = fma(r.a[i].x, r.z[i].y, acc[1]);
+      acc[2] = fma(r.a[i].y, r.z[i].x, acc[2]);
+      acc[3] = fma(r.a[i].y, r.z[i].y, acc[3]);
+    } else {
+      acc[2 * i] = fma(r.a[i].y, r.z[0].y, fma(r.a[i].x, r.z[0].x, acc[2 * i]));
+      acc[2 * i + 1] = fma(r.a[i].y, r.z[1].y, fma(r.a[i].x, r.z[1].x, acc[2 * i + 1]));
+    }
+  }
+}
+
+// Sums of a warp's 2 RPW values over its lanes, halving: lane l returns its
+// part of value l / LPE (the rest is with the other lanes of the LPE).
+__device__ __forceinline__ double lanes_reduce(const double *acc, int lane) {
+  double v[2 * RPW];
+#pragma unroll
+  for (int i = 0; i < 2 * RPW; i++) v[i] = acc[i];
+  int o = 16;
+#pragma unroll
+  for (int n = RPW; n >= 1; n /= 2) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; i++) v[i] = (up ? v[i + n] : v[i]) + __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + n], o);
+    o /= 2;
+  }
+  return v[0];
+}
+
+// The whole of an element from its lanes' parts, in each of them.
+__device__ __forceinline__ double lane_sum(double s) {
+#pragma unroll
+  for (int o = LPE / 2; o >= 1; o /= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// Off-diagonal tiles of step t (t < nblk: forward block t, else backward
+// block 2 nblk - 1 - t) inside the band and the factor's envelope.
+struct StepTab {
+  const int *jf, *jb;
+  int nblk, J;
+  // the envelope's entry of step t, and the step's tiles given it: a step
+  // takes its entry from a register loaded steps earlier, off the chain
+  __device__ __forceinline__ int entry(int t) const {
+    if (t >= 2 * nblk) return 0;
+    if (t < nblk) return jf ? __ldg(jf + t) : J;
+    return jb ? __ldg(jb + 2 * nblk - 1 - t) : J;
+  }
+  __device__ __forceinline__ int tiles(int t, int entry) const {
+    const int b = t < nblk ? t : t - nblk;
+    return max(0, min(min(J, b), entry));
+  }
+  __device__ __forceinline__ int jmax(int t) const { return tiles(t, entry(t)); }
+};
+
+// The far tiles (j > NEAR) a CTA owns, ascending: round-robin over the ranks
+// 1..C-1, except the last of every Q (Q >= 2), which are the leader's.  C = 1:
+// all of them.
+__device__ int own_list(unsigned short *own, int J, int C, int rank, int Q) {
+  int n = 0, m = 0;  // m: position among the ranks' tiles
+  for (int j = NEAR + 1; j <= J; j++) {
+    const bool lead = C == 1 || (Q >= 2 && (j - NEAR - 1) % Q == Q - 1);
+    if (lead ? rank == 0 : (rank > 0 && m == rank - 1)) own[n++] = (unsigned short)j;
+    if (!lead && ++m == C - 1) m = 0;
+  }
+  return n;
+}
+
+// Tiles of the list with j <= jm, from the count at the last step.
+__device__ __forceinline__ int own_count(const unsigned short *own, int len, int n, int jm) {
+  while (n < len && own[n] <= jm) n++;
+  while (n > 0 && own[n - 1] > jm) n--;
+  return n;
+}
+
+using Fwd = std::true_type;
+using Bwd = std::false_type;
+
+}  // namespace
+
+__global__ void __launch_bounds__(SWP_THREADS, 1)
     k_band_sweep(const Job *__restrict__ jobs, int C, int S, int Wmax, int Q) {
   const int rank = (int)cluster_ctarank();
   const Job Jb = jobs[blockIdx.x / C];
-  const int P = Jb.P, nblk = Jb.nblk, W = Jb.J + 2;
+  const int P = Jb.P, nblk = Jb.nblk, T = 2 * nblk, J = Jb.J;
+  const int W = window_blocks(J);
+  constexpr int D = DEPTH;
   extern __shared__ __align__(128) unsigned char smraw[];
-  double *ring = reinterpret_cast<double *>(smraw);      // S * TSZ
-  double *ysl = ring + (size_t)S * TSZ;                  // 2 * PMAX * NB: y of this tile and the next
-  double *pbuf = ysl + (size_t)2 * PMAX * NB;            // 2 * (C-1) * PMAX * NB
-  double *qpart = pbuf + (size_t)2 * max(C - 1, 1) * PMAX * NB;  // 4 * PMAX * NB
-  double *acc = qpart + 4 * PMAX * NB;                   // PMAX * NB
-  double *yk = acc + PMAX * NB;                          // PMAX * NB
-  uint64_t *full = reinterpret_cast<uint64_t *>(yk + PMAX * NB);  // S
-  uint64_t *ybar = full + S;                             // Wmax
-  uint64_t *pbar = ybar + Wmax;                          // 2
-  __shared__ int abort_flag;
+  double *ring = reinterpret_cast<double *>(smraw);             // S tiles
+  double *zwin = ring + (size_t)S * TSZ;                        // Wmax blocks
+  // the warps' sums: one buffer in the leader, whose steps end with a barrier,
+  // and its D * (C - 1) partial sums after it; two buffers in a rank
+  double *red = zwin + (size_t)Wmax * VEC;
+  double *pbuf = red + SWP_WARPS * RED;
+  double *vd = red + red_doubles(C);                            // D_k^T z_k
+  uint64_t *full = reinterpret_cast<uint64_t *>(vd + VEC);      // S
+  uint64_t *empty = full + S;                                   // S
+  uint64_t *zbar = empty + S;                                   // Wmax
+  uint64_t *pbar = zbar + Wmax;                                 // D
+  unsigned short *own = reinterpret_cast<unsigned short *>(pbar + D);  // J + 1
+  __shared__ int abort_flag, own_len;
 
-  const int tid = threadIdx.x, c = tid & (NB - 1), q = tid >> 6;
-  const SweepGeom G{nblk,
-                    Jb.J,
-                    C,
-                    rank,
-                    Q,
-                    FastDiv((unsigned)max(C - 1, 1)),
-                    FastDiv((unsigned)max(Q, 1)),
-                    FastDiv((unsigned)max(Q - 1, 1)),
-                    Jb.jf,
-                    Jb.jb};
-  const FastDiv dW((unsigned)W);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const StepTab tab{Jb.jf, Jb.jb, nblk, J};
   const long long lim = g_sweep_wait;
   if (tid == 0) {
-    for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
-    for (int w = 0; w < Wmax; w++) mbar_init(&ybar[w], 1);
-    mbar_init(&pbar[0], max(C - 1, 1));
-    mbar_init(&pbar[1], max(C - 1, 1));
+    for (int s = 0; s < S; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], SWP_WARPS);
+    }
+    for (int s = 0; s < W; s++) mbar_init(&zbar[s], 1);
+    for (int s = 0; s < D; s++) mbar_init(&pbar[s], 1);
     fence_mbar_init_cluster();
+    // each phase of these barriers ends with its bytes; the owner arms it
+    if (rank != 0)
+      for (int s = 0; s < min(W, T); s++) mbar_arrive_expect_tx(&zbar[s], VEC * sizeof(double));
+    if (rank == 0 && C > 1)
+      for (int s = 0; s < min(D, T); s++) mbar_arrive_expect_tx(&pbar[s], (C - 1) * VEC * sizeof(double));
+    own_len = own_list(own, J, C, rank, Q);
     abort_flag = 0;
   }
   __syncthreads();
   cluster_sync_all();
+  volatile int *const aborted = &abort_flag;
+  const int len = own_len;
 
-  const int T = 2 * nblk;
-  // producer state (thread 0): next tile (tp, ip); counters are uniform.
-  int tp = 0, ip = 0, pslot = 0;
-  SweepGeom::Step ps = G.step(0);  // the producer's step tp
-  long long nissued = 0, ncons = 0;
-  int cslot = 0;
-  uint32_t cphase = 0;  // slot and phase parity of tile ncons
-  auto consumed = [&]() {
-    ncons++;
-    if (++cslot == S) {
-      cslot = 0;
-      cphase ^= 1u;
-    }
-  };
-  auto produce = [&](long long limit) {
-    while (nissued < limit) {
-      while (tp < T && ip >= G.count(ps)) {
-        tp++;
-        ip = 0;
-        ps = SweepGeom::Step{ps.jm1, G.jmax(tp + 1)};
-      }
-      if (tp >= T) return;
-      const int j = G.jat(ps, ip);
-      double *dst = ring + (size_t)pslot * TSZ;
-      uint64_t *bar = &full[pslot];
-      if (++pslot == S) pslot = 0;
-      mbar_arrive_expect_tx(bar, (uint32_t)(TSZ * sizeof(double)));
-      // the leader's share is listed a step early: the tile is step tp + 1's
-      bulk_g2s(dst, tile_src(Jb, G.ahead(j) ? tp + 1 : tp, j), (uint32_t)(TSZ * sizeof(double)), bar);
-      nissued++;
-      ip++;
-    }
-  };
-  if (tid == 0) produce(S);
-
-  // Block src (the one solved at step src) from the RHS array into ysl[b]:
-  // threads tid < P NB / 2 copy one 16-byte chunk each through L2.
-  auto copy_y = [&](int src, int b) {
-    if (tid < P * (NB / 2)) {
-      const int p = tid / (NB / 2), ch = tid - p * (NB / 2);
-      const int blk = src < nblk ? src : 2 * nblk - 1 - src;
-      cp_async16_cg(ysl + ((size_t)b * PMAX + p) * NB + 2 * ch,
-                    Jb.rhs + (size_t)p * Jb.rhs_stride + (size_t)blk * NB + 2 * ch);
-    }
-    cp_async_commit();
-  };
-  // The block a tile (t, j >= 2) multiplies, solved at step t - j (t + 1 - j
-  // for the leader's tiles of the next step): every thread of a rank waits
-  // (bounded) for the leader's release of it, then copies its chunk.  False
-  // if the wait ran out (nothing is copied then).
-  auto fetch_y = [&](int t, int j, int b) -> bool {
-    const int src = (G.ahead(j) ? t + 1 : t) - j;
-    // only the copying threads need the release (the others read the block
-    // after a barrier that follows the copies)
-    if (rank != 0 && tid < P * (NB / 2)) {
-      const int qw = dW.div(src);
-      if (!mbar_wait(&ybar[src - qw * W], (uint32_t)(qw & 1), lim)) return false;
-    }
-    copy_y(src, b);
-    return true;
-  };
-  // Tiles that multiply a fetched block alternate between the two halves of
-  // ysl (ytile counts them, the same in every thread).  The next step's
-  // first such block is fetched under the current step's last one when its
-  // release is already visible to this thread (one probe, no wait): each
-  // thread copies its own chunk, so each may decide alone (pre).
-  long long ytile = 0;
-  bool pre = false;
-
-  // the leader's right-hand side of the next block column, loaded a step
-  // ahead (threads q == 0: column c, each plane); the first backward step's
-  // is the forward sweep's last block, taken from the registers that solve it
-  double bnext[PMAX];
-  if (rank == 0 && q == 0) {
-#pragma unroll
-    for (int p = 0; p < PMAX; p++)
-      if (p < P) bnext[p] = Jb.rhs[(size_t)p * Jb.rhs_stride + c];
-  }
-
-  // the leader's partial sums of its tiles of the next step (leader share)
-  double sn[PMAX];
-#pragma unroll
-  for (int p = 0; p < PMAX; p++) sn[p] = 0.0;
-
-  for (int t = 0; t < T; t++) {
-    const bool fwd = t < nblk;
-    const int k = fwd ? t : 2 * nblk - 1 - t;
-    const SweepGeom::Step cs = G.step(t);
-    const int n = G.count(cs);
-    double s[PMAX];
-#pragma unroll
-    for (int p = 0; p < PMAX; p++) {
-      s[p] = sn[p];  // zero unless the leader worked on this step's tiles during the last one
-      sn[p] = 0.0;
-    }
-    bool bad = false;
-    // the step's first tile's block; each later one is fetched under the
-    // work of the tile before it (j = 1 uses the leader's own yk, D_k none)
-    int jn = n > 0 ? G.jat(cs, 0) : 0;
-    if (jn >= 2 && !pre && !fetch_y(t, jn, (int)(ytile & 1))) bad = true;
-    pre = false;
-    for (int idx = 0; idx < n; idx++) {
-      const int j = jn;
-      if (j == 0) break;  // D_k: handled below by the leader
-      const int slot = cslot;
-      if (!mbar_wait(&full[slot], cphase, lim)) bad = true;
-      cp_async_wait_all();  // this thread's chunks of the tile's block
-      if (bad) abort_flag = 1;
-      __syncthreads();
-      if (abort_flag) break;
-      const double *yv = yk;
-      if (j >= 2) yv = ysl + (size_t)(ytile++ & 1) * PMAX * NB;
-      jn = idx + 1 < n ? G.jat(cs, idx + 1) : 0;
-      // ysl[ytile & 1] was last read two fetched tiles ago, before the
-      // barrier that ended it; a failed wait is seen after this tile's barrier
-      if (jn >= 2) {
-        if (!fetch_y(t, jn, (int)(ytile & 1))) abort_flag = 1;
-      } else if (t + 1 < T) {
-        const SweepGeom::Step ns = SweepGeom::Step{cs.jm1, G.jmax(t + 2)};
-        const int n1 = G.count(ns), j1 = n1 > 0 ? G.jat(ns, 0) : 0;
-        const int src = (G.ahead(j1) ? t + 2 : t + 1) - j1;
-        // the leader copies without a release; block t itself is solved
-        // only at the end of this step
-        const int qw = dW.div(src);
-        if (j1 >= 2 && (rank == 0 ? src < t : mbar_test_cluster(&ybar[src - qw * W], (uint32_t)(qw & 1)))) {
-          copy_y(src, (int)(ytile & 1));
-          pre = true;
+  if (w == SWP_WARPS) {
+    // ---- the copying warp: every tile this CTA reads, in its order of use
+    cluster_arrive();  // the barrier between the sweeps: nothing to wait for here
+    if (lane == 0) {
+      long long n = 0;  // tiles issued
+      int slot = 0;
+      uint32_t use = 0;  // times the ring has gone round
+      bool stop = false;
+      auto issue = [&](const double *src) {
+        if (stop) return;
+        if (use > 0) {
+          if (!mbar_wait_tx(&empty[slot], (use - 1) & 1, lim)) *aborted = 1;
+          if (*aborted) {
+            stop = true;
+            return;
+          }
         }
-      }
-      const double *Tt = ring + (size_t)slot * TSZ;
-      // the leader's tiles of the next step go to sn, every other tile to s
-      auto tile_dot = [&](double(&acc)[PMAX]) {
-        if (fwd) {
-#pragma unroll 4
-          for (int rr = q * 16; rr < q * 16 + 16; rr++) {
-            const double tv = Tt[rr * LDT + c];
-#pragma unroll
-            for (int p = 0; p < PMAX; p++)
-              if (p < P) acc[p] += tv * yv[p * NB + rr];
-          }
-        } else {
-#pragma unroll 4
-          for (int cc = q * 16; cc < q * 16 + 16; cc++) {
-            const double tv = Tt[c * LDT + cc];
-#pragma unroll
-            for (int p = 0; p < PMAX; p++)
-              if (p < P) acc[p] += tv * yv[p * NB + cc];
-          }
+        mbar_arrive_expect_tx(&full[slot], (uint32_t)(TSZ * sizeof(double)));
+        bulk_g2s(ring + (size_t)slot * TSZ, src, (uint32_t)(TSZ * sizeof(double)), &full[slot]);
+        n++;
+        if (++slot == S) {
+          slot = 0;
+          use++;
         }
       };
-      if (G.ahead(j))
-        tile_dot(sn);
-      else
-        tile_dot(s);
-      __syncthreads();
-      consumed();
-      if (tid == 0) produce(ncons + S);
-    }
-    if (abort_flag) break;
-    // reduce the four row quarters in fixed order
-#pragma unroll
-    for (int p = 0; p < PMAX; p++)
-      if (p < P) qpart[(q * PMAX + p) * NB + c] = s[p];
-    __syncthreads();
-    if (rank != 0) {
-      // The leader reads pbuf[t & 1] of step t-2 before it publishes block
-      // t-2; seeing that block means the slot is free again.
-      if (t >= 2) {
-        const int src = t - 2, qw = dW.div(src);
-        if (!mbar_wait(&ybar[src - qw * W], (uint32_t)(qw & 1), lim)) abort_flag = 1;
-        __syncthreads();
-        if (abort_flag) break;
-      }
-      // partial -> leader's pbuf[t & 1][rank-1]
-      if (q == 0) {
-        for (int p = 0; p < P; p++) {
-          const double v = qpart[(0 * PMAX + p) * NB + c] + qpart[(1 * PMAX + p) * NB + c] +
-                           qpart[(2 * PMAX + p) * NB + c] + qpart[(3 * PMAX + p) * NB + c];
-          double *dst = pbuf + ((size_t)((t & 1) * (C - 1) + (rank - 1)) * PMAX + p) * NB + c;
-          st_cluster_f64(map_rank(dst, 0), v);
+      const size_t J1 = J + 1;
+      auto off = [&](int t, int j) {  // tile j of step t
+        return Jb.tiles + ((size_t)(t < nblk ? t : 2 * nblk - 1 - t + j) * J1 + j) * TSZ;
+      };
+      int cnt = 0;
+      if (rank == 0) {
+        int jm = tab.jmax(0);
+        for (int t = 0; t < T && !stop; t++) {
+          if (jm >= 1) issue(off(t, 1));
+          if (C == 1 && t < nblk) issue(Jb.dinv + (size_t)t * TSZ);
+          jm = tab.jmax(t + 1);
+          cnt = own_count(own, len, cnt, jm);
+          for (int i = cnt - 1; i >= 0; i--) issue(off(t + 1, own[i]));
+          for (int j = min(jm, NEAR); j >= 2; j--) issue(off(t + 1, j));
         }
-        fence_acq_rel_cluster();
+      } else {
+        int dm = 0;  // block t - DLAG modulo C - 1
+        for (int t = 0; t < T && !stop; t++) {
+          if (t >= DLAG && t < nblk) {
+            if (dm == rank - 1) issue(Jb.dinv + (size_t)(t - DLAG) * TSZ);
+            if (++dm == C - 1) dm = 0;
+          }
+          cnt = own_count(own, len, cnt, tab.jmax(t));
+          for (int i = cnt - 1; i >= 0; i--) issue(off(t, own[i]));
+          if (t == nblk - 1)
+            for (int k = max(0, nblk - DLAG); k < nblk; k++) {
+              if (dm == rank - 1) issue(Jb.dinv + (size_t)k * TSZ);
+              if (++dm == C - 1) dm = 0;
+            }
+        }
       }
-      __syncthreads();
-      if (tid == 0) mbar_arrive_cluster(map_rank(&pbar[t & 1], 0));
-      continue;
-    }
-    // ---- leader: combine partials, apply D_k, broadcast ----
-    if (C > 1) {
-      if (!mbar_wait(&pbar[t & 1], (uint32_t)((t >> 1) & 1), lim)) abort_flag = 1;
-    }
-    if (!mbar_wait(&full[cslot], cphase, lim)) abort_flag = 1;
-    __syncthreads();
-    if (abort_flag) break;
-    if (q == 0) {
-#pragma unroll
-      for (int p = 0; p < PMAX; p++) {
-        if (p >= P) continue;
-        double v = qpart[(0 * PMAX + p) * NB + c] + qpart[(1 * PMAX + p) * NB + c] +
-                   qpart[(2 * PMAX + p) * NB + c] + qpart[(3 * PMAX + p) * NB + c];
-        for (int r = 1; r < C; r++) v += pbuf[((size_t)((t & 1) * (C - 1) + (r - 1)) * PMAX + p) * NB + c];
-        acc[p * NB + c] = bnext[p] - v;
-      }
-    }
-    __syncthreads();
-    {
-      const double *Dk = ring + (size_t)cslot * TSZ;
-#pragma unroll
-      for (int p = 0; p < PMAX; p++) s[p] = 0.0;
-      for (int cc = q * 16; cc < q * 16 + 16; cc++) {
-        const double dv = fwd ? Dk[cc * LDT + c] : Dk[c * LDT + cc];
-#pragma unroll
-        for (int p = 0; p < PMAX; p++)
-          if (p < P) s[p] += dv * acc[p * NB + cc];
+      // the copies still in flight (none unless the sweep was given up)
+      for (int s = 0; s < S && s < n; s++) {
+        const uint32_t u = s < slot ? use : use - 1;  // the slot's last use
+        mbar_wait_tx(&full[s], u & 1, WAIT_LIMIT);
       }
     }
-    __syncthreads();  // all reads of D_k done
-    consumed();
-    if (tid == 0) produce(ncons + S);
-#pragma unroll
-    for (int p = 0; p < PMAX; p++)
-      if (p < P) qpart[(q * PMAX + p) * NB + c] = s[p];
-    __syncthreads();
-    if (q == 0) {
-#pragma unroll
-      for (int p = 0; p < PMAX; p++) {
-        if (p >= P) continue;
-        const double v = qpart[(0 * PMAX + p) * NB + c] + qpart[(1 * PMAX + p) * NB + c] +
-                         qpart[(2 * PMAX + p) * NB + c] + qpart[(3 * PMAX + p) * NB + c];
-        yk[p * NB + c] = v;
-        Jb.rhs[(size_t)p * Jb.rhs_stride + (size_t)k * NB + c] = v;
-        if (t + 1 == nblk) bnext[p] = v;  // backward from the last block: its y is its right-hand side
-      }
-    }
-    // block t is in rhs (and yk): release it to every other rank (slot
-    // t % W of their barriers); the writers' fence orders their stores
-    // before the arrivals that follow the barrier
-    if (q == 0) fence_acq_rel_cluster();
-    __syncthreads();
-    if (tid > 0 && tid < C) mbar_arrive_cluster(map_rank(&ybar[dW.mod(t)], (uint32_t)tid));
-    // the next step's right-hand side, issued after the fence (which would
-    // wait for it) and used a step later
-    if (q == 0 && t + 1 < T && t + 1 != nblk) {
-      const int kn = t + 1 < nblk ? t + 1 : 2 * nblk - 2 - t;  // next step's block column
-#pragma unroll
-      for (int p = 0; p < PMAX; p++)
-        if (p < P) bnext[p] = Jb.rhs[(size_t)p * Jb.rhs_stride + (size_t)kn * NB + c];
-    }
+    __syncwarp();
+    cluster_wait();
+    cluster_sync_all();
+    return;
   }
 
-  if (abort_flag) {
-    cp_async_wait_all();
-    if (tid == 0) {
-      atomicOr(Jb.status, 1 << SX_ERR_TIMEOUT);
-      // drain this CTA's bulk copies still in flight (bounded)
-      for (long long i = ncons; i < nissued; i++) {
-        mbar_wait(&full[cslot], cphase, WAIT_LIMIT);
-        if (++cslot == S) {
-          cslot = 0;
-          cphase ^= 1u;
-        }
-      }
+  // ---- the working warps
+  bool dead = false;
+  auto wait = [&](uint64_t *bar, uint32_t parity) {
+    if (!dead && !mbar_wait_tx(bar, parity, lim)) {
+      dead = true;
+      *aborted = 1;
     }
-    __syncthreads();
+  };
+  int cs = 0;  // ring slot and phase of the next tile
+  uint32_t cph = 0;
+  bool here = false;  // the next tile is known to have landed
+  // A wait for a phase that is already complete still takes some 120 cycles, so
+  // the next tile's is probed as soon as this one is in registers, under its
+  // arithmetic.
+  auto await_tile = [&]() {
+    if (!here) wait(&full[cs], cph);
+  };
+  auto release = [&]() {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[cs]);
+    if (++cs == S) {
+      cs = 0;
+      cph ^= 1u;
+    }
+    here = mbar_test_cta(&full[cs], cph);
+  };
+  const int e = tid / LPE, q4 = tid % LPE;  // this thread's element of a block, shared by LPE lanes
+  const int ec = e >> 1, ep = e & 1;       // its row and plane
+  double *const gx = Jb.rhs + (size_t)(ep < P ? ep : 0) * Jb.rhs_stride + ec;
+  double acc[2 * RPW];
+  auto clear = [&]() {
+#pragma unroll
+    for (int i = 0; i < 2 * RPW; i++) acc[i] = 0.0;
+  };
+  // acc += tile j of a step whose window slot is bs times the block solved j
+  // steps before it, which the caller knows to be in the window
+  auto tile = [&](auto F, int j, int bs) {
+    const int zs = bs - j < 0 ? bs - j + W : bs - j;
+    TileRegs r;
+    await_tile();
+    tile_load<decltype(F)::value>(r, ring + (size_t)cs * TSZ, zwin + (size_t)zs * VEC, w, lane);
+    release();
+    tile_fma<decltype(F)::value>(r, acc);
+  };
+  const int pf = e, pb = ep * NB + ec;  // its place in a block of the forward and the backward sweep
+  // this CTA's sum of element e, in parts over its lanes
+  // (the leader's partial sums are read on the way to the barrier, by `also`)
+  auto reduce = [&](auto F, int par, auto also) -> double {
+    if (!decltype(F)::value) {
+      const double o = also();
+      return lanes_reduce(acc, lane) + o;
+    }
+    double *r = rank == 0 ? red : red + par * SWP_WARPS * RED;
+    double2 *r2 = reinterpret_cast<double2 *>(r + w * RED) + 2 * lane;
+    r2[0] = make_double2(acc[0], acc[1]);
+    r2[1] = make_double2(acc[2], acc[3]);
+    const double o = also();
+    bar_sync(1, SWP_WARPS * 32);
+    const double *q = r + (SWP_WARPS / LPE) * q4 * RED + e;
+    static_assert(SWP_WARPS / LPE == 4, "four warps' sums a lane");
+    return ((q[0] + q[RED]) + (q[2 * RED] + q[3 * RED])) + o;
+  };
+  auto none = []() { return 0.0; };
+  // w_k = D_k D_k^T z_k from the window slot zs, into rhs
+  auto apply_d = [&](int k, int zs, int par) {
+    clear();
+    TileRegs r;
+    await_tile();
+    const double *t = ring + (size_t)cs * TSZ;
+    tile_load<true>(r, t, zwin + (size_t)zs * VEC, w, lane);
+    tile_fma<true>(r, acc);
+    const double v = lane_sum(reduce(Fwd(), par, none));
+    if (q4 == 0) vd[pb] = v;
+    bar_sync(1, SWP_WARPS * 32);
+    clear();
+    tile_load<false>(r, t, vd, w, lane);
+    release();
+    tile_fma<false>(r, acc);
+    const double x = lane_sum(lanes_reduce(acc, lane));
+    if (q4 == 0 && ep < P) gx[(size_t)k * NB] = x;
+    clear();
+  };
+  auto between_sweeps = [&]() {
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+  };
+
+  clear();
+  int cnt = 0, bs = 0, ps = 0;  // bs, bp: window slot and parity of step t; ps, pp: of its partial sums
+  uint32_t bp = 0, pp = 0;
+  if (rank == 0) {
+    int jm = tab.jmax(0), e1 = tab.entry(1);
+    double b = nblk > 0 && ep < P ? __ldcg(gx) : 0.0;
+    // this lane's ranks to send to: 1 + q4, 1 + q4 + LPE, ... (at most 15 ranks)
+    constexpr int NTO = 16 / LPE;
+    uint32_t to_z[NTO], to_bar[NTO];
+#pragma unroll
+    for (int i = 0; i < NTO; i++) {
+      const int r = min(1 + q4 + LPE * i, C - 1);
+      to_z[i] = map_rank(zwin, r);
+      to_bar[i] = map_rank(zbar, r);
+    }
+    auto step = [&](auto F, int t) {
+      const int e2 = tab.entry(t + 2);
+      const bool parts = C > 1 && mbar_test_cta(&pbar[ps], pp);  // the ranks' partial sums are here
+      if (jm >= 1) tile(F, 1, bs);
+      const double s = reduce(F, t & 1, [&]() {
+        double o = 0.0;
+        if (C > 1) {
+          if (!parts) wait(&pbar[ps], pp);
+          const double *q = pbuf + (size_t)ps * (C - 1) * VEC + e;
+          for (int r = q4; r < C - 1; r += LPE) o += q[(size_t)r * VEC];
+        }
+        return o;
+      });
+      const double z = b - lane_sum(s);
+      const int zo = bs * VEC + (decltype(F)::value ? pf : pb);
+      if (q4 == 0) zwin[zo] = z;
+      if (C > 1 && !dead) {
+#pragma unroll
+        for (int i = 0; i < NTO; i++)
+          if (1 + q4 + LPE * i < C)
+            st_async_f64(to_z[i] + zo * (int)sizeof(double), z, to_bar[i] + bs * (int)sizeof(uint64_t));
+      }
+      if (C > 1 && tid == 0 && t + D < T && !dead)
+        mbar_arrive_expect_tx(&pbar[ps], (C - 1) * VEC * sizeof(double));
+      // the next step's right-hand side (the first backward one is read after the barrier)
+      const int tn = t + 1;
+      if (!decltype(F)::value && q4 == 0 && ep < P) gx[(size_t)(T - 1 - t) * NB] = z;
+      if (tn < T && tn != nblk && ep < P) b = __ldcg(gx + (size_t)(tn < nblk ? tn : T - 1 - tn) * NB);
+      bar_sync(1, SWP_WARPS * 32);
+      clear();
+      if (C == 1 && decltype(F)::value) apply_d(t, bs, t & 1);
+      if (++bs == W) {
+        bs = 0;
+        bp ^= 1u;
+      }
+      if (++ps == D) {
+        ps = 0;
+        pp ^= 1u;
+      }
+      jm = tab.tiles(tn, e1);
+      e1 = e2;
+      if (len > 0) {
+        cnt = own_count(own, len, cnt, jm);
+        for (int i = cnt - 1; i >= 0; i--) tile(F, own[i], bs);
+      }
+      for (int j = min(jm, NEAR); j >= 2; j--) tile(F, j, bs);
+    };
+    for (int t = 0; t < nblk; t++) step(Fwd(), t);
+    between_sweeps();
+    if (nblk > 0 && ep < P) b = __ldcg(gx + (size_t)(nblk - 1) * NB);
+    for (int t = nblk; t < T; t++) step(Bwd(), t);
+  } else {
+    int dm = 0, ej = tab.entry(0);
+    const uint32_t to_p = map_rank(pbuf + (rank - 1) * VEC + e, 0), to_pbar = map_rank(pbar, 0);
+    // block t - back's slot and parity
+    auto slot_back = [&](int back, uint32_t &par) {
+      int s = bs - back;
+      par = bp;
+      if (s < 0) {
+        s += W;
+        par ^= 1u;
+      }
+      return s;
+    };
+    auto step = [&](auto F, int t) {
+      const int jm = tab.tiles(t, ej);
+      ej = tab.entry(t + 1);
+      // block t's phase in this CTA's window: the leader sends it once it has
+      // this step's partial sum, below
+      if (tid == 0 && t >= W) {
+        wait(&zbar[bs], bp ^ 1u);
+        if (!dead) mbar_arrive_expect_tx(&zbar[bs], VEC * sizeof(double));
+      }
+      if (decltype(F)::value && t >= DLAG) {
+        if (dm == rank - 1) {
+          uint32_t par;
+          const int zs = slot_back(DLAG, par);
+          wait(&zbar[zs], par);
+          apply_d(t - DLAG, zs, t & 1);
+        }
+        if (++dm == C - 1) dm = 0;
+      }
+      // Each step waits for one block, t - D, once: before the tile that needs
+      // it (j = NEAR + 1 = D), or before the partial sum goes out -- its slot
+      // has been read once block t - D is here.  Older blocks were waited for
+      // in earlier steps.
+      bool waited = t < D;
+      auto wait_block = [&]() {
+        if (waited) return;
+        uint32_t par;
+        const int zs = slot_back(D, par);
+        wait(&zbar[zs], par);
+        waited = true;
+      };
+      cnt = own_count(own, len, cnt, jm);
+      for (int i = cnt - 1; i >= 0; i--) {
+        const int j = own[i];
+        if (j <= D) wait_block();
+        tile(F, j, bs);
+      }
+      const double s = lane_sum(reduce(F, t & 1, none));
+      wait_block();
+      if (q4 == 0 && !dead)
+          st_async_f64(to_p + ps * (C - 1) * (VEC * (int)sizeof(double)), s, to_pbar + ps * (int)sizeof(uint64_t));
+      clear();
+      if (++bs == W) {
+        bs = 0;
+        bp ^= 1u;
+      }
+      if (++ps == D) ps = 0;
+    };
+    for (int t = 0; t < nblk; t++) step(Fwd(), t);
+    for (int k = max(0, nblk - DLAG); k < nblk; k++) {
+      if (dm == rank - 1) {
+        uint32_t par;
+        const int zs = slot_back(nblk - k, par);
+        wait(&zbar[zs], par);
+        apply_d(k, zs, nblk & 1);  // not the buffer that step nblk - 1 may still be reading
+      }
+      if (++dm == C - 1) dm = 0;
+    }
+    between_sweeps();
+    for (int t = nblk; t < T; t++) step(Bwd(), t);
+    // every block the leader sent has landed before this CTA leaves
+    for (int back = min(W, T); back >= 1; back--) {
+      uint32_t par;
+      const int zs = slot_back(back, par);
+      wait(&zbar[zs], par);
+    }
   }
+  __syncwarp();
   cluster_sync_all();
+  if (*aborted) {
+    if (tid == 0) atomicOr(Jb.status, 1 << SX_ERR_TIMEOUT);
+    // another CTA's last stores into this one's shared memory, sent before it
+    // met the barrier above, land within a microsecond or two
+    const long long t0 = clock64();
+    while (clock64() - t0 < 200000) {
+    }
+  }
 }
 
-size_t sweep_smem(int pmax, int C, int S, int Wmax) {
-  return sizeof(double) * ((size_t)S * TSZ + (size_t)2 * pmax * NB +
-                           (size_t)2 * std::max(C - 1, 1) * pmax * NB + 6 * (size_t)pmax * NB) +
-         sizeof(uint64_t) * (S + Wmax + 2);
+static size_t sweep_smem(int C, int S, int Wmax) {
+  return sizeof(double) * ((size_t)S * TSZ + ((size_t)Wmax + 1) * VEC + red_doubles(C)) +
+         sizeof(uint64_t) * (2 * S + Wmax + DEPTH) + ((sizeof(unsigned short) * (Wmax + 1) + 15) & ~(size_t)15);
 }
 
-// Dynamic shared memory available to the sweep kernels: the opt-in limit
-// minus their static shared memory.
+// Dynamic shared memory available to the sweep kernel: the opt-in limit
+// minus its static shared memory.
 static int smem_optin() {
   static int v = 0;
   if (!v) {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes a2, a8;
-    cudaFuncGetAttributes(&a2, k_band_sweep<2>);
-    cudaFuncGetAttributes(&a8, k_band_sweep<8>);
-    v = optin - (int)std::max(a2.sharedSizeBytes, a8.sharedSizeBytes);
+    cudaFuncAttributes a;
+    cudaFuncGetAttributes(&a, k_band_sweep);
+    v = optin - (int)a.sharedSizeBytes;
   }
   return v;
 }
 
+// The deepest ring of at most smax tiles that fits (0: none).
+static int fit_stages(int C, int smax, int Wmax) {
+  int S = std::max(1, std::min(smax, BAND_STAGES_MAX));
+  while (S > 0 && sweep_smem(C, S, Wmax) > (size_t)smem_optin()) S--;
+  return S;
+}
+
 // Launch both sweeps for every job: one cluster of sc.C CTAs per job.
 int band_sweep_jobs(const Job *djobs, const std::vector<Job> &hjobs, const BandSched &sc, cudaStream_t st) {
-  const int C = sc.C, smax = sc.S;
+  const int C = sc.C;
   const int nj = (int)hjobs.size();
   if (nj == 0) return SX_OK;
   int maxP = 0, Wmax = 0;
   for (const Job &j : hjobs) {
     maxP = std::max(maxP, j.P);
-    Wmax = std::max(Wmax, j.J + 2);
+    Wmax = std::max(Wmax, window_blocks(j.J));
   }
-  if (maxP > 8) return SX_ERR_UNSUPPORTED;
-  const int pmax = maxP <= 2 ? 2 : 8;
-  const int limit = smem_optin();
-  int S = std::max(1, std::min(smax, BAND_STAGES_MAX));
-  while (S > 1 && sweep_smem(pmax, C, S, Wmax) > (size_t)limit) S--;
-  const size_t sm = sweep_smem(pmax, C, S, Wmax);
-  if (sm > (size_t)limit) {
-    set_error("band sweep needs %zu B of shared memory (limit %d)", sm, limit);
+  if (maxP > 2) return SX_ERR_UNSUPPORTED;
+  const int S = fit_stages(C, sc.S, Wmax);
+  if (S < 1) {
+    set_error("band sweep needs %zu B of shared memory (limit %d)", sweep_smem(C, 1, Wmax), smem_optin());
     return SX_ERR_UNSUPPORTED;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C * nj, 1, 1);
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.dynamicSmemBytes = sm;
+  cfg.blockDim = dim3(SWP_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = sweep_smem(C, S, Wmax);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -503,39 +618,32 @@ int band_sweep_jobs(const Job *djobs, const std::vector<Job> &hjobs, const BandS
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (pmax == 2)
-    SX_CUDA(cudaLaunchKernelEx(&cfg, k_band_sweep<2>, djobs, C, S, Wmax, std::max(sc.Q, 0)));
-  else
-    SX_CUDA(cudaLaunchKernelEx(&cfg, k_band_sweep<8>, djobs, C, S, Wmax, std::max(sc.Q, 0)));
+  SX_CUDA(cudaLaunchKernelEx(&cfg, k_band_sweep, djobs, C, S, Wmax, std::max(sc.Q, 0)));
   return SX_OK;
 }
 
 int prepare_band_kernels() {
   const int limit = smem_optin();
-  SX_CUDA(cudaFuncSetAttribute(k_band_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
-  SX_CUDA(cudaFuncSetAttribute(k_band_sweep<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
-  SX_CUDA(cudaFuncSetAttribute(k_band_sweep<2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  SX_CUDA(cudaFuncSetAttribute(k_band_sweep<8>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  SX_CUDA(cudaFuncSetAttribute(k_band_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+  SX_CUDA(cudaFuncSetAttribute(k_band_sweep, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   return SX_OK;
 }
 
-int default_lead(int C, int J) {
-  // an equal share (the last of every C positions) was the fastest share on
-  // every cluster size measured (config-3 band, 64 systems: C = 2, 3, 4);
-  // with fewer than C positions per block column the leader gets none
-  return (C >= 2 && J - 1 >= C) ? C : 0;
+int default_lead(int C, int) {
+  // the leader's j <= NEAR tiles are its share in clusters of four or more;
+  // in smaller ones the ranks would have most of the band to themselves (64
+  // systems, C = 2: half 16.6 ms, a third 17.8, none 20.7; 12 systems, C = 9:
+  // none 3.97, a sixth 6.0)
+  return C == 2 ? 2 : C == 3 ? 4 : 0;
 }
 
-// Largest cluster size (<= cmax) for which `nj` clusters can be resident at
-// once; at least 1.
-int band_active_clusters(int C, int pmax, int Wmax, int smax) {
-  int S = std::max(1, std::min(smax, BAND_STAGES_MAX));
-  while (S > 1 && sweep_smem(pmax, C, S, Wmax) > (size_t)smem_optin()) S--;
-  if (sweep_smem(pmax, C, S, Wmax) > (size_t)smem_optin()) return 0;
+// Clusters of C CTAs (ring of S tiles) that can be resident at once.
+static int resident_clusters(int C, int S, int Wmax) {
+  if (S < 1) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.dynamicSmemBytes = sweep_smem(pmax, C, S, Wmax);
+  cfg.blockDim = dim3(SWP_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = sweep_smem(C, S, Wmax);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C;
@@ -544,57 +652,47 @@ int band_active_clusters(int C, int pmax, int Wmax, int smax) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  const cudaError_t e = pmax == 2 ? cudaOccupancyMaxActiveClusters(&n, k_band_sweep<2>, &cfg)
-                                  : cudaOccupancyMaxActiveClusters(&n, k_band_sweep<8>, &cfg);
-  if (e != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, k_band_sweep, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return n;
 }
 
-// Largest cluster size C <= cmax (and ring depth) for which all nj clusters
-// are resident at once, over the ring depths 4, 2 and 1 (a shallower ring
-// shrinks a CTA's shared memory, so that two share an SM); the deeper ring
-// on a tie.  Depth 1 puts the leader's load of D_k on each block column's
-// critical path; it is taken only where the deeper rings leave at most 2
-// CTAs per system resident (measured at 4 CTAs on 64 systems with a 37-tile
-// band: depth 2, two CTAs per SM, 46 ms; depth 1 61 ms; and at 8 CTAs on 32
-// systems with a 17-tile band: depth 2 2.9 ms, depth 1 3.1 ms).
+int band_active_clusters(int C, int J, int smax) {
+  const int W = window_blocks(J);
+  return resident_clusters(C, fit_stages(C, smax, W), W);
+}
+
+// Cluster size C <= cmax and ring depth for nj systems of J tiles a block
+// column: the deepest ring with which every system's cluster is resident,
+// and the largest such cluster.  Depth comes first: a CTA alone on its SM
+// with four tiles in flight keeps up with its share of HBM, and shallower
+// rings are slower before they let a larger cluster in (32 systems, 4 CTAs
+// each: depth 4 0.78 ms, 3 0.84, 2 0.96; 5 CTAs at depth 2, in two waves,
+// 1.63).  Where not even one CTA a
+// system is resident, C = 1 at the depth with the most CTAs on the chip.
 // stages_forced > 0 fixes the depth.
-int pick_cluster(int nj, int cmax, int pmax, int Wmax, int *stages_out, int stages_forced) {
-  int bestC = 1, bestS = BAND_STAGES_MAX;
-  for (int S0 : {BAND_STAGES_MAX, 3, 2, 1}) {
-    if (stages_forced > 0 && S0 != stages_forced) continue;
-    if (S0 == 1 && stages_forced != 1 && bestC > 2) continue;
-    for (int C = 1; C <= cmax; C++) {
-      int S = S0;
-      while (S > 1 && sweep_smem(pmax, C, S, Wmax) > (size_t)smem_optin()) S--;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(C * nj, 1, 1);
-      cfg.blockDim = dim3(256, 1, 1);
-      cfg.dynamicSmemBytes = sweep_smem(pmax, C, S, Wmax);
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = C;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int n = 0;
-      const cudaError_t e = pmax == 2 ? cudaOccupancyMaxActiveClusters(&n, k_band_sweep<2>, &cfg)
-                                      : cudaOccupancyMaxActiveClusters(&n, k_band_sweep<8>, &cfg);
-      if (e != cudaSuccess) {
-        cudaGetLastError();
-        continue;
-      }
-      if (n >= nj && C > bestC) {
+int pick_cluster(int nj, int cmax, int J, int *stages_out, int stages_forced) {
+  int bestC = 0, bestS = BAND_STAGES_MAX, mostS = BAND_STAGES_MAX, most = 0;
+  for (int S = BAND_STAGES_MAX; S >= 1 && bestC == 0; S--) {
+    if (stages_forced > 0 && S != stages_forced) continue;
+    for (int C = cmax; C >= 1 && bestC == 0; C--) {
+      const int n = band_active_clusters(C, J, S);
+      if (n >= nj) {
         bestC = C;
-        bestS = S0;
+        bestS = S;
+      }
+      if (C == 1 && S >= 2 && n > most) {
+        most = n;
+        mostS = S;
       }
     }
   }
-  if (stages_forced > 0) bestS = stages_forced;
+  if (bestC == 0) {
+    bestC = 1;
+    bestS = stages_forced > 0 ? stages_forced : mostS;
+  }
   if (stages_out) *stages_out = bestS;
   return bestC;
 }

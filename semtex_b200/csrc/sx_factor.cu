@@ -16,6 +16,10 @@
 //      tile and forms its inverse, k_trsm forms the off-diagonal tiles of
 //      block row k, k_update applies the trailing rank-nb update inside the
 //      band.  All systems of a batch share each launch.
+//      What is kept is the block LDL^T form of the same factor: the diagonal
+//      tiles U_kk, their inverses D_k, and off the diagonal U_kk^-1 U(k, k+i)
+//      in place of U(k, k+i), so that the sweeps' block-column chains carry
+//      no diagonal solve (sx_band.cu).
 // JACPCG (src/matrix.cpp:276-317): k_elem_diag + k_diag_dss.
 #include <cmath>
 #include <cstring>
@@ -199,19 +203,18 @@ __global__ void k_band_mixed(MeshView M, double *tiles, int J, int nsolve) {
 // Tiled banded Cholesky
 // ---------------------------------------------------------------------------
 
+// In shared memory the diagonal tile's rows are PLD doubles apart (odd: row
+// and column walks are free of bank conflicts).
+constexpr int PLD = NB + 1;
+
 __device__ __forceinline__ void tile_load(double *dst, const double *__restrict__ src) {
-  const double2 *s = reinterpret_cast<const double2 *>(src);
-  double2 *d = reinterpret_cast<double2 *>(dst);
-  for (int i = threadIdx.x; i < TSZ / 2; i += blockDim.x) d[i] = s[i];
+  for (int i = threadIdx.x; i < TSZ; i += blockDim.x) dst[(i / LDT) * PLD + i % LDT] = src[i];
 }
 
 __device__ __forceinline__ void tile_store(double *dst, const double *src) {
-  const double2 *s = reinterpret_cast<const double2 *>(src);
-  double2 *d = reinterpret_cast<double2 *>(dst);
-  for (int i = threadIdx.x; i < TSZ / 2; i += blockDim.x) d[i] = s[i];
+  for (int i = threadIdx.x; i < TSZ; i += blockDim.x) dst[i] = src[(i / LDT) * PLD + i % LDT];
 }
 
-// Factor the diagonal tile of block column k and store its inverse.
 // Factor the diagonal tile of block column k, A = U^T U (upper), and form
 // D_k = U^-1, one CTA of 256 threads per system.
 //   Cholesky, right-looking: thread t owns column j = t % 64 at rows i = t /
@@ -226,18 +229,18 @@ __global__ void __launch_bounds__(256) k_potrf(const SysDesc *__restrict__ sys, 
   const SysDesc S = sys[blockIdx.x];
   if (k >= S.nblk) return;
   extern __shared__ __align__(16) double smp[];
-  double *A = smp, *X = smp + TSZ;
+  double *A = smp, *X = smp + NB * PLD;
   __shared__ int bad;
   const int tid = threadIdx.x;
   double *T = S.tiles + ((size_t)k * (S.J + 1)) * TSZ;
   if (tid == 0) bad = 0;
   tile_load(A, T);
-  for (int idx = tid; idx < TSZ; idx += 256) X[idx] = 0.0;
+  for (int idx = tid; idx < NB * PLD; idx += 256) X[idx] = 0.0;
   __syncthreads();
   const int j = tid & (NB - 1), rg = tid >> 6;
   double d_prev = 1.0, r_prev = 1.0;
   for (int c = 0; c < NB; c++) {
-    double a = A[c * LDT + c];
+    double a = A[c * PLD + c];
     if (!(a > 0.0)) {
       if (tid == 0) bad = 1;
       a = 1.0;
@@ -245,20 +248,20 @@ __global__ void __launch_bounds__(256) k_potrf(const SysDesc *__restrict__ sys, 
     const double d = sqrt(a), r = 1.0 / d;
     // row c - 1 is final: its owners scale it (and set its diagonal)
     if (c > 0 && ((c - 1) & 3) == rg && j >= c - 1)
-      A[(c - 1) * LDT + j] = j == c - 1 ? d_prev : A[(c - 1) * LDT + j] * r_prev;
+      A[(c - 1) * PLD + j] = j == c - 1 ? d_prev : A[(c - 1) * PLD + j] * r_prev;
     if (j > c) {
-      const double ucj = A[c * LDT + j] * r;
-      for (int i = c + 1 + ((rg - (c + 1)) & 3); i <= j; i += 4) A[i * LDT + j] -= (A[c * LDT + i] * r) * ucj;
+      const double ucj = A[c * PLD + j] * r;
+      for (int i = c + 1 + ((rg - (c + 1)) & 3); i <= j; i += 4) A[i * PLD + j] -= (A[c * PLD + i] * r) * ucj;
     }
     d_prev = d;
     r_prev = r;
     __syncthreads();
   }
-  if (rg == ((NB - 1) & 3) && j == NB - 1) A[(NB - 1) * LDT + NB - 1] = d_prev;
+  if (rg == ((NB - 1) & 3) && j == NB - 1) A[(NB - 1) * PLD + NB - 1] = d_prev;
   __syncthreads();
   for (int idx = tid; idx < NB * NB; idx += 256) {
     const int ii = idx / NB, jj = idx % NB;
-    if (jj < ii) A[ii * LDT + jj] = 0.0;
+    if (jj < ii) A[ii * PLD + jj] = 0.0;
   }
   __syncthreads();
   tile_store(T, A);
@@ -266,10 +269,10 @@ __global__ void __launch_bounds__(256) k_potrf(const SysDesc *__restrict__ sys, 
   for (int i = NB - 1; i >= 0; i--) {
     double s = 0.0;
     if (jc > i)
-      for (int l = i + 1 + q; l <= jc; l += 4) s += A[i * LDT + l] * X[l * LDT + jc];
+      for (int l = i + 1 + q; l <= jc; l += 4) s += A[i * PLD + l] * X[l * PLD + jc];
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (q == 0 && jc >= i) X[i * LDT + jc] = jc == i ? 1.0 / A[i * LDT + i] : -s / A[i * LDT + i];
+    if (q == 0 && jc >= i) X[i * PLD + jc] = jc == i ? 1.0 / A[i * PLD + i] : -s / A[i * PLD + i];
     __syncthreads();
   }
   tile_store(S.dinv + (size_t)k * TSZ, X);
@@ -286,9 +289,9 @@ __global__ void __launch_bounds__(256) k_potrf(const SysDesc *__restrict__ sys, 
 constexpr int LDM = NB + 4;
 
 __device__ __forceinline__ void tile_stage_mma(double *dst, const double *__restrict__ src) {
-  for (int idx = threadIdx.x; idx < NB * NB; idx += blockDim.x) {
-    const int r = idx >> 6, c = idx & (NB - 1);
-    cp_async8_ca(dst + r * LDM + c, src + r * LDT + c);
+  for (int idx = threadIdx.x; idx < NB * NB / 2; idx += blockDim.x) {
+    const int r = idx >> 5, c = 2 * (idx & (NB / 2 - 1));
+    cp_async16_cg(dst + r * LDM + c, src + r * LDT + c);
   }
 }
 
@@ -311,17 +314,19 @@ __device__ __forceinline__ void mma_f64(double &d0, double &d1, double a, double
                : "d"(a), "d"(b));
 }
 
-// acc += (neg ? -1 : 1) * A^T B over the NB rows of the staged tiles:
-// entry (r, c) gains sum_l A[l][r] B[l][c].
-__device__ __forceinline__ void mma_tn(MmaAcc &acc, const double *As, const double *Bs, bool neg) {
+// acc += op(A) B over the staged tiles: entry (r, c) gains sum_l A[l][r]
+// B[l][c] (TRANS, op(A) = A^T) or sum_l A[r][l] B[l][c].
+template <bool TRANS>
+__device__ __forceinline__ void mma_tile(MmaAcc &acc, const double *As, const double *Bs) {
   int r0, c0, g, t;
   mma_coords(r0, c0, g, t);
 #pragma unroll 4
   for (int l0 = 0; l0 < NB; l0 += 4) {
-    const double *Ar = As + (l0 + t) * LDM + r0 + g, *Br = Bs + (l0 + t) * LDM + c0 + g;
+    const double *Ar = TRANS ? As + (l0 + t) * LDM + r0 + g : As + (r0 + g) * LDM + l0 + t;
+    const double *Br = Bs + (l0 + t) * LDM + c0 + g;
     double a[2], b[4];
 #pragma unroll
-    for (int m = 0; m < 2; m++) a[m] = neg ? -Ar[8 * m] : Ar[8 * m];
+    for (int m = 0; m < 2; m++) a[m] = Ar[TRANS ? 8 * m : 8 * m * LDM];
 #pragma unroll
     for (int n = 0; n < 4; n++) b[n] = Br[8 * n];
 #pragma unroll
@@ -331,16 +336,11 @@ __device__ __forceinline__ void mma_tn(MmaAcc &acc, const double *As, const doub
   }
 }
 
-// Load (or zero) and store this thread's result elements of a band tile.
-__device__ __forceinline__ void mma_load(MmaAcc &acc, const double *__restrict__ T) {
-  int r0, c0, g, t;
-  mma_coords(r0, c0, g, t);
+__device__ __forceinline__ void mma_zero(MmaAcc &acc) {
 #pragma unroll
   for (int m = 0; m < 2; m++)
 #pragma unroll
-    for (int n = 0; n < 4; n++)
-#pragma unroll
-      for (int q = 0; q < 2; q++) acc.v[m][n][q] = T ? T[(r0 + 8 * m + g) * LDT + c0 + 8 * n + 2 * t + q] : 0.0;
+    for (int n = 0; n < 4; n++) acc.v[m][n][0] = acc.v[m][n][1] = 0.0;
 }
 
 // T -= acc at this thread's result elements (one subtraction each, after
@@ -360,6 +360,8 @@ __device__ __forceinline__ void mma_sub_store(double *T, const MmaAcc &acc) {
       }
 }
 
+// Stores this thread's result elements into a tile of row pitch LD.
+template <int LD>
 __device__ __forceinline__ void mma_store(double *T, const MmaAcc &acc) {
   int r0, c0, g, t;
   mma_coords(r0, c0, g, t);
@@ -367,13 +369,15 @@ __device__ __forceinline__ void mma_store(double *T, const MmaAcc &acc) {
   for (int m = 0; m < 2; m++)
 #pragma unroll
     for (int n = 0; n < 4; n++)
-#pragma unroll
-      for (int q = 0; q < 2; q++) T[(r0 + 8 * m + g) * LDT + c0 + 8 * n + 2 * t + q] = acc.v[m][n][q];
+      *reinterpret_cast<double2 *>(&T[(r0 + 8 * m + g) * LD + c0 + 8 * n + 2 * t]) =
+          make_double2(acc.v[m][n][0], acc.v[m][n][1]);
 }
 
-// Off-diagonal tiles of block row k: U(k, k+i) = U_kk^-T A(k, k+i), for the
-// tiles inside the envelope (i <= jb[k]); the others stay zero.
-__global__ void __launch_bounds__(256, 3) k_trsm(const SysDesc *__restrict__ sys, int k) {
+// Off-diagonal tiles of block row k inside the envelope (i <= jb[k]; the
+// others stay zero): U(k, k+i) = U_kk^-T A(k, k+i) into the row buffer, which
+// the trailing update reads (J tiles: they stay in L2), and U_kk^-1 U(k, k+i)
+// (scaled) or U(k, k+i) into the tile itself.
+__global__ void __launch_bounds__(256, 3) k_trsm(const SysDesc *__restrict__ sys, int k, bool scaled) {
   const SysDesc S = sys[blockIdx.y];
   const int i = blockIdx.x + 1;
   if (k >= S.nblk || i > S.J || k + i >= S.nblk || (S.jb && i > S.jb[k])) return;
@@ -384,11 +388,21 @@ __global__ void __launch_bounds__(256, 3) k_trsm(const SysDesc *__restrict__ sys
   tile_stage_mma(B, T);
   cp_async_commit();
   MmaAcc acc;
-  mma_load(acc, nullptr);
+  mma_zero(acc);
   cp_async_wait_all();
   __syncthreads();
-  mma_tn(acc, X, B, false);
-  mma_store(T, acc);
+  mma_tile<true>(acc, X, B);
+  mma_store<LDT>(S.row + (size_t)(i - 1) * TSZ, acc);
+  if (!scaled) {
+    mma_store<LDT>(T, acc);
+    return;
+  }
+  __syncthreads();  // every warp has read the staged A(k, k+i)
+  mma_store<LDM>(B, acc);
+  __syncthreads();
+  mma_zero(acc);
+  mma_tile<false>(acc, X, B);
+  mma_store<LDT>(T, acc);
 }
 
 // Trailing update inside the band: A(k+i, k+j) -= U(k,k+i)^T U(k,k+j),
@@ -404,16 +418,15 @@ __global__ void __launch_bounds__(256, 3) k_update(const SysDesc *__restrict__ s
   if (k >= S.nblk || j > S.J || k + j >= S.nblk || (S.jb && j > S.jb[k])) return;
   extern __shared__ __align__(16) double smt[];
   double *A = smt, *B = A + NB * LDM;
-  const size_t J1 = S.J + 1;
-  double *Ct = S.tiles + ((size_t)(k + j) * J1 + (j - i)) * TSZ;
-  tile_stage_mma(A, S.tiles + ((size_t)(k + i) * J1 + i) * TSZ);
-  tile_stage_mma(B, S.tiles + ((size_t)(k + j) * J1 + j) * TSZ);
+  double *Ct = S.tiles + ((size_t)(k + j) * (S.J + 1) + (j - i)) * TSZ;
+  tile_stage_mma(A, S.row + (size_t)(i - 1) * TSZ);
+  tile_stage_mma(B, S.row + (size_t)(j - 1) * TSZ);
   cp_async_commit();
   MmaAcc acc;
-  mma_load(acc, nullptr);
+  mma_zero(acc);
   cp_async_wait_all();
   __syncthreads();
-  mma_tn(acc, A, B, false);
+  mma_tile<true>(acc, A, B);
   mma_sub_store(Ct, acc);
 }
 
@@ -492,14 +505,16 @@ size_t System::bytes() const {
 
 int system_check_status(System &S) { return S.status.p ? check_status(S.status) : SX_OK; }
 
-int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync) {
+int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync, bool scaled) {
   if (systems.empty()) return SX_OK;
   std::vector<SysDesc> hd(systems.size());
   int maxblk = 0, maxJ = 0;
+  size_t rows = 0;
   for (size_t s = 0; s < systems.size(); s++) {
     System &S = *systems[s];
     const sx_mesh_s &Mh = *S.mesh;
-    hd[s] = SysDesc{S.tiles.p, S.dinv.p, S.nblk, S.J, S.status.p, Mh.denv.p + Mh.env_nblk};
+    hd[s] = SysDesc{S.tiles.p, S.dinv.p, S.nblk, S.J, S.status.p, Mh.denv.p + Mh.env_nblk, nullptr};
+    rows += S.J;
     maxblk = std::max(maxblk, S.nblk);
     maxJ = std::max(maxJ, S.J);
   }
@@ -510,6 +525,9 @@ int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync) {
     for (int k = 0; k < Sp->nblk; k++)
       rowmax[k] = std::max(rowmax[k], std::min(std::min(Sp->J, Mh.env[Mh.env_nblk + k]), Sp->nblk - 1 - k));
   }
+  DBuf<double> rowbuf;
+  SX_TRY(rowbuf.alloc_on(rows * TSZ, st));
+  for (size_t s = 0, o = 0; s < systems.size(); o += systems[s]->J, s++) hd[s].row = rowbuf.p + o * TSZ;
   DBuf<SysDesc> dd;
   SX_TRY(dd.upload_on(hd.data(), hd.size(), st));
   std::vector<int2> pairs;
@@ -517,7 +535,7 @@ int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync) {
     for (int i = 1; i <= j; i++) pairs.push_back(make_int2(i, j));
   DBuf<int2> dpairs;
   if (!pairs.empty()) SX_TRY(dpairs.upload_on(pairs.data(), pairs.size(), st));
-  const size_t smm = 2 * NB * LDM * sizeof(double), sm2 = 2 * TSZ * sizeof(double);
+  const size_t smm = 2 * NB * LDM * sizeof(double), sm2 = 2 * NB * PLD * sizeof(double);
   SX_CUDA(cudaFuncSetAttribute(k_potrf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
   SX_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm));
   SX_CUDA(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm));
@@ -527,7 +545,7 @@ int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync) {
     const int m = rowmax[k];
     if (m > 0) {
       // pairs are listed by j, so those with j <= m come first
-      k_trsm<<<dim3(m, ns), 256, smm, st>>>(dd.p, k);
+      k_trsm<<<dim3(m, ns), 256, smm, st>>>(dd.p, k, scaled);
       k_update<<<dim3((unsigned)(m * (m + 1) / 2), ns), 256, smm, st>>>(dd.p, k, dpairs.p);
     }
   }
@@ -612,12 +630,22 @@ int system_build_jacobi_diag(System &S, cudaStream_t st, bool sync) {
   return SX_OK;
 }
 
-// Copy the factor out of the tiles into LAPACK "U" band storage, ldab = nband.
+// The factor U in LAPACK "U" band storage, ldab = nband.  The resident tiles
+// hold it scaled, and U_kk times a scaled tile would give rounding noise where
+// U is exactly zero: the system is assembled and factored once more, keeping U.
 int system_band_export(const System &S, double *ab) {
   const sx_mesh_s &Mh = *S.mesh;
   const int nband = Mh.nband, kd = nband - 1;
-  std::vector<double> t((size_t)S.tiles.n);
-  SX_CUDA(cudaMemcpy(t.data(), S.tiles.p, t.size() * 8, cudaMemcpyDeviceToHost));
+  System X;
+  X.mesh = S.mesh;
+  X.lambda2 = S.lambda2;
+  X.betak2 = S.betak2;
+  X.pool = S.pool;
+  SX_TRY(system_build_direct(X, 0));
+  std::vector<System *> one(1, &X);
+  if (X.nsolve > 0) SX_TRY(factor_batch(one, 0, true, false));
+  std::vector<double> t((size_t)X.tiles.n);
+  SX_CUDA(cudaMemcpy(t.data(), X.tiles.p, t.size() * 8, cudaMemcpyDeviceToHost));
   std::memset(ab, 0, sizeof(double) * (size_t)S.nsolve * nband);
   for (int n = 0; n < S.nsolve; n++)
     for (int m = std::max(0, n - kd); m <= n; m++) ab[(size_t)n * nband + kd + m - n] = t[tile_addr(m, n, S.J)];

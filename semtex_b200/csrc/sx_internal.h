@@ -20,12 +20,12 @@ constexpr double EPSSP = 6.0e-7;
 constexpr double EPSDP = 6.0e-14;
 
 // Band tiles: the condensed matrix is held as nb x nb tiles; tile (k, j)
-// holds U(rows of block k-j, cols of block k).  Rows are padded to
-// LDT = NB + 1 doubles so that both row- and column-wise smem traversals
-// are free of bank conflicts.
+// holds the rows of block k-j and the columns of block k.  Rows are not
+// padded: the sweeps read whole rows (512 contiguous bytes a warp) in both
+// directions.
 constexpr int NB = 64;
-constexpr int LDT = NB + 1;
-constexpr int TSZ = NB * LDT;  // doubles per tile (33280 B, 16-B multiple)
+constexpr int LDT = NB;
+constexpr int TSZ = NB * LDT;  // doubles per tile (32768 B)
 
 constexpr int NP_MIN = 3;
 constexpr int NP_MAX = 12;
@@ -246,7 +246,7 @@ struct System {
   bool singular = false;
   int nsolve = 0;
   int nblk = 0, J = 0;     // band tiles: nblk block columns, J off-diagonal tiles
-  DBuf<double> tiles;      // nblk*(J+1)*TSZ
+  DBuf<double> tiles;      // nblk*(J+1)*TSZ: U_kk, and U_bb^-1 U(b, k) off the diagonal
   DBuf<double> dinv;       // nblk*TSZ: inverse of the diagonal U tiles
   DBuf<double> hbi;        // nel*next*nint  (hbi hii^-1, row-major next x nint)
   DBuf<double> hii;        // nel*nint*nint  (hii^-1, column-major)

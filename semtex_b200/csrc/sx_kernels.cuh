@@ -12,6 +12,7 @@ struct SysDesc {
   int nblk, J;
   int *status;
   const int *jb;  // tiles right of the diagonal in each block row (null: J)
+  double *row;    // J*TSZ: U's tiles of the block row being factored
 };
 
 // Address of U(m, n), m <= n, n - m <= kd, inside the tile array.
@@ -34,6 +35,8 @@ __device__ __forceinline__ float warp_sumf(float v) {
 
 // Factor the systems' bands, all systems in each launch; sync = false
 // returns without waiting (statuses to be checked after st completes).
-int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync = true);
+// scaled: off-diagonal tiles as the sweeps read them, U_kk^-1 U(k, k+i); else
+// U's own.
+int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync = true, bool scaled = true);
 
 }  // namespace sx

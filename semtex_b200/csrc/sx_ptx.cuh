@@ -24,10 +24,26 @@ __device__ __forceinline__ void fence_mbar_init_cluster() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-__device__ __forceinline__ void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
-
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The two halves of cluster_sync_all (each by whole warps).
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Barrier `id` (1-15) over `threads` threads of the CTA (whole warps).
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
@@ -69,6 +85,41 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long l
   if (mbar_try_wait_cluster(bar, parity)) return true;
   const long long t0 = clock64();
   while (!mbar_try_wait_cluster(bar, parity))
+    if (clock64() - t0 > limit_cycles) return false;
+  return true;
+}
+
+// The same wait for this CTA's own threads or for bytes that complete on the
+// barrier itself (bulk copies, st.async): the phase's completion makes them
+// visible, and no acquire wider than the CTA is needed.
+__device__ __forceinline__ bool mbar_try_wait_cta(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// One non-blocking probe of such a phase.
+__device__ __forceinline__ bool mbar_test_cta(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_tx(uint64_t *bar, uint32_t parity, long long limit_cycles) {
+  if (limit_cycles <= 0) return mbar_test_cta(bar, parity);
+  if (mbar_try_wait_cta(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait_cta(bar, parity))
     if (clock64() - t0 > limit_cycles) return false;
   return true;
 }
@@ -136,12 +187,13 @@ __device__ __forceinline__ uint32_t map_rank(const void *p, uint32_t rank) {
   return r;
 }
 
-__device__ __forceinline__ void st_cluster_f64(uint32_t addr, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+// Asynchronous store of v to `addr` in another CTA's shared memory; its
+// eight bytes complete on that CTA's barrier `bar` (both from map_rank), and
+// whoever waits for the barrier's phase sees them.
+__device__ __forceinline__ void st_async_f64(uint32_t addr, double v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(addr), "d"(v),
+               "r"(bar)
+               : "memory");
 }
 
 }  // namespace sx

@@ -121,7 +121,7 @@ size_t system_estimate(const MeshCopy &m, int kind) {
   size_t b = npts * 12;  // Jacobi diagonal, FP64 + FP32
   if (kind == SX_DIRECT) {
     const size_t nblk = (m.nsolve + NB - 1) / NB, J = (m.nband - 1 + NB - 1) / NB;
-    b += (nblk * (J + 2)) * TSZ * 8 + (size_t)m.nel * (next * nint + nint * nint) * 8;
+    b += (nblk * (J + 2) + J) * TSZ * 8 + (size_t)m.nel * (next * nint + nint * nint) * 8;
   }
   return b;
 }

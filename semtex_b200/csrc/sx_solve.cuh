@@ -71,12 +71,11 @@ __device__ __forceinline__ void helm_op(const T *D, const T *Q1, const T *Q2, co
 
 // Direct solve of all jobs; the band sweeps run one cluster of C CTAs per job.
 // Returns the number of kernels launched through *launches when non-null.
-// Ring depth (tiles in flight per CTA) of the band sweeps: at most 4; 2
-// lets two CTAs share an SM, so that larger clusters stay resident.
+// Ring depth (tiles in flight per CTA) of the band sweeps: at most 4.
 constexpr int BAND_STAGES_MAX = 4;
 // Schedule of one band-sweep launch: C CTAs per system's cluster, S tiles in
-// flight per CTA, and the leader's share of the tiles j >= 2: Q = 0 none,
-// Q = K >= 2 the last of every K of them (worked on a step ahead).
+// flight per CTA, and the leader's share of the ranks' tiles (j >= 3): Q = 0
+// none, Q = K >= 2 the last of every K of them (worked on a step ahead).
 struct BandSched {
   int C = 1, S = BAND_STAGES_MAX, Q = 0;
   bool operator==(const BandSched &o) const { return C == o.C && S == o.S && Q == o.Q; }
@@ -98,14 +97,13 @@ int prepare_band_kernels();
 constexpr long long SWEEP_WAIT_DEFAULT = 4000000000LL, CG_WAIT_DEFAULT = 2000000000LL;
 int set_sweep_wait_limit(long long cycles);
 int set_cg_wait_limit(long long cycles);
-int pick_cluster(int nj, int cmax, int pmax, int Wmax, int *stages_out = nullptr, int stages_forced = 0);
+int pick_cluster(int nj, int cmax, int J, int *stages_out = nullptr, int stages_forced = 0);
 // Default leader share Q (0 or a cycle length K >= 2) of a cluster of C CTAs
 // on a band of J off-diagonal tiles per block column.
 int default_lead(int C, int J);
 // Clusters of C band-sweep CTAs that can be resident at once (0: C does not
 // fit an SM group, so a launch with it would fail).
-int band_active_clusters(int C, int pmax, int Wmax, int stages = BAND_STAGES_MAX);
-size_t sweep_smem(int pmax, int C, int S, int Wmax);
+int band_active_clusters(int C, int J, int stages = BAND_STAGES_MAX);
 // Set kernel attributes (max dynamic smem) ahead of any stream capture.
 int prepare_direct_kernels(const MeshView &M);
 
