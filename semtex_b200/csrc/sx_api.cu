@@ -327,7 +327,6 @@ static int reserve_ws(sx_modal_s &M, int planes) {
   if (M.rhs.n < (size_t)planes * npad) SX_TRY(M.rhs.alloc_in((size_t)planes * npad, M.pool, st));
   if (M.Fb.n < (size_t)planes * Mh.nel * Mh.next)
     SX_TRY(M.Fb.alloc_in((size_t)planes * Mh.nel * Mh.next, M.pool, st));
-  if (M.gess.n < (size_t)planes * Mh.nglobal) SX_TRY(M.gess.alloc_in((size_t)planes * Mh.nglobal, M.pool, st));
   return SX_OK;
 }
 
@@ -357,7 +356,6 @@ static Job make_job(sx_modal_s &M, const Group &g, int slot, double *u, double *
   j.rhs_stride = (long long)M.npad_max;
   j.rhs = M.rhs.p + (size_t)slot * M.npad_max;
   j.Fb = M.Fb.p + (size_t)slot * Mh.nel * Mh.next;
-  j.gess = M.gess.p + (size_t)slot * Mh.nglobal;
   j.pc = S.pc.p;
   j.status = M.dstatus.p;
   return j;
@@ -452,8 +450,7 @@ static int direct_batched(sx_modal_s *s, DirectBatch &B, const std::vector<Group
   }
   SX_TRY(reserve_ws(*s, planes));
   const bool same = B.exec && B.key[0] == d_u && B.key[1] == d_f && B.key[2] == d_bc && B.key[3] == s->rhs.p &&
-                    B.key[4] == s->Fb.p && B.key[5] == s->gess.p && B.nz == nz && B.stride == plane_stride &&
-                    B.modes == modes;
+                    B.key[4] == s->Fb.p && B.nz == nz && B.stride == plane_stride && B.modes == modes;
   const MeshView M = s->mesh->view();
   if (!same || !s->use_graphs) {
     B.reset();
@@ -489,7 +486,6 @@ static int direct_batched(sx_modal_s *s, DirectBatch &B, const std::vector<Group
     B.key[2] = d_bc;
     B.key[3] = s->rhs.p;
     B.key[4] = s->Fb.p;
-    B.key[5] = s->gess.p;
     B.nz = nz;
     B.stride = plane_stride;
   }
@@ -1019,7 +1015,6 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
     key_ptr(key, q.bc);
     key_ptr(key, q.s->rhs.p);
     key_ptr(key, q.s->Fb.p);
-    key_ptr(key, q.s->gess.p);
     key.push_back(q.nz);
     key.push_back(q.stride);
     key.push_back(q.s->forced_cluster);

@@ -174,6 +174,7 @@ struct MeshView {
   const int *b_elmt, *b_side, *b_kind;
   const double *b_K, *b_C, *b_area;      // b_area: nbound*np
   const int *nat_ptr, *nat_idx;          // CSR: global node -> (b*np+i) natural/mixed terms
+  const int *ess_src;                    // nglobal: the b*np+i whose essential value the node takes, -1 none
   int mixed;                             // any mixed boundary
 };
 
@@ -206,7 +207,7 @@ struct sx_mesh_s {
   sx::DBuf<unsigned char> dhasQ3;
   sx::DBuf<int> dpmap;
   sx::DBuf<int> demap, dbtog, dbmask, demask, dg2e_ptr, dg2e_idx, dg2e_last, dbe, dbs, dbk;
-  sx::DBuf<int> dnat_ptr, dnat_idx, dcolour_elmt;
+  sx::DBuf<int> dnat_ptr, dnat_idx, dess_src, dcolour_elmt;
   sx::DBuf<int4> dg2e4, de2w4;
   sx::DBuf<float4> dGf;
   // max over nodes of the assembled stiffness diagonal over the assembled
@@ -314,7 +315,6 @@ struct Work {
   int planes = 0;
   DBuf<double> Fb;      // planes*nel*next condensed element boundary forcing
   DBuf<double> rhs;     // planes*npad
-  DBuf<double> gess;    // planes*nglobal essential values
   DBuf<int> status;     // device status word
   int reserve(const sx_mesh_s &M, int planes, int npad);
 };

@@ -215,7 +215,7 @@ sx::MeshView sx_mesh_s::view() const {
   v.e2w4 = de2w4.p; v.Gf = dGf.p; v.pmap = dpmap.p;
   v.nbound = nbound; v.b_elmt = dbe.p; v.b_side = dbs.p; v.b_kind = dbk.p;
   v.b_K = dK.p; v.b_C = dC.p; v.b_area = darea.p;
-  v.nat_ptr = dnat_ptr.p; v.nat_idx = dnat_idx.p;
+  v.nat_ptr = dnat_ptr.p; v.nat_idx = dnat_idx.p; v.ess_src = dess_src.p;
   v.mixed = mixed ? 1 : 0;
   return v;
 }
@@ -514,6 +514,13 @@ extern "C" int sx_mesh_create(const sx_mesh_desc *d, sx_mesh *out) {
     }
     if (nidx.empty()) nidx.push_back(0);
   }
+  // The boundary-line value each essential node takes: where two boundaries
+  // meet, the later one's, as the reference's loop over them overwrites
+  // (getEssential, src/field.cpp:994-1019).
+  std::vector<int> ess(d->nglobal, -1);
+  for (int b = 0; b < nb; b++)
+    if (M->b_kind[b] == SX_BC_ESSENTIAL)
+      for (int i = 0; i < np; i++) ess[bnd_node(*M, b, i)] = b * np + i;
   // Greedy element colouring: elements of one colour share no global node.
   {
     std::vector<int> colour(nel, -1);
@@ -627,6 +634,7 @@ extern "C" int sx_mesh_create(const sx_mesh_desc *d, sx_mesh *out) {
   SX_TRY(M->darea.upload_in(M->b_area.data(), M->b_area.size(), up.pool, up.s));
   SX_TRY(M->dnat_ptr.upload_in(nptr.data(), nptr.size(), up.pool, up.s));
   SX_TRY(M->dnat_idx.upload_in(nidx.data(), nidx.size(), up.pool, up.s));
+  SX_TRY(M->dess_src.upload_in(ess.data(), ess.size(), up.pool, up.s));
   SX_TRY(M->dcolour_elmt.upload_in(M->colour_elmt.data(), M->colour_elmt.size(), up.pool, up.s));
   *out = M.release();
   return SX_OK;

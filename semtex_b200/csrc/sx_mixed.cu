@@ -255,36 +255,6 @@ static int ensure_constD() {
 // RHS (FP64)
 // ---------------------------------------------------------------------------
 
-// Essential values of plane p into gess (Boundary::set through btog,
-// src/boundary.cpp:50-64); one thread per plane.
-__device__ __forceinline__ void ess_body(const MxMember &B, int p) {
-  const MeshView &M = B.M;
-  const MxParams &P = B.P;
-  if (threadIdx.x || !P.bc || !real_plane(P, p)) return;
-  const int np = M.np, nm = np - 1;
-  double *g = P.gess + (size_t)p * M.nglobal;
-  const double *bc = P.bc + (size_t)p * P.bcstride;
-  for (int b = 0; b < M.nbound; b++) {
-    if (M.b_kind[b] != SX_BC_ESSENTIAL) continue;
-    const int *bmap = M.btog + (size_t)M.b_elmt[b] * M.next;
-    const int side = M.b_side[b];
-    const double *src = bc + (size_t)b * np;
-    for (int i = 0; i < nm; i++) g[bmap[side * nm + i]] = src[i];
-    if (side == 3)
-      g[bmap[0]] = src[nm];
-    else
-      g[bmap[side * nm + nm]] = src[nm];
-  }
-}
-
-__global__ void k_x_ess(const __grid_constant__ MxMember B) { ess_body(B, blockIdx.x); }
-
-__global__ void k_x_ess_multi(MxTable T) {
-  __shared__ MxMember sB;
-  int t;
-  if (tile_member(T, sB, t)) ess_body(sB, t);
-}
-
 // (A_e u)(w, j), j = 0..NP-1, in FP64 for the calling warp's tensor row w
 // and lane's plane, on tensor lines as in k_cg: warp w holds row w (the
 // x-derivative terms) and column w (the y-derivative terms) in registers,
@@ -394,12 +364,12 @@ __device__ __forceinline__ void constrain_body(const MxMember &B, int e, int y) 
 #pragma unroll
   for (int j = 0; j < NP; j++) F[j] = M.Q8[eo + w * NP + j] * T[lane * TS + w * NP + j];
   if (M.emask[e]) {  // block-uniform: H g, g the essential values
-    const double *g = P.gess + (size_t)p * M.nglobal;
     const bool rp = real_plane(P, p);
+    const double *bc = P.bc && rp ? P.bc + (size_t)p * P.bcstride : nullptr;
 #pragma unroll
     for (int k = 0; k < NP; k++) {
       const int a = w + k * NP;
-      B0[emt[a] * MX_CH + lane] = (rp && a < NE) ? g[gtab[a]] : 0.0;
+      B0[emt[a] * MX_CH + lane] = (rp && a < NE) ? ess_value(M, bc, gtab[a]) : 0.0;
     }
     __syncthreads();
     double hg[NP];
@@ -917,7 +887,7 @@ __global__ void __launch_bounds__(256) k_x_res_multi(MxTable T) {
   if (tile_member(T, sB, t)) res_body(sB, t % sB.G, t / sB.G);
 }
 
-// u = x at element nodes, essential values from gess (global2local +
+// u = x at element nodes, essential values from the boundary lines (global2local +
 // setEssential, src/field.cpp:710-713, 1022-1040); transposed back to the
 // caller's plane-major layout through shared memory.
 template <int NP>
@@ -936,11 +906,12 @@ __device__ __forceinline__ void unpack_body(const MxMember &B, int e, int y) {
   for (int i = tid; i < NN; i += 256) emap[i] = M.emap[i];
   __syncthreads();
   const bool masked = M.emask[e] != 0;
+  const double *bc = P.bc && real_plane(P, p) ? P.bc + (size_t)p * P.bcstride : nullptr;
   for (int a = row; a < NN; a += MX_ROWS) {
     double v;
     if (a < NE) {
       const int g = M.btog[(size_t)e * NE + a];
-      v = (masked && M.bmask[(size_t)e * NE + a]) ? P.gess[(size_t)p * M.nglobal + g] : x64[(size_t)g * PP + p];
+      v = (masked && M.bmask[(size_t)e * NE + a]) ? ess_value(M, bc, g) : x64[(size_t)g * PP + p];
     } else {
       v = x64[((size_t)M.nglobal + (size_t)e * M.nint + (a - NE)) * PP + p];
     }
@@ -1060,16 +1031,11 @@ static MxMember member_of(const MeshView &M, MixedWork &W) {
   return B;
 }
 
-static int enqueue_init(const MeshView &M, MixedWork &W, bool any_bc, cudaStream_t st, int *nl) {
+static int enqueue_init(const MeshView &M, MixedWork &W, cudaStream_t st, int *nl) {
   const MxMember B = member_of(M, W);
-  *nl = 0;
-  if (any_bc) {
-    k_x_ess<<<W.PP, 32, 0, st>>>(B);
-    (*nl)++;
-  }
   SX_NP_SWITCH_M(M.np, (k_x_constrain<N_><<<dim3(M.nel, B.nch), N_ * 32, x64_smem(N_), st>>>(B)));
   k_x_rhs<<<dim3(W.G, B.nch), 256, 0, st>>>(B);
-  *nl += 2;
+  *nl = 2;
   SX_CUDA(cudaGetLastError());
   return SX_OK;
 }
@@ -1170,7 +1136,6 @@ static int setup(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &gr
     SX_TRY(need(W.pcE, ne / 2));
     SX_TRY(need(W.scal, (size_t)MX_NSCAL * PP));
     SX_TRY(need(W.hcon, (size_t)PP));
-    SX_TRY(need(W.gess, (size_t)PP * M.nglobal));
     SX_TRY(need(W.nsolve, (size_t)PP));
     SX_TRY(need(W.active, (size_t)PP));
     SX_TRY(need(W.skip, (size_t)PP / MX_CH));
@@ -1232,7 +1197,6 @@ static void bind_params(const MeshView &M, MixedWork &W, int nz, double *d_u, do
   P.stride = stride;
   P.bc = d_bc;
   P.bcstride = (long long)std::max(M.nbound, 1) * M.np;
-  P.gess = W.gess.p;
 }
 
 // Largest relative residual over the planes of one member from its norms
@@ -1268,8 +1232,7 @@ int mixed_solve(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &gro
     SX_TRY(attr_rc);
     bind_params(M, W, nz, d_u, d_f, d_bc, stride);
     if (graphs) {
-      const bool any_bc = d_bc != nullptr;
-      SX_TRY(capture(st, &W.g_init, [&]() { return enqueue_init(M, W, any_bc, st, &W.launches_init); }));
+      SX_TRY(capture(st, &W.g_init, [&]() { return enqueue_init(M, W, st, &W.launches_init); }));
       SX_TRY(capture(st, &W.g_round,
                      [&]() { return enqueue_round(M, W, n_inner, check_stop, st, &W.launches_round); }));
     }
@@ -1277,12 +1240,10 @@ int mixed_solve(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &gro
     W.check_stop = check_stop;
     W.graph_epoch = W.epoch;
   }
-  // essential values: zeroed here, set from the BC lines inside g_init
-  SX_CUDA(cudaMemsetAsync(W.gess.p, 0, sizeof(double) * (size_t)W.PP * M.nglobal, st));
   if (graphs)
     SX_CUDA(cudaGraphLaunch(W.g_init, st));
   else
-    SX_TRY(enqueue_init(M, W, d_bc != nullptr, st, &W.launches_init));
+    SX_TRY(enqueue_init(M, W, st, &W.launches_init));
   int rounds = 0, launches = W.launches_init + 1;
   double worst = 0.0;
   const int PP = W.PP;
@@ -1335,7 +1296,7 @@ MxBatch::~MxBatch() {
   for (cudaStream_t s : streams) cudaStreamDestroy(s);
 }
 
-// The three tile tables of class c: element, node and plane tiles.
+// The two tile tables of class c: element and node tiles.
 static MxTable class_table(const MxBatch &B, const MxBatch::Class &c, int kind) {
   MxTable T;
   T.mem = B.mem.p + c.m0;
@@ -1379,11 +1340,9 @@ static int per_class(MxBatch &B, cudaStream_t st,
   return rc;
 }
 
-static int enqueue_init_multi(MxBatch &B, bool any_bc, cudaStream_t st, int *nl) {
-  *nl = 0;
-  for (auto &c : B.cls) *nl += any_bc ? 3 : 2;
+static int enqueue_init_multi(MxBatch &B, cudaStream_t st, int *nl) {
+  *nl = 2 * (int)B.cls.size();
   return per_class(B, st, [&](const MxBatch::Class &c, cudaStream_t s) {
-    if (any_bc) k_x_ess_multi<<<c.tp, 32, 0, s>>>(class_table(B, c, 2));
     SX_NP_SWITCH_M(c.np, (k_x_constrain_multi<N_><<<c.te, N_ * 32, x64_smem(N_), s>>>(class_table(B, c, 0))));
     k_x_rhs_multi<<<c.tn, 256, 0, s>>>(class_table(B, c, 1));
     SX_CUDA(cudaGetLastError());
@@ -1430,8 +1389,6 @@ int mixed_solve_multi(std::vector<MxItem> &items, MxBatch &B, bool rebuild, doub
     if (it.groups.empty() || !it.W) return SX_ERR_ARG;
   }
   SX_TRY(ensure_constD());
-  bool any_bc = false;
-  for (const MxItem &it : items) any_bc |= it.bc != nullptr;
   bool stale = (int)B.order.size() != n || B.epochs.size() != B.order.size();
   for (int m = 0; !stale && m < n; m++) stale = items[B.order[m]].W->epoch != B.epochs[m];
   if (rebuild || stale || !graphs || !B.g_init || B.n_inner != n_inner || B.check_stop != check_stop) {
@@ -1471,19 +1428,16 @@ int mixed_solve_multi(std::vector<MxItem> &items, MxBatch &B, bool rebuild, doub
     }
     for (auto &c : B.cls) {
       c.t0 = tiles.size();
-      std::vector<int> te(1, 0), tn(1, 0), tp(1, 0);
+      std::vector<int> te(1, 0), tn(1, 0);
       for (int m = c.m0; m < c.m0 + c.count; m++) {
         const MxMember &b = mem[m];
         te.push_back(te.back() + b.M.nel * b.nch);
         tn.push_back(tn.back() + b.G * b.nch);
-        tp.push_back(tp.back() + b.P.PP);
       }
       c.te = te.back();
       c.tn = tn.back();
-      c.tp = tp.back();
       tiles.insert(tiles.end(), te.begin(), te.end());
       tiles.insert(tiles.end(), tn.begin(), tn.end());
-      tiles.insert(tiles.end(), tp.begin(), tp.end());
     }
     B.epochs.clear();
     for (int m = 0; m < n; m++) B.epochs.push_back(items[B.order[m]].W->epoch);
@@ -1494,20 +1448,17 @@ int mixed_solve_multi(std::vector<MxItem> &items, MxBatch &B, bool rebuild, doub
     SX_CUDA(cudaStreamSynchronize(st));
     SX_TRY(ensure_streams(B));
     if (graphs) {
-      SX_TRY(capture(st, &B.g_init, [&]() { return enqueue_init_multi(B, any_bc, st, &B.launches_init); }));
+      SX_TRY(capture(st, &B.g_init, [&]() { return enqueue_init_multi(B, st, &B.launches_init); }));
       SX_TRY(capture(st, &B.g_round,
                      [&]() { return enqueue_round_multi(B, n_inner, check_stop, st, &B.launches_round); }));
     }
     B.n_inner = n_inner;
     B.check_stop = check_stop;
   }
-  // essential values: zeroed here, set from the BC lines inside the init
-  for (const MxItem &it : items)
-    SX_CUDA(cudaMemsetAsync(it.W->gess.p, 0, sizeof(double) * (size_t)it.W->PP * it.M.nglobal, st));
   if (graphs)
     SX_CUDA(cudaGraphLaunch(B.g_init, st));
   else
-    SX_TRY(enqueue_init_multi(B, any_bc, st, &B.launches_init));
+    SX_TRY(enqueue_init_multi(B, st, &B.launches_init));
   int rounds = 0, launches = B.launches_init + (int)B.cls.size();
   std::vector<double> worst(n, 0.0);
   for (rounds = 1; rounds <= max_refine; rounds++) {

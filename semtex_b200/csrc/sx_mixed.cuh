@@ -26,7 +26,6 @@ struct MxParams {
   long long stride;     // plane stride of f and u
   const double *bc;     // bc lines per plane or nullptr
   long long bcstride;
-  double *gess;         // [PP * nglobal] essential values, plane-major
 };
 
 // Per-plane scalars, each an array of PP doubles: residual and RHS norms
@@ -80,7 +79,7 @@ struct MxMember {
 
 struct MixedWork {
   int PP = 0, npts = 0, n_inner = 0, M = 0, G = 0;
-  DBuf<double> hcon, b64, x64, Ye64, scal, part, gess;
+  DBuf<double> hcon, b64, x64, Ye64, scal, part;
   DBuf<int> nsolve, active, skip;
   DBuf<unsigned> cnt;
   DBuf<float> pcf, r0, rE, sE, pE, dE, WE0, WE1, pcE;
@@ -136,13 +135,13 @@ struct MxItem {
 // Device tables, streams and graphs of a multi-mesh mixed-precision solve.
 // Members are ordered by element order; the members of one order form a
 // class, and every kernel runs once per class over all its members' tiles
-// (element tiles: nel * nch per member; node tiles: G * nch; plane tiles:
-// PP), the classes on their own streams side by side.
+// (element tiles: nel * nch per member; node tiles: G * nch), the classes on
+// their own streams side by side.
 struct MxBatch {
   struct Class {
     int np = 0, m0 = 0, count = 0;  // order, first member, members
-    int te = 0, tn = 0, tp = 0;     // element, node and plane tiles
-    size_t t0 = 0;                  // offset of the 3 (count + 1) tile prefixes
+    int te = 0, tn = 0;             // element and node tiles
+    size_t t0 = 0;                  // offset of the 2 (count + 1) tile prefixes
   };
   DBuf<MxMember> mem;
   DBuf<int> tiles;

@@ -19,7 +19,7 @@ namespace sx {
 // arguments it was captured for stay the same.
 struct DirectBatch {
   cudaGraphExec_t exec = nullptr;
-  const void *key[6] = {};  // u, f, bc, and the workspace buffers rhs, Fb, gess
+  const void *key[5] = {};  // u, f, bc, and the workspace buffers rhs, Fb
   int nz = 0, stride = 0;
   std::vector<int> modes;  // local mode of each group, in job order
   DBuf<Job> djobs;
@@ -45,7 +45,7 @@ struct sx_modal_s {
   std::vector<std::shared_ptr<sx::System>> sys;   // per local mode
   std::vector<std::shared_ptr<sx::System>> uniq;  // distinct systems
   // solve workspace, sized for all planes at once
-  sx::DBuf<double> rhs, Fb, gess;
+  sx::DBuf<double> rhs, Fb;
   sx::PcgWork pcg;
   sx::DBuf<sx::Job> djobs;
   size_t npad_max = 0;

@@ -186,7 +186,7 @@ __global__ void k_op_dss(MeshView M, const double *__restrict__ Ye, const double
 // constrain (src/field.cpp:728-768): Ye[e] = -(M f + H g) in emap order.
 template <int NP>
 __global__ void __launch_bounds__(128) k_constrain(MeshView M, double hCon, const double *__restrict__ f,
-                                                   const double *__restrict__ gess, double *__restrict__ Ye) {
+                                                   const double *__restrict__ bc, double *__restrict__ Ye) {
   constexpr int NN = NP * NP, NE = 4 * (NP - 1);
   const int e = blockIdx.x, tid = threadIdx.x;
   __shared__ double D[NN], Q[4][NN], u[NN], R[NN], S[NN], out[NN], F[NN];
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(128) k_constrain(MeshView M, double hCon, cons
   }
   __syncthreads();
   if (M.emask[e]) {
-    for (int a = tid; a < NE; a += 128) u[emap[a]] = gess[M.btog[(size_t)e * NE + a]];
+    for (int a = tid; a < NE; a += 128) u[emap[a]] = ess_value(M, bc, M.btog[(size_t)e * NE + a]);
     __syncthreads();
     helm_op<NP, double>(D, Q[0], Q[1], Q[2], Q[3], M.hasQ3[e] != 0, hCon, u, R, S, out, 128);
     for (int i = tid; i < NN; i += 128) F[i] += out[i];
@@ -234,34 +234,18 @@ __global__ void k_l2g(MeshView M, const double *__restrict__ u, double *x) {
 }
 
 // global2local + setEssential (src/field.cpp:710-713, 1022-1040).
-__global__ void k_g2l(MeshView M, const double *__restrict__ x, const double *__restrict__ gess, double *u) {
+__global__ void k_g2l(MeshView M, const double *__restrict__ x, const double *__restrict__ bc, double *u) {
   const int e = blockIdx.x;
   const size_t eo = (size_t)e * M.npnp;
   for (int a = threadIdx.x; a < M.npnp; a += blockDim.x) {
     double v;
     if (a < M.next) {
       const int g = M.btog[(size_t)e * M.next + a];
-      v = (M.emask[e] && M.bmask[(size_t)e * M.next + a]) ? gess[g] : x[g];
+      v = (M.emask[e] && M.bmask[(size_t)e * M.next + a]) ? ess_value(M, bc, g) : x[g];
     } else {
       v = x[M.nglobal + (size_t)e * M.nint + (a - M.next)];
     }
     u[eo + M.emap[a]] = v;
-  }
-}
-
-__global__ void k_essential_one(MeshView M, const double *__restrict__ bc, double *g) {
-  if (threadIdx.x || blockIdx.x) return;
-  const int np = M.np, nm = np - 1;
-  for (int b = 0; b < M.nbound; b++) {
-    if (M.b_kind[b] != SX_BC_ESSENTIAL) continue;
-    const int *bmap = M.btog + (size_t)M.b_elmt[b] * M.next;
-    const int side = M.b_side[b];
-    const double *src = bc + (size_t)b * np;
-    for (int i = 0; i < nm; i++) g[bmap[side * nm + i]] = src[i];
-    if (side == 3)
-      g[bmap[0]] = src[nm];
-    else
-      g[bmap[side * nm + nm]] = src[nm];
   }
 }
 
@@ -304,12 +288,9 @@ int pcg_solve_job(const MeshView &M, const System &S, PcgWork &W, const Job &job
     double *u = job.u + (size_t)p * job.ustride;
     const double *f = job.f + (size_t)p * job.fstride;
     const double *bc = job.bc ? job.bc + (size_t)p * job.bcstride : nullptr;
-    double *g = job.gess + (size_t)p * M.nglobal;
-    SX_CUDA(cudaMemsetAsync(g, 0, sizeof(double) * M.nglobal, st));
-    if (bc) k_essential_one<<<1, 1, 0, st>>>(M, bc, g);
     SX_CUDA(cudaMemsetAsync(sc, 0, sizeof(double) * 16, st));
     // RHS
-    SX_NP_SWITCH(M.np, (k_constrain<N_><<<M.nel, 128, 0, st>>>(M, hCon, f, g, W.Ye.p)));
+    SX_NP_SWITCH(M.np, (k_constrain<N_><<<M.nel, 128, 0, st>>>(M, hCon, f, bc, W.Ye.p)));
     k_op_dss<<<vb, 256, 0, st>>>(M, W.Ye.p, nullptr, bc, 1, W.r.p);
     if (nzero > 0) k_zero_range<<<(nzero + 255) / 256, 256, 0, st>>>(W.r.p, nsolve, M.nglobal);
     k_dot<<<gb, 256, 0, st>>>(W.r.p, W.r.p, nullptr, npts, W.part.p);
@@ -351,7 +332,7 @@ int pcg_solve_job(const MeshView &M, const System &S, PcgWork &W, const Job &job
       const int bodies = (i == step_max) ? i - 1 : i;
       *launches += 10 + 3 * zr + (bc ? 1 : 0) + bodies * (9 + zr) + 1;
     }
-    k_g2l<<<M.nel, 128, 0, st>>>(M, W.x.p, g, u);
+    k_g2l<<<M.nel, 128, 0, st>>>(M, W.x.p, bc, u);
     SX_CUDA(cudaGetLastError());
     *iters_max = std::max(*iters_max, i);
     const double b2 = epsb2 / (tol_rel * tol_rel);

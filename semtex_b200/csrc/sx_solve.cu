@@ -5,8 +5,6 @@
 // of a Fourier mode).  Every kernel takes an array of jobs (grid.y = job), so
 // the plain form launches one job per mode and the batched form all modes
 // at once.  Per job:
-//   k_essential   getEssential: essential BC values into a global vector
-//                 (src/field.cpp:994-1019, Essential::set src/condition.cpp:80-101)
 //   k_rhs_elem    constrain  f <- -(M f + H g)  (src/field.cpp:728-768) and the
 //                 element half of local2globalSumSC: edge-major gather,
 //                 F_b -= (hbi hii^-1) F_i  (src/element.cpp:356-395)
@@ -23,32 +21,6 @@
 #include "sx_solve.cuh"
 
 namespace sx {
-
-// ---------------------------------------------------------------------------
-// Essential BC values
-// ---------------------------------------------------------------------------
-
-// One thread per plane; boundaries in order so later boundaries overwrite
-// shared corner nodes exactly as the reference's sequential loop does.
-__global__ void k_essential(MeshView M, const Job *__restrict__ jobs) {
-  const Job J = jobs[blockIdx.y];
-  const int p = threadIdx.x;
-  if (p >= J.P || J.bc == nullptr) return;
-  const double *bc = J.bc + (size_t)p * J.bcstride;
-  double *g = J.gess + (size_t)p * M.nglobal;
-  const int np = M.np, nm = np - 1;
-  for (int b = 0; b < M.nbound; b++) {
-    if (M.b_kind[b] != SX_BC_ESSENTIAL) continue;
-    const int *bmap = M.btog + (size_t)M.b_elmt[b] * M.next;
-    const int side = M.b_side[b];
-    const double *src = bc + (size_t)b * np;
-    for (int i = 0; i < nm; i++) g[bmap[side * nm + i]] = src[i];
-    if (side == 3)
-      g[bmap[0]] = src[nm];
-    else
-      g[bmap[side * nm + nm]] = src[nm];
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Element forcing and condensation
@@ -102,11 +74,11 @@ __global__ void __launch_bounds__(ELEM_WARPS * 32) k_rhs_elem(MeshView M, const 
     const bool q3 = M.hasQ3[e];
     const int *bt = M.btog + (size_t)e * NE;
     for (int p = 0; p < P; p++) {
-      const double *g = J.gess + (size_t)p * M.nglobal;
+      const double *bc = J.bc ? J.bc + (size_t)p * J.bcstride : nullptr;
       __syncthreads();
       for (int i = tid; i < NN; i += NT) u[i] = 0.0;
       __syncthreads();
-      for (int i = tid; i < NE; i += NT) u[emap[i]] = g[bt[i]];
+      for (int i = tid; i < NE; i += NT) u[emap[i]] = ess_value(M, bc, bt[i]);
       __syncthreads();
       helm_op<NP, double>(D, Q[0], Q[1], Q[2], Q[3], q3, J.hCon, u, R, S, T, NT);
       for (int i = tid; i < NN; i += NT) F[p][i] += T[i];
@@ -215,7 +187,8 @@ __global__ void __launch_bounds__(back_threads<NP>()) k_backsub(MeshView M, cons
     const int n = M.emap[b];
     const bool ess = masked && M.bmask[(size_t)e * NE + b];
     for (int p = 0; p < P; p++)
-      J.u[(size_t)p * J.ustride + eo + n] = ess ? J.gess[(size_t)p * M.nglobal + bt[b]] : ub[p][b];
+      J.u[(size_t)p * J.ustride + eo + n] =
+          ess ? ess_value(M, J.bc ? J.bc + (size_t)p * J.bcstride : nullptr, bt[b]) : ub[p][b];
   }
   if (tid < NI) {
     const int r = tid;
@@ -280,7 +253,6 @@ int direct_rhs_jobs(const MeshView &M, const Job *djobs, const std::vector<Job> 
                     int *launches) {
   const int nj = (int)hjobs.size();
   int maxpad = 0;
-  bool any_bc = false;
   for (const Job &j : hjobs) {
     // the element kernels take both planes of a mode in one pass, no more
     if (j.P < 1 || j.P > 2) {
@@ -288,14 +260,11 @@ int direct_rhs_jobs(const MeshView &M, const Job *djobs, const std::vector<Job> 
       return SX_ERR_UNSUPPORTED;
     }
     maxpad = std::max(maxpad, j.npad);
-    any_bc |= j.bc != nullptr;
-    SX_CUDA(cudaMemsetAsync(j.gess, 0, sizeof(double) * (size_t)j.P * M.nglobal, st));
   }
-  if (any_bc) k_essential<<<dim3(1, nj), 32, 0, st>>>(M, djobs);
   dispatch_elem(M, djobs, nj, true, st);
   k_rhs_dss<<<dim3((maxpad + 255) / 256, nj), 256, 0, st>>>(M, djobs);
   SX_CUDA(cudaGetLastError());
-  if (launches) *launches += (any_bc ? 1 : 0) + 2;
+  if (launches) *launches += 2;
   return SX_OK;
 }
 

@@ -24,11 +24,20 @@ struct Job {
   double *rhs;          // P * rhs_stride
   long long rhs_stride;
   double *Fb;           // P * nel * next
-  double *gess;         // P * nglobal
   // JACPCG
   const double *pc;
   int *status;          // device status bits (1 << SX_ERR_*)
 };
+
+// The essential value of global node g from a plane's boundary lines (zero
+// where no essential boundary sets it, or without lines): getEssential /
+// Essential::set (src/field.cpp:994-1019, src/condition.cpp:80-101) read
+// where it is needed, instead of a vector that a kernel fills first.
+__device__ __forceinline__ double ess_value(const MeshView &M, const double *bc, int g) {
+  if (!bc) return 0.0;
+  const int s = M.ess_src[g];
+  return s >= 0 ? bc[s] : 0.0;
+}
 
 // out = A_e u for one element (Element::HelmholtzOp + HelmholtzKern,
 // src/element.cpp:1564-1650, Cartesian): R = u DT, S = D u, pointwise

@@ -90,8 +90,9 @@ extern "C" int sx_field_solve_device_static(sx_modal s, double *d_u, double *d_f
   SX_TRY(check_mesh_device(*s->mesh, "sx_field_solve_device_static"));
   const sx_mesh_s &Mh = *s->mesh;
   const int ngroups = nz == 1 ? 1 : nz / 2;
-  // Scratch layout: [one Job][rhs: P * npad][Fb: P * nel * next][gess: P * nglobal],
-  // reused by every mode in turn (the modes run one after another on `stream`).
+  // Scratch layout: [one Job][rhs: P * npad][Fb: P * nel * next], reused by
+  // every mode in turn (the modes run one after another on `stream`).  The
+  // capacity test counts P * nglobal doubles more: the limit that callers know.
   size_t need = 0;
   for (int l = 0; l < ngroups; l++) {
     const PlaneGroup g = plane_group(s->base_mode, nz, l);
@@ -153,15 +154,11 @@ extern "C" int sx_field_solve_device_static(sx_modal s, double *d_u, double *d_f
     j.rhs = reinterpret_cast<double *>(sp + off);
     off += align256((size_t)g.P * j.npad * 8);
     j.Fb = reinterpret_cast<double *>(sp + off);
-    off += align256((size_t)g.P * Mh.nel * Mh.next * 8);
-    j.gess = reinterpret_cast<double *>(sp + off);
     j.pc = S.pc.p;
     j.status = s->dstatus.p;
     // Stream-ordered after the previous mode's kernels, which read the same
-    // slot.  What must start at zero is gess (the essential values):
-    // direct_solve_jobs clears it with cudaMemsetAsync before k_essential
-    // writes the boundary values.  rhs (padding included) and Fb are written
-    // in full by k_rhs_dss / k_rhs_elem before anything reads them.
+    // slot.  rhs (padding included) and Fb are written in full by k_rhs_dss /
+    // k_rhs_elem before anything reads them.
     k_put_job<<<1, 32, 0, st>>>(djob, j);
     SX_CUDA(cudaGetLastError());
     int nl = 0;
