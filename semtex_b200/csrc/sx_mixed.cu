@@ -81,16 +81,17 @@ __device__ __forceinline__ size_t ye_index(const MeshView &M, int e, int a, int 
 // of RED_GROUP blocks (an integer counter per chunk and group) sums the
 // group's partials in block order into part[G + group]; the last group to
 // finish sums the group totals in group order.  Returns true in warp 0 of
-// that last block, with the chunk's totals in fa, fb.  part holds (G +
-// ceil(G / RED_GROUP)) * PP double2; cnt holds nch * (1 + ceil(G /
-// RED_GROUP)) counters, zero on entry and left zero.
+// that last block, with the chunk's totals in fa, fb (in every lane of a
+// plane).  part holds (G + ceil(G / RED_GROUP)) * 32 nch double2; cnt holds
+// nch * (1 + ceil(G / RED_GROUP)) counters, zero on entry and left zero.  sh:
+// 2 * ROWS * 32 doubles of shared memory that nothing else uses any more.
 constexpr int RED_GROUP = 32;
 inline int red_groups(int G) { return (G + RED_GROUP - 1) / RED_GROUP; }
 
 template <int ROWS>
 __device__ __forceinline__ bool chunk_sum(double a, double b, double *part, unsigned *cnt, int blk, int G, int y,
-                                          int nch, double &fa, double &fb) {
-  __shared__ double sa[ROWS][MX_CH], sb[ROWS][MX_CH];
+                                          int nch, int lp, double *sh, double &fa, double &fb) {
+  double(*sa)[MX_CH] = reinterpret_cast<double(*)[MX_CH]>(sh), (*sb)[MX_CH] = sa + ROWS;
   __shared__ int last;
   const int row = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int p = y * MX_CH + lane, PPc = nch * MX_CH;
@@ -157,19 +158,39 @@ __device__ __forceinline__ bool chunk_sum(double a, double b, double *part, unsi
     fa += sa[r][lane];
     fb += sb[r][lane];
   }
+  for (int o = 16; o >= lp; o >>= 1) {  // a plane's elements
+    fa += __shfl_xor_sync(0xffffffffu, fa, o);
+    fb += __shfl_xor_sync(0xffffffffu, fb, o);
+  }
   return true;
 }
 
 // chunk_sum for the 8-warp node kernels, storing the totals.
 __device__ __forceinline__ void chunk_reduce2(double a, double b, double *part, unsigned *cnt, int blk, int G,
-                                              int y, int nch, double *outA, double *outB) {
+                                              int y, int nch, int lp, double *outA, double *outB) {
+  __shared__ double sh[2 * MX_ROWS * MX_CH];
   double fa, fb;
-  if (chunk_sum<MX_ROWS>(a, b, part, cnt, blk, G, y, nch, fa, fb)) {
-    const int p = y * MX_CH + (threadIdx.x & 31);
+  const int lane = threadIdx.x & 31;
+  if (chunk_sum<MX_ROWS>(a, b, part, cnt, blk, G, y, nch, lp, sh, fa, fb) && lane < lp) {
+    const int p = y * lp + lane;
     if (outA) outA[p] = fa;
     if (outB) outB[p] = fb;
   }
 }
+
+// Where a lane works: lp = 32, 16 or 8 planes a chunk (MxMember::lp) and
+// 32 / lp elements (or nodes) side by side.  PK = false: lp = 32.
+template <bool PK>
+struct Lane {
+  int lp, sub, pl;
+  __device__ __forceinline__ explicit Lane(const MxMember &B) {
+    const int lane = threadIdx.x & 31;
+    lp = PK ? B.lp : MX_CH;
+    sub = PK ? lane >> B.lsh : 0;
+    pl = PK ? lane & (lp - 1) : lane;
+  }
+  __device__ __forceinline__ int ep() const { return PK ? MX_CH / lp : 1; }
+};
 
 // ---------------------------------------------------------------------------
 // tiles of a multi-mesh batch
@@ -262,9 +283,10 @@ static int ensure_constD() {
 // u in B0 ([NN][32], tensor order; overwritten on curved elements), B1 an
 // exchange buffer; entered with B0 filled and the block synchronised, left
 // with both buffers still being read (synchronise before reusing them).
+// curved (block-uniform): some element of the block has cross terms.
 template <int NP>
-__device__ __forceinline__ void line_apply64(const MeshView &M, int e, double hc, double *B0, double *B1,
-                                             double out[NP]) {
+__device__ __forceinline__ void line_apply64(const MeshView &M, int e, bool curved, double hc, double *B0,
+                                             double *B1, double out[NP]) {
   constexpr int NN = NP * NP, DO = DOff<NP>::v;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t eo = (size_t)e * NN;
@@ -288,7 +310,7 @@ __device__ __forceinline__ void line_apply64(const MeshView &M, int e, double hc
       S[j] = s;
     }
   }
-  if (M.hasQ3[e]) {
+  if (curved) {
     __syncthreads();  // every warp has its u lines: B0 is free
 #pragma unroll
     for (int j = 0; j < NP; j++) {
@@ -338,45 +360,52 @@ constexpr size_t x64_smem(int np) {
 // (element, 32 planes).  The forcing of the 32 planes is staged plane by
 // plane with coalesced loads into [32][NN | 1] (an odd row stride keeps the
 // lanes' column reads on distinct bank pairs), then read by lane.
-template <int NP>
-__device__ __forceinline__ void constrain_body(const MxMember &B, int e, int y) {
-  constexpr int NN = NP * NP, NE = 4 * (NP - 1), NI = NN - NE, TS = NN | 1;
+template <int NP, bool PK>
+__device__ __forceinline__ void constrain_body(const MxMember &B, int eg, int y) {
+  constexpr int NN = NP * NP, NE = 4 * (NP - 1), TS = NN | 1;
   const MeshView &M = B.M;
   const MxParams &P = B.P;
   double *__restrict__ Ye = B.Ye;
   extern __shared__ __align__(16) double smx[];
   double *B0 = smx, *B1 = B0 + NN * MX_CH, *T = B1 + NN * MX_CH;
-  __shared__ int gtab[NN], emt[NN], tsl[NN];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p0 = y * MX_CH, p = p0 + lane;
+  __shared__ int emt[NN], tsl[NN];
+  const Lane<PK> L(B);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, ep = L.ep(), e0 = eg * ep;
+  const int p = y * L.lp + L.pl, e = min(e0 + L.sub, M.nel - 1);
+  const bool rp = real_plane(P, p), in = e0 + L.sub < M.nel;
   const size_t eo = (size_t)e * NN;
+  bool masked = false, curved = false;  // any element of the block
+  for (int q = 0; q < ep && e0 + q < M.nel; q++) {
+    masked |= M.emask[e0 + q] != 0;
+    curved |= M.hasQ3[e0 + q] != 0;
+  }
   for (int a = threadIdx.x; a < NN; a += NP * 32) {
-    gtab[a] = a < NE ? M.btog[(size_t)e * NE + a] : M.nglobal + e * NI + (a - NE);
     emt[a] = M.emap[a];
     tsl[a] = M.pmap[a];
   }
   for (int i = threadIdx.x; i < MX_CH * NN; i += NP * 32) {
-    const int q = i / NN, k = i - q * NN, pl = p0 + q;
-    T[q * TS + k] = real_plane(P, pl) ? P.f[(size_t)pl * P.stride + eo + k] : 0.0;
+    const int q = i / NN, k = i - q * NN, pl = PK ? y * L.lp + (q & (L.lp - 1)) : y * MX_CH + q;
+    const int eq = PK ? e0 + (q >> B.lsh) : e0;
+    T[q * TS + k] = eq < M.nel && real_plane(P, pl) ? P.f[(size_t)pl * P.stride + (size_t)eq * NN + k] : 0.0;
   }
   __syncthreads();
   double F[NP];
 #pragma unroll
   for (int j = 0; j < NP; j++) F[j] = M.Q8[eo + w * NP + j] * T[lane * TS + w * NP + j];
-  if (M.emask[e]) {  // block-uniform: H g, g the essential values
-    const bool rp = real_plane(P, p);
+  if (masked) {  // block-uniform: H g, g the essential values (zero on elements without)
     const double *bc = P.bc && rp ? P.bc + (size_t)p * P.bcstride : nullptr;
 #pragma unroll
     for (int k = 0; k < NP; k++) {
       const int a = w + k * NP;
-      B0[emt[a] * MX_CH + lane] = (rp && a < NE) ? ess_value(M, bc, gtab[a]) : 0.0;
+      B0[emt[a] * MX_CH + lane] = (rp && a < NE) ? ess_value(M, bc, M.btog[(size_t)e * NE + a]) : 0.0;
     }
     __syncthreads();
     double hg[NP];
-    line_apply64<NP>(M, e, P.hcon[p], B0, B1, hg);
+    line_apply64<NP>(M, e, curved, P.hcon[p], B0, B1, hg);
 #pragma unroll
     for (int j = 0; j < NP; j++) F[j] += hg[j];
   }
+  if (!in) return;
 #pragma unroll
   for (int j = 0; j < NP; j++) {
     const int t = w * NP + j;
@@ -384,33 +413,35 @@ __device__ __forceinline__ void constrain_body(const MxMember &B, int e, int y) 
   }
 }
 
-template <int NP>
+template <int NP, bool PK>
 __global__ void __launch_bounds__(NP * 32, 2) k_x_constrain(const __grid_constant__ MxMember B) {
-  constrain_body<NP>(B, blockIdx.x, blockIdx.y);
+  constrain_body<NP, PK>(B, blockIdx.x, blockIdx.y);
 }
 
 template <int NP>
 __global__ void __launch_bounds__(NP * 32, 2) k_x_constrain_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) constrain_body<NP>(sB, t % sB.M.nel, t / sB.M.nel);
+  if (tile_member(T, sB, t)) constrain_body<NP, true>(sB, t % sB.neg, t / sB.neg);
 }
 
 // b = DSS(Ye) + <h,w>, essential tail zero; x = 0, r = b (FP32); per-plane
 // ||b||^2.
+template <bool PK>
 __device__ __forceinline__ void rhs_body(const MxMember &B, int blk, int y) {
   const MeshView &M = B.M;
   const MxParams &P = B.P;
   const double *__restrict__ Ye = B.Ye;
   double *b64 = B.b64, *x64 = B.V.x64;
   float *r32 = B.V.r0;
-  const int row = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = y * MX_CH + lane, PP = P.PP;
+  const Lane<PK> L(B);
+  const int row = (threadIdx.x >> 5) * L.ep() + L.sub, rows = MX_ROWS * L.ep();
+  const int p = y * L.lp + L.pl, PP = P.PP;
   const int npts = M.nglobal + M.nel * M.nint;
   const int ns = P.nsolve[p];
   const bool rp = real_plane(P, p);
   double bb = 0.0;
-  for (int g = blk * MX_ROWS + row; g < npts; g += B.G * MX_ROWS) {
+  for (int g = blk * rows + row; g < npts; g += B.G * rows) {
     double s = 0.0;
     if (g < M.nglobal) {
       if (g < ns) {
@@ -433,17 +464,18 @@ __device__ __forceinline__ void rhs_body(const MxMember &B, int blk, int y) {
     r32[o] = (float)s;
     bb += s * s;
   }
-  chunk_reduce2(bb, 0.0, B.part, B.cnt, blk, B.G, y, B.nch, B.b2, nullptr);
+  chunk_reduce2(bb, 0.0, B.part, B.cnt, blk, B.G, y, B.nch, L.lp, B.b2, nullptr);
 }
 
+template <bool PK>
 __global__ void __launch_bounds__(256) k_x_rhs(const __grid_constant__ MxMember B) {
-  rhs_body(B, blockIdx.x, blockIdx.y);
+  rhs_body<PK>(B, blockIdx.x, blockIdx.y);
 }
 
 __global__ void __launch_bounds__(256) k_x_rhs_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) rhs_body(sB, t % sB.G, t / sB.G);
+  if (tile_member(T, sB, t)) rhs_body<true>(sB, t % sB.G, t / sB.G);
 }
 
 // ---------------------------------------------------------------------------
@@ -466,10 +498,11 @@ enum { CG_INIT = 0, CG_ITER = 1, CG_LAST = 2, CG_MODE = 3 };
 // well before the round ends; otherwise the read is only latency)
 constexpr int CG_CHECK_STOP = 4;
 
-// Element-layout address of (element e, plane chunk y, tensor node t, lane l).
+// Element-layout address of (element group eg, plane chunk y, tensor node t,
+// lane l).
 template <int NN>
-__device__ __forceinline__ size_t eidx(int e, int nch, int y, int t, int l) {
-  return (((size_t)e * nch + y) * NN + t) * MX_CH + l;
+__device__ __forceinline__ size_t eidx(int eg, int nch, int y, int t, int l) {
+  return (((size_t)eg * nch + y) * NN + t) * MX_CH + l;
 }
 
 // Direct-stiffness sum of the element-layout W at global node g, in element
@@ -477,26 +510,32 @@ __device__ __forceinline__ size_t eidx(int e, int nch, int y, int t, int l) {
 // tensor node; .w == -2: walk the CSR, whose entries are element * next +
 // slot, slot -> tensor node through emt).  Every holder of g forms the same
 // sum in the same order.
-template <int NN>
-__device__ __forceinline__ float gather_we(const MeshView &M, const float *__restrict__ W, int4 q, int g, int nch,
-                                           int y, int l, const int *emt) {
+template <int NN, bool PK>
+__device__ __forceinline__ float gather_we(const MxMember &B, const float *__restrict__ W, int4 q, int g, int y,
+                                           const Lane<PK> &L, const int *emt) {
+  const MeshView &M = B.M;
+  auto at = [&](int e, int t) {
+    return PK ? W[eidx<NN>(e >> (5 - B.lsh), B.nch, y, t, ((e & (MX_CH / L.lp - 1)) << B.lsh) + L.pl)]
+              : W[eidx<NN>(e, B.nch, y, t, L.pl)];
+  };
   if (q.w == -2) {
     float s = 0.0f;
     for (int k = M.g2e_ptr[g]; k < M.g2e_ptr[g + 1]; k++) {
       const int ei = M.g2e_idx[k], eh = ei / M.next;
-      s += W[eidx<NN>(eh, nch, y, emt[ei - eh * M.next], l)];
+      s += at(eh, emt[ei - eh * M.next]);
     }
     return s;
   }
-  const float v0 = W[eidx<NN>(q.x >> 8, nch, y, q.x & 255, l)];
-  const float v1 = q.y >= 0 ? W[eidx<NN>(q.y >> 8, nch, y, q.y & 255, l)] : 0.0f;
-  const float v2 = q.z >= 0 ? W[eidx<NN>(q.z >> 8, nch, y, q.z & 255, l)] : 0.0f;
-  const float v3 = q.w >= 0 ? W[eidx<NN>(q.w >> 8, nch, y, q.w & 255, l)] : 0.0f;
+  const float v0 = at(q.x >> 8, q.x & 255);
+  const float v1 = q.y >= 0 ? at(q.y >> 8, q.y & 255) : 0.0f;
+  const float v2 = q.z >= 0 ? at(q.z >> 8, q.z & 255) : 0.0f;
+  const float v3 = q.w >= 0 ? at(q.w >> 8, q.w & 255) : 0.0f;
   return ((v0 + v1) + v2) + v3;
 }
 
-// One launch = one iteration for every plane: block (element e, chunk y of
-// 32 planes), NP warps.  Thread 0 stages the element's spans of r, s, p, d,
+// One launch = one iteration for every plane: block (element group eg, chunk y
+// of lp planes: 32 / lp elements share a block's lanes, so that few planes
+// still fill them), NP warps.  Thread 0 stages the element's spans of r, s, p, d,
 // its own A u and the preconditioner into shared memory with TMA bulk copies
 // on one mbarrier while the block loads its tables.  Phase A walks the
 // element's nodes in edge-map order (warp w takes slots w, w + NP, ...: the
@@ -528,11 +567,13 @@ int set_cg_wait_limit(long long cycles) {
 }
 
 // Dynamic shared memory of k_cg: six [NN][32] spans, the [NN][16]
-// preconditioner pairs and the element's geometry (one float4 a node).
-constexpr size_t cg_smem(int np) { return (size_t)np * np * ((6 * MX_CH + 16) * sizeof(float) + 16); }
+// preconditioner pairs and the geometry of the block's ep elements (one
+// float4 a node).
+constexpr size_t cg_smem(int np, int ep) { return (size_t)np * np * ((6 * MX_CH + 16) * sizeof(float) + 16 * ep); }
+constexpr int MX_EP = 4;  // elements a block holds at most (lp = 8)
 
-template <int NP>
-__device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it, int mode) {
+template <int NP, bool PK>
+__device__ __forceinline__ void cg_body(const MxMember &B, int eg, int y, int it, int mode) {
   constexpr int NN = NP * NP, NE = 4 * (NP - 1), NI = NN - NE, DO = DOff<NP>::v;
   const MeshView &M = B.M;
   const MxParams &P = B.P;
@@ -549,12 +590,20 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
   float *B1 = Ds + NN * MX_CH, *B0 = B1 + NN * MX_CH, *PCs = B0 + NN * MX_CH;
   float4 *Gs = reinterpret_cast<float4 *>(PCs + NN * 16);
   constexpr uint32_t GSPAN = NN * sizeof(float4);
-  __shared__ int gtab[NN], emt[NN];
-  __shared__ int4 w4[NE];
+  constexpr int EPM = PK ? MX_EP : 1;
+  // global node of each slot: boundary slots only where a block holds several
+  // elements, the interior ones following from the element
+  __shared__ int gtab[PK ? EPM * NE : NN], emt[NN];
+  __shared__ int4 w4[EPM * NE];
   __shared__ __align__(8) uint64_t bar;
   __shared__ int staged;
-  const int nch = B.nch, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = y * MX_CH + lane, PP = P.PP;
+  const Lane<PK> L(B);
+  const int nch = B.nch, w = threadIdx.x >> 5, lane = threadIdx.x & 31, ep = L.ep(), e0 = eg * ep;
+  const int p = y * L.lp + L.pl, PP = P.PP;
+  // the last group may hold fewer than ep elements: its idle lanes work on
+  // the last element's numbers and contribute nothing
+  const int e = PK ? min(e0 + L.sub, M.nel - 1) : e0, nin = PK ? min(ep, M.nel - e0) : 1;
+  const bool in = !PK || L.sub < nin;
   const bool check = (mode & CG_CHECK_STOP) != 0;
   mode &= CG_MODE;
   const bool init = mode == CG_INIT, last = mode == CG_LAST;
@@ -565,18 +614,18 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
   if (stopped && !last) return;
   const int cur = init ? 0 : (it & 1), nxt = init ? 0 : (cur ^ 1);
   const bool warm = !init && it > 0;  // s, p, d hold previous iterates
-  const size_t base = eidx<NN>(e, nch, y, 0, 0), pbase = ((size_t)e * nch + y) * NN * 16;
+  const size_t base = eidx<NN>(eg, nch, y, 0, 0), pbase = ((size_t)eg * nch + y) * NN * 16;
   // buffers of this launch, selected without indexing the parameter arrays
   const float *__restrict__ Win = cur ? V.WE[1] : V.WE[0];
   float *__restrict__ Wout = nxt ? V.WE[1] : V.WE[0];
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     fence_mbar_init_cluster();
-    const uint32_t bytes = PSPAN + (last ? 0u : GSPAN) + (init ? 0u : SPAN) + (!init && !last ? SPAN : 0u) +
+    const uint32_t bytes = PSPAN + (last ? 0u : nin * GSPAN) + (init ? 0u : SPAN) + (!init && !last ? SPAN : 0u) +
                            (warm ? (last ? 2u : 3u) * SPAN : 0u);
     mbar_arrive_expect_tx(&bar, bytes);
     bulk_g2s(PCs, V.pcE + pbase, PSPAN, &bar);
-    if (!last) bulk_g2s(Gs, M.Gf + (size_t)e * NN, GSPAN, &bar);
+    if (!last) bulk_g2s(Gs, M.Gf + (size_t)e0 * NN, nin * GSPAN, &bar);
     if (!init) bulk_g2s(Rs, V.rE + base, SPAN, &bar);
     if (!init && !last) bulk_g2s(B1, Win + base, SPAN, &bar);
     if (warm) {
@@ -586,10 +635,15 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
     }
   }
   for (int a = threadIdx.x; a < NN; a += NP * 32) {
-    gtab[a] = a < NE ? M.btog[(size_t)e * NE + a] : M.nglobal + e * NI + (a - NE);
     emt[a] = M.emap[a];
-    if (a < NE) w4[a] = M.e2w4[(size_t)e * NE + a];
+    if (!PK) gtab[a] = a < NE ? M.btog[(size_t)e * NE + a] : M.nglobal + e * NI + (a - NE);
+    if (!PK && a < NE) w4[a] = M.e2w4[(size_t)e * NE + a];
   }
+  if (PK)
+    for (int a = threadIdx.x; a < nin * NE; a += NP * 32) {
+      gtab[a] = M.btog[(size_t)e0 * NE + a];
+      w4[a] = M.e2w4[(size_t)e0 * NE + a];
+    }
   const double *gam_in = cur ? V.gam[1] : V.gam[0], *alpha_in = cur ? V.alpha[1] : V.alpha[0];
   const double *beta_in = cur ? V.beta[1] : V.beta[0];
   double *gam_out = nxt ? V.gam[1] : V.gam[0], *alpha_out = nxt ? V.alpha[1] : V.alpha[0];
@@ -601,6 +655,8 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
     beta = (float)beta_in[p];
   }
   const unsigned long long own = M.owner[e];
+  const int eb = PK ? (e - e0) * NE : 0, gi = M.nglobal + e * NI - NE;
+  auto gnode = [&](int a) { return !PK ? gtab[a] : a < NE ? gtab[eb + a] : gi + a; };
   __syncthreads();  // the tables
   // Global loads of phase A -- A u of the previous launch at the element's
   // boundary nodes through their holders (or r at INIT) -- issued now, so
@@ -608,13 +664,13 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
   float gv[NP];
 #pragma unroll
   for (int k = 0; k < NP; k++) {
-    const int a = w + k * NP, g = gtab[a];
+    const int a = w + k * NP, g = gnode(a);
     gv[k] = 0.0f;
     if (!(a >= NE || g < ns)) continue;
     if (init)
       gv[k] = V.r0[(size_t)g * PP + p];
     else if (!last && a < NE)
-      gv[k] = gather_we<NN>(M, Win, w4[a], g, nch, y, lane, emt);
+      gv[k] = gather_we<NN, PK>(B, Win, w4[eb + a], g, y, L, emt);
   }
   // the staged spans: thread 0 waits (bounded) and tells the block; the
   // others then pass the completed phase, which orders the TMA writes for them
@@ -635,9 +691,9 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
   double gam = 0.0;
 #pragma unroll
   for (int k = 0; k < NP; k++) {
-    const int a = w + k * NP, g = gtab[a], t = emt[a], o = t * MX_CH + lane;
+    const int a = w + k * NP, g = gnode(a), t = emt[a], o = t * MX_CH + lane;
     const bool solve = a >= NE || g < ns;
-    const bool mine = a >= NE || ((own >> a) & 1ull);
+    const bool mine = in && (a >= NE || ((own >> a) & 1ull));
     const float pc = PCs[t * 16 + (lane >> 1)];
     float un = 0.0f;
     if (init) {
@@ -700,8 +756,11 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
       S[j] = s;
     }
   }
-  const float4 *G = Gs;
-  if (M.hasQ3[e]) {
+  const float4 *G = Gs + (PK ? (e - e0) * NN : 0);
+  bool curved = M.hasQ3[e0] != 0;  // some element of the block
+  if (PK)
+    for (int q = 1; q < nin; q++) curved |= M.hasQ3[e0 + q] != 0;
+  if (curved) {
     // curved: R = Q1 r + Q3 s, S = Q2 s + Q3 r need both at every node
     __syncthreads();  // every warp has its u lines: B0 is free
 #pragma unroll
@@ -745,7 +804,7 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
     const int t = w * NP + j;
     const float out = G[t].w * hc * ur[j] + B1[t * MX_CH + lane] + b;
     B0[t * MX_CH + lane] = out;  // every warp is past its reads of u in B0
-    del += (double)ur[j] * (double)out;
+    if (in) del += (double)ur[j] * (double)out;
   }
   fence_proxy_async_smem();
   __syncthreads();
@@ -757,7 +816,12 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
   // ---- gamma = (r, u), delta = (A u, u); the chunk's last block forms the
   // next iteration's scalars
   double gn, dn;
-  if (chunk_sum<NP>(gam, del, B.part, B.cnt, e, M.nel, y, nch, gn, dn)) {
+  // B1 is free (every warp has passed the barrier after its last reads), and
+  // holds the reduction from np = 4 on
+  constexpr bool IN_B1 = 2 * NP * MX_CH * sizeof(double) <= SPAN;
+  __shared__ double rsh[IN_B1 ? 1 : 2 * NP * MX_CH];
+  if (chunk_sum<NP>(gam, del, B.part, B.cnt, eg, B.neg, y, nch, L.lp, IN_B1 ? reinterpret_cast<double *>(B1) : rsh,
+                    gn, dn)) {
     double an, bn;
     if (init) {
       bn = 0.0;
@@ -784,17 +848,17 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int e, int y, int it,
   if (threadIdx.x == 0) bulk_wait_read_all();  // the stores have read shared memory
 }
 
-template <int NP>
+template <int NP, bool PK>
 __global__ void __launch_bounds__(NP * 32, cg_min_blocks(NP))
     k_cg(const __grid_constant__ MxMember B, int it, int mode) {
-  cg_body<NP>(B, blockIdx.x, blockIdx.y, it, mode);
+  cg_body<NP, PK>(B, blockIdx.x, blockIdx.y, it, mode);
 }
 
 template <int NP>
 __global__ void __launch_bounds__(NP * 32, cg_min_blocks(NP)) k_cg_multi(MxTable T, int it, int mode) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) cg_body<NP>(sB, t % sB.M.nel, t / sB.M.nel, it, mode);
+  if (tile_member(T, sB, t)) cg_body<NP, true>(sB, t % sB.neg, t / sB.neg, it, mode);
 }
 
 // ---------------------------------------------------------------------------
@@ -804,8 +868,8 @@ __global__ void __launch_bounds__(NP * 32, cg_min_blocks(NP)) k_cg_multi(MxTable
 // Ye = A_e x at the element's slots (FP64), NP warps per (element, 32
 // planes): x gathered through btog in slot order, the operator on tensor
 // lines (line_apply64).
-template <int NP>
-__device__ __forceinline__ void op64_body(const MxMember &B, int e, int y) {
+template <int NP, bool PK>
+__device__ __forceinline__ void op64_body(const MxMember &B, int eg, int y) {
   constexpr int NN = NP * NP, NE = 4 * (NP - 1), NI = NN - NE;
   const MeshView &M = B.M;
   const MxParams &P = B.P;
@@ -813,54 +877,66 @@ __device__ __forceinline__ void op64_body(const MxMember &B, int e, int y) {
   double *__restrict__ Ye = B.Ye;
   extern __shared__ __align__(16) double smx[];
   double *B0 = smx, *B1 = B0 + NN * MX_CH;
-  __shared__ int gtab[NN], emt[NN], tsl[NN];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = y * MX_CH + lane, PP = P.PP;
+  __shared__ int gtab[(PK ? MX_EP : 1) * NE], emt[NN], tsl[NN];
+  const Lane<PK> L(B);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, ep = L.ep(), e0 = eg * ep;
+  const int p = y * L.lp + L.pl, PP = P.PP;
+  const int e = PK ? min(e0 + L.sub, M.nel - 1) : e0, nin = PK ? min(ep, M.nel - e0) : 1;
   for (int a = threadIdx.x; a < NN; a += NP * 32) {
-    gtab[a] = a < NE ? M.btog[(size_t)e * NE + a] : M.nglobal + e * NI + (a - NE);
     emt[a] = M.emap[a];
     tsl[a] = M.pmap[a];
   }
+  for (int a = threadIdx.x; a < nin * NE; a += NP * 32) gtab[a] = M.btog[(size_t)e0 * NE + a];
+  bool curved = M.hasQ3[e0] != 0;  // some element of the block
+  if (PK)
+    for (int q = 1; q < nin; q++) curved |= M.hasQ3[e0 + q] != 0;
+  const int eb = PK ? (e - e0) * NE : 0, gi = M.nglobal + e * NI - NE;
   __syncthreads();
   double xv[NP];
 #pragma unroll
-  for (int k = 0; k < NP; k++) xv[k] = x64[(size_t)gtab[w + k * NP] * PP + p];
+  for (int k = 0; k < NP; k++) {
+    const int a = w + k * NP;
+    xv[k] = x64[(size_t)(a < NE ? gtab[eb + a] : gi + a) * PP + p];
+  }
 #pragma unroll
   for (int k = 0; k < NP; k++) B0[emt[w + k * NP] * MX_CH + lane] = xv[k];
   __syncthreads();
   double out[NP];
-  line_apply64<NP>(M, e, P.hcon[p], B0, B1, out);
+  line_apply64<NP>(M, e, curved, P.hcon[p], B0, B1, out);
+  if (PK && L.sub >= nin) return;
 #pragma unroll
   for (int j = 0; j < NP; j++) Ye[ye_index(M, e, tsl[w * NP + j], PP) + p] = out[j];
 }
 
-template <int NP>
+template <int NP, bool PK>
 __global__ void __launch_bounds__(NP * 32, 2) k_x_op64(const __grid_constant__ MxMember B) {
-  op64_body<NP>(B, blockIdx.x, blockIdx.y);
+  op64_body<NP, PK>(B, blockIdx.x, blockIdx.y);
 }
 
 template <int NP>
 __global__ void __launch_bounds__(NP * 32, 2) k_x_op64_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) op64_body<NP>(sB, t % sB.M.nel, t / sB.M.nel);
+  if (tile_member(T, sB, t)) op64_body<NP, true>(sB, t % sB.neg, t / sB.neg);
 }
 
 // r = b - A x (FP64), essential tail zero; the next round's inner solve
 // starts from r32 = r (and d = 0, which its first iteration assumes);
 // per-plane ||r||^2.
+template <bool PK>
 __device__ __forceinline__ void res_body(const MxMember &B, int blk, int y) {
   const MeshView &M = B.M;
   const MxParams &P = B.P;
   const double *__restrict__ Ye = B.Ye;
   const double *__restrict__ b64 = B.b64;
   float *r32 = B.V.r0;
-  const int row = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = y * MX_CH + lane, PP = P.PP;
+  const Lane<PK> L(B);
+  const int row = (threadIdx.x >> 5) * L.ep() + L.sub, rows = MX_ROWS * L.ep();
+  const int p = y * L.lp + L.pl, PP = P.PP;
   const int npts = M.nglobal + M.nel * M.nint;
   const int ns = P.nsolve[p];
   double rr = 0.0;
-  for (int g = blk * MX_ROWS + row; g < npts; g += B.G * MX_ROWS) {
+  for (int g = blk * rows + row; g < npts; g += B.G * rows) {
     double ax = 0.0;
     bool solve = true;
     if (g < M.nglobal) {
@@ -874,24 +950,25 @@ __device__ __forceinline__ void res_body(const MxMember &B, int blk, int y) {
     r32[o] = (float)r;
     rr += r * r;
   }
-  chunk_reduce2(rr, 0.0, B.part, B.cnt, blk, B.G, y, B.nch, B.r2, nullptr);
+  chunk_reduce2(rr, 0.0, B.part, B.cnt, blk, B.G, y, B.nch, L.lp, B.r2, nullptr);
 }
 
+template <bool PK>
 __global__ void __launch_bounds__(256) k_x_res(const __grid_constant__ MxMember B) {
-  res_body(B, blockIdx.x, blockIdx.y);
+  res_body<PK>(B, blockIdx.x, blockIdx.y);
 }
 
 __global__ void __launch_bounds__(256) k_x_res_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) res_body(sB, t % sB.G, t / sB.G);
+  if (tile_member(T, sB, t)) res_body<true>(sB, t % sB.G, t / sB.G);
 }
 
 // u = x at element nodes, essential values from the boundary lines (global2local +
 // setEssential, src/field.cpp:710-713, 1022-1040); transposed back to the
 // caller's plane-major layout through shared memory.
-template <int NP>
-__device__ __forceinline__ void unpack_body(const MxMember &B, int e, int y) {
+template <int NP, bool PK>
+__device__ __forceinline__ void unpack_body(const MxMember &B, int eg, int y) {
   constexpr int NN = NP * NP, NE = 4 * (NP - 1);
   const MeshView &M = B.M;
   const MxParams &P = B.P;
@@ -902,7 +979,8 @@ __device__ __forceinline__ void unpack_body(const MxMember &B, int e, int y) {
   __shared__ double V[NN * VS];
   __shared__ int emap[NN];
   const int tid = threadIdx.x, row = tid >> 5, lane = tid & 31;
-  const int p0 = y * MX_CH, p = p0 + lane, PP = P.PP;
+  const Lane<PK> L(B);
+  const int p = y * L.lp + L.pl, PP = P.PP, e0 = eg * L.ep(), e = min(e0 + L.sub, M.nel - 1);
   for (int i = tid; i < NN; i += 256) emap[i] = M.emap[i];
   __syncthreads();
   const bool masked = M.emask[e] != 0;
@@ -921,21 +999,22 @@ __device__ __forceinline__ void unpack_body(const MxMember &B, int e, int y) {
   // plane q's NN values are contiguous in the caller's array: all threads
   // over (plane, node) pairs
   for (int i = tid; i < MX_CH * NN; i += 256) {
-    const int q = i / NN, k = i - q * NN, pl = p0 + q;
-    if (real_plane(P, pl)) P.u[(size_t)pl * P.stride + (size_t)e * NN + k] = V[k * VS + q];
+    const int q = i / NN, k = i - q * NN, pl = PK ? y * L.lp + (q & (L.lp - 1)) : y * MX_CH + q;
+    const int eq = PK ? e0 + (q >> B.lsh) : e0;
+    if (eq < M.nel && real_plane(P, pl)) P.u[(size_t)pl * P.stride + (size_t)eq * NN + k] = V[k * VS + q];
   }
 }
 
-template <int NP>
+template <int NP, bool PK>
 __global__ void __launch_bounds__(256) k_x_unpack(const __grid_constant__ MxMember B) {
-  unpack_body<NP>(B, blockIdx.x, blockIdx.y);
+  unpack_body<NP, PK>(B, blockIdx.x, blockIdx.y);
 }
 
 template <int NP>
 __global__ void __launch_bounds__(256) k_x_unpack_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) unpack_body<NP>(sB, t % sB.M.nel, t / sB.M.nel);
+  if (tile_member(T, sB, t)) unpack_body<NP, true>(sB, t % sB.neg, t / sB.neg);
 }
 
 // ---------------------------------------------------------------------------
@@ -957,20 +1036,46 @@ __global__ void __launch_bounds__(256) k_x_unpack_multi(MxTable T) {
     default: break;                                            \
   }
 
-static int grid_nodes(int npts) {
-  // node-loop kernels: a fixed grid, up to 6 blocks of 8 node rows per SM,
-  // each thread taking 4 nodes per pass
-  return std::max(1, std::min((npts + 4 * MX_ROWS - 1) / (4 * MX_ROWS), 6 * 148));
+// Runs the statements with PK_ = whether workspace W's chunks hold fewer than 32 planes.
+#define SX_PK_SWITCH(W, ...)           \
+  do {                                 \
+    if ((W).lp < MX_CH) {              \
+      constexpr bool PK_ = true;       \
+      __VA_ARGS__;                     \
+    } else {                           \
+      constexpr bool PK_ = false;      \
+      __VA_ARGS__;                     \
+    }                                  \
+  } while (0)
+
+static int grid_nodes(int npts, int ep) {
+  // node-loop kernels: a fixed grid, up to 6 blocks of 8 node rows (of ep
+  // nodes) per SM, each thread taking 4 nodes per pass
+  return std::max(1, std::min((npts + 4 * MX_ROWS * ep - 1) / (4 * MX_ROWS * ep), 6 * 148));
 }
 
-template <int NP>
+// Planes a chunk: 32, 16 or 8, whichever pads nz planes least (the widest on a
+// tie).  The iterations stream whole chunks, so an idle lane costs what a
+// working one does; a narrower chunk reads the element geometry once more for
+// the same planes (16 bytes a node for 8 planes, against 40 bytes a node and
+// plane of vectors).  Measured: 16 planes of 8192 elements of order 10, one
+// solve 15.8 ms in 32-plane chunks, 8.9 ms in 16-plane ones.
+static int chunk_planes(int nz) {
+  int best = MX_CH;
+  for (int lp = MX_CH / 2; lp >= 8; lp /= 2)
+    if ((nz + lp - 1) / lp * lp < (nz + best - 1) / best * best) best = lp;
+  return best;
+}
+
+template <int NP, bool PK>
 static int set_smem_attrs() {
-  SX_CUDA(cudaFuncSetAttribute(k_x_constrain<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  SX_CUDA(cudaFuncSetAttribute((k_x_constrain<NP, PK>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)x64_smem(NP)));
-  SX_CUDA(cudaFuncSetAttribute(k_x_op64<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x64_smem(NP)));
-  SX_CUDA(cudaFuncSetAttribute(k_cg<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(NP)));
+  SX_CUDA(cudaFuncSetAttribute((k_x_op64<NP, PK>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x64_smem(NP)));
+  SX_CUDA(cudaFuncSetAttribute((k_cg<NP, PK>), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)cg_smem(NP, PK ? MX_EP : 1)));
   // the largest carveout, so that cg_min_blocks(NP) blocks fit an SM
-  SX_CUDA(cudaFuncSetAttribute(k_cg<NP>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  SX_CUDA(cudaFuncSetAttribute((k_cg<NP, PK>), cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   return SX_OK;
 }
 
@@ -1026,15 +1131,20 @@ static MxMember member_of(const MeshView &M, MixedWork &W) {
   B.b2 = s.b2;
   B.part = W.part.p;
   B.cnt = W.cnt.p;
-  B.nch = W.PP / MX_CH;
+  B.nch = W.PP / W.lp;
+  B.lp = W.lp;
+  B.lsh = W.lp == 32 ? 5 : W.lp == 16 ? 4 : 3;
+  B.neg = (M.nel + MX_CH / W.lp - 1) / (MX_CH / W.lp);
   B.G = W.G;
   return B;
 }
 
 static int enqueue_init(const MeshView &M, MixedWork &W, cudaStream_t st, int *nl) {
   const MxMember B = member_of(M, W);
-  SX_NP_SWITCH_M(M.np, (k_x_constrain<N_><<<dim3(M.nel, B.nch), N_ * 32, x64_smem(N_), st>>>(B)));
-  k_x_rhs<<<dim3(W.G, B.nch), 256, 0, st>>>(B);
+  SX_PK_SWITCH(W, {
+    SX_NP_SWITCH_M(M.np, (k_x_constrain<N_, PK_><<<dim3(B.neg, B.nch), N_ * 32, x64_smem(N_), st>>>(B)));
+    k_x_rhs<PK_><<<dim3(W.G, B.nch), 256, 0, st>>>(B);
+  });
   *nl = 2;
   SX_CUDA(cudaGetLastError());
   return SX_OK;
@@ -1045,15 +1155,18 @@ static int enqueue_init(const MeshView &M, MixedWork &W, cudaStream_t st, int *n
 static int enqueue_round(const MeshView &M, MixedWork &W, int n_inner, bool check_stop, cudaStream_t st,
                          int *nl) {
   const MxMember B = member_of(M, W);
-  const dim3 eg(M.nel, B.nch);
+  const dim3 eg(B.neg, B.nch);
+  const int ep = MX_CH / B.lp;
   *nl = 0;
-  SX_NP_SWITCH_M(M.np, (k_cg<N_><<<eg, N_ * 32, cg_smem(N_), st>>>(B, 0, CG_INIT)));
-  for (int it = 0; it < n_inner; it++) {
-    const int mode = (it == n_inner - 1 ? CG_LAST : CG_ITER) | (check_stop ? CG_CHECK_STOP : 0);
-    SX_NP_SWITCH_M(M.np, (k_cg<N_><<<eg, N_ * 32, cg_smem(N_), st>>>(B, it, mode)));
-  }
-  SX_NP_SWITCH_M(M.np, (k_x_op64<N_><<<eg, N_ * 32, x64_smem(N_), st>>>(B)));
-  k_x_res<<<dim3(W.G, B.nch), 256, 0, st>>>(B);
+  SX_PK_SWITCH(W, {
+    SX_NP_SWITCH_M(M.np, (k_cg<N_, PK_><<<eg, N_ * 32, cg_smem(N_, ep), st>>>(B, 0, CG_INIT)));
+    for (int it = 0; it < n_inner; it++) {
+      const int mode = (it == n_inner - 1 ? CG_LAST : CG_ITER) | (check_stop ? CG_CHECK_STOP : 0);
+      SX_NP_SWITCH_M(M.np, (k_cg<N_, PK_><<<eg, N_ * 32, cg_smem(N_, ep), st>>>(B, it, mode)));
+    }
+    SX_NP_SWITCH_M(M.np, (k_x_op64<N_, PK_><<<eg, N_ * 32, x64_smem(N_), st>>>(B)));
+    k_x_res<PK_><<<dim3(W.G, B.nch), 256, 0, st>>>(B);
+  });
   *nl = n_inner + 3;
   SX_CUDA(cudaGetLastError());
   return SX_OK;
@@ -1066,7 +1179,8 @@ int mixed_profile_iterations(const MeshView &M, MixedWork &W, int reps, cudaStre
   // every chunk works in the timed launches
   SX_CUDA(cudaMemsetAsync(W.skip.p, 0, sizeof(int) * B.nch, st));
   for (int r = 0; r < reps; r++)
-    SX_NP_SWITCH_M(M.np, (k_cg<N_><<<dim3(M.nel, B.nch), N_ * 32, cg_smem(N_), st>>>(B, 1, CG_ITER)));
+    SX_PK_SWITCH(W, SX_NP_SWITCH_M(M.np, (k_cg<N_, PK_><<<dim3(B.neg, B.nch), N_ * 32,
+                                                          cg_smem(N_, MX_CH / B.lp), st>>>(B, 1, CG_ITER))));
   SX_CUDA(cudaGetLastError());
   return SX_OK;
 }
@@ -1094,38 +1208,39 @@ __global__ void k_x_pc(int npts, int M, const float *const *pcs, float *out) {
   for (int m = 0; m < M; m++) out[(size_t)g * M + m] = pcs[m][g];
 }
 
-// Element-layout preconditioner pairs, pcE[((e * nch + y) * np^2 + t) * 16 +
-// q] = the inverse Jacobi diagonal of mode column 16 y + q (clamped to the
-// last mode) at the global node of (e, t); lanes 2q and 2q + 1 -- the mode's
-// two planes -- read it.
-__global__ void k_x_pce(MeshView M, int nch, int Mc, const float *__restrict__ pcf, float *pcE) {
-  const int NN = M.npnp;
-  const size_t n = (size_t)M.nel * nch * NN * 16;
+// Element-layout preconditioner pairs, pcE[((eg * nch + y) * np^2 + t) * 16 +
+// q] = the inverse Jacobi diagonal that lanes 2q and 2q + 1 read, the two
+// planes of one mode (clamped to the last mode) at the global node of tensor
+// node t of their element (clamped to the last element).
+__global__ void k_x_pce(MeshView M, int nch, int neg, int lp, int Mc, const float *__restrict__ pcf, float *pcE) {
+  const int NN = M.npnp, ep = MX_CH / lp;
+  const size_t n = (size_t)neg * nch * NN * 16;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const int q = (int)(i & 15);
     const size_t r = i >> 4;
     const int t = (int)(r % NN);
     const size_t ey = r / NN;
-    const int y = (int)(ey % nch), e = (int)(ey / nch);
+    const int y = (int)(ey % nch), e = min((int)(ey / nch) * ep + 2 * q / lp, M.nel - 1);
     const int g = gidx(M, e, M.pmap[t]);
-    pcE[i] = pcf[(size_t)g * Mc + min(16 * y + q, Mc - 1)];
+    pcE[i] = pcf[(size_t)g * Mc + min((y * lp + 2 * q % lp) / 2, Mc - 1)];
   }
 }
 
 static int setup(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &groups, int nz, int num_modes,
                  cudaStream_t st) {
   const int npts = M.nglobal + M.nel * M.nint;
-  const int PP = ((nz + MX_CH - 1) / MX_CH) * MX_CH;
+  const int lp = chunk_planes(nz), nch = (nz + lp - 1) / lp, PP = nch * lp;
+  const int ep = MX_CH / lp, neg = (M.nel + ep - 1) / ep;
   const int Mc = std::max(1, num_modes);
   {
     // grow-only: a workspace is reused across solves of different sizes
     auto need = [&](auto &b, size_t n) { return b.n < n ? b.alloc_in(n, W.pool, st) : SX_OK; };
     const size_t n = (size_t)PP * npts;
-    W.G = grid_nodes(npts);
+    W.G = grid_nodes(npts, ep);
     SX_TRY(need(W.b64, n));
     SX_TRY(need(W.x64, n));
     SX_TRY(need(W.Ye64, (size_t)PP * M.nel * M.npnp));
-    const size_t ne = (size_t)PP * M.nel * M.npnp;  // one E-vector
+    const size_t ne = (size_t)neg * nch * M.npnp * MX_CH;  // one E-vector
     SX_TRY(need(W.r0, n));
     SX_TRY(need(W.rE, ne));
     SX_TRY(need(W.sE, ne));
@@ -1138,18 +1253,19 @@ static int setup(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &gr
     SX_TRY(need(W.hcon, (size_t)PP));
     SX_TRY(need(W.nsolve, (size_t)PP));
     SX_TRY(need(W.active, (size_t)PP));
-    SX_TRY(need(W.skip, (size_t)PP / MX_CH));
+    SX_TRY(need(W.skip, (size_t)nch));
     SX_TRY(need(W.pcf, (size_t)npts * Mc));
     // reduction tree: block and group partials, chunk and group counters
-    const int gmax = std::max(W.G, M.nel);
-    SX_TRY(need(W.part, (size_t)PP * (gmax + red_groups(gmax)) * 2));
-    const size_t ncnt = (size_t)(PP / MX_CH) * (1 + red_groups(gmax));
+    const int gmax = std::max(W.G, neg);
+    SX_TRY(need(W.part, (size_t)nch * MX_CH * (gmax + red_groups(gmax)) * 2));
+    const size_t ncnt = (size_t)nch * (1 + red_groups(gmax));
     if (W.cnt.n < ncnt) {
       SX_TRY(W.cnt.alloc_in(ncnt, W.pool, st));
       SX_TRY(W.cnt.zero(st));
     }
     W.hscal.assign((size_t)2 * PP, 0.0);
     W.PP = PP;
+    W.lp = lp;
     W.npts = npts;
     W.M = Mc;
   }
@@ -1169,12 +1285,12 @@ static int setup(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &gr
   SX_CUDA(cudaMemcpyAsync(W.hcon.p, hc.data(), sizeof(double) * PP, cudaMemcpyHostToDevice, st));
   SX_CUDA(cudaMemcpyAsync(W.nsolve.p, ns.data(), sizeof(int) * PP, cudaMemcpyHostToDevice, st));
   SX_CUDA(cudaMemcpyAsync(W.active.p, act.data(), sizeof(int) * PP, cudaMemcpyHostToDevice, st));
-  SX_CUDA(cudaMemsetAsync(W.skip.p, 0, sizeof(int) * (PP / MX_CH), st));
+  SX_CUDA(cudaMemsetAsync(W.skip.p, 0, sizeof(int) * nch, st));
   DBuf<const float *> dp;
   SX_TRY(dp.upload_on(pcs.data(), pcs.size(), st));
   k_x_pc<<<(npts + 255) / 256, 256, 0, st>>>(npts, Mc, dp.p, W.pcf.p);
-  const size_t npce = (size_t)M.nel * (PP / MX_CH) * M.npnp * 16;
-  k_x_pce<<<(int)std::min<size_t>((npce + 255) / 256, 8 * 148), 256, 0, st>>>(M, PP / MX_CH, Mc, W.pcf.p,
+  const size_t npce = (size_t)neg * nch * M.npnp * 16;
+  k_x_pce<<<(int)std::min<size_t>((npce + 255) / 256, 8 * 148), 256, 0, st>>>(M, nch, neg, lp, Mc, W.pcf.p,
                                                                                W.pcE.p);
   SX_CUDA(cudaGetLastError());
   SX_CUDA(cudaStreamSynchronize(st));
@@ -1228,7 +1344,7 @@ int mixed_solve(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &gro
     W.g_init = W.g_round = nullptr;
     SX_TRY(setup(M, W, groups, nz, num_modes, st));
     int attr_rc = SX_OK;
-    SX_NP_SWITCH_M(M.np, (attr_rc = set_smem_attrs<N_>()));
+    SX_PK_SWITCH(W, SX_NP_SWITCH_M(M.np, (attr_rc = set_smem_attrs<N_, PK_>())));
     SX_TRY(attr_rc);
     bind_params(M, W, nz, d_u, d_f, d_bc, stride);
     if (graphs) {
@@ -1260,7 +1376,10 @@ int mixed_solve(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &gro
     if (worst <= tol_rel) break;
   }
   if (rounds > max_refine) rounds = max_refine;
-  SX_NP_SWITCH_M(M.np, (k_x_unpack<N_><<<dim3(M.nel, PP / MX_CH), 256, 0, st>>>(member_of(M, W))));
+  {
+    const MxMember B = member_of(M, W);
+    SX_PK_SWITCH(W, SX_NP_SWITCH_M(M.np, (k_x_unpack<N_, PK_><<<dim3(B.neg, B.nch), 256, 0, st>>>(B))));
+  }
   SX_CUDA(cudaGetLastError());
   int solved = 0;
   for (const MxGroup &g : groups) solved += g.P;
@@ -1354,10 +1473,10 @@ static int enqueue_round_multi(MxBatch &B, int n_inner, bool check_stop, cudaStr
   *nl = (int)B.cls.size() * (n_inner + 3);
   return per_class(B, st, [&](const MxBatch::Class &c, cudaStream_t s) {
     const MxTable Te = class_table(B, c, 0), Tn = class_table(B, c, 1);
-    SX_NP_SWITCH_M(c.np, (k_cg_multi<N_><<<c.te, N_ * 32, cg_smem(N_), s>>>(Te, 0, CG_INIT)));
+    SX_NP_SWITCH_M(c.np, (k_cg_multi<N_><<<c.te, N_ * 32, cg_smem(N_, c.ep), s>>>(Te, 0, CG_INIT)));
     for (int it = 0; it < n_inner; it++) {
       const int mode = (it == n_inner - 1 ? CG_LAST : CG_ITER) | (check_stop ? CG_CHECK_STOP : 0);
-      SX_NP_SWITCH_M(c.np, (k_cg_multi<N_><<<c.te, N_ * 32, cg_smem(N_), s>>>(Te, it, mode)));
+      SX_NP_SWITCH_M(c.np, (k_cg_multi<N_><<<c.te, N_ * 32, cg_smem(N_, c.ep), s>>>(Te, it, mode)));
     }
     SX_NP_SWITCH_M(c.np, (k_x_op64_multi<N_><<<c.te, N_ * 32, x64_smem(N_), s>>>(Te)));
     k_x_res_multi<<<c.tn, 256, 0, s>>>(Tn);
@@ -1372,7 +1491,8 @@ static int set_smem_attrs_multi() {
                                (int)x64_smem(NP)));
   SX_CUDA(cudaFuncSetAttribute(k_x_op64_multi<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)x64_smem(NP)));
-  SX_CUDA(cudaFuncSetAttribute(k_cg_multi<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(NP)));
+  SX_CUDA(cudaFuncSetAttribute(k_cg_multi<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)cg_smem(NP, MX_EP)));
   SX_CUDA(cudaFuncSetAttribute(k_cg_multi<NP>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   return SX_OK;
 }
@@ -1431,7 +1551,8 @@ int mixed_solve_multi(std::vector<MxItem> &items, MxBatch &B, bool rebuild, doub
       std::vector<int> te(1, 0), tn(1, 0);
       for (int m = c.m0; m < c.m0 + c.count; m++) {
         const MxMember &b = mem[m];
-        te.push_back(te.back() + b.M.nel * b.nch);
+        te.push_back(te.back() + b.neg * b.nch);
+        c.ep = std::max(c.ep, MX_CH / b.lp);
         tn.push_back(tn.back() + b.G * b.nch);
       }
       c.te = te.back();

@@ -9,11 +9,13 @@
 
 namespace sx {
 
-constexpr int MX_CH = 32;  // planes per block chunk (one warp lane per plane)
+// Lanes of a block's chunk.  A chunk is lp = 32, 16 or 8 planes of 32 / lp
+// elements (or nodes): lane l works on plane l % lp of element l / lp.
+constexpr int MX_CH = 32;
 
 // Per-solve constants (device side).
 struct MxParams {
-  int PP;               // padded plane count (multiple of MX_CH)
+  int PP;               // padded plane count (multiple of the chunk's lp)
   int nz;               // real planes in the caller's arrays
   const int *active;    // [PP] 1 for planes this form solves (not the Nyquist
                         // plane, padding, or planes routed to the direct path)
@@ -39,8 +41,8 @@ struct MxScalPtrs {
 
 // Vectors of the FP32 inner iteration in element layout ("E-vectors"): every
 // element keeps its own copy of its nodes' values, chunk-major,
-// V[((e * nch + y) * np^2 + t) * 32 + l] for element e, plane chunk y,
-// tensor node t and lane (plane) l, so one block's data is one contiguous
+// V[((eg * nch + y) * np^2 + t) * 32 + l] for element group eg, plane chunk y,
+// tensor node t and lane l, so one block's data is one contiguous
 // np^2 * 128-byte span that a single TMA bulk copy moves.  The copies of a
 // shared node are updated by every element that holds it, with the same
 // arithmetic on the same inputs, so they stay equal; r, s, p, d are read and
@@ -49,7 +51,7 @@ struct MxScalPtrs {
 struct CgVecs {
   float *rE, *sE, *pE, *dE;
   float *WE[2];       // A u at every element node (unassembled)
-  const float *pcE;   // inverse Jacobi diagonal, [e][y][t][16] by mode pair
+  const float *pcE;   // inverse Jacobi diagonal, [eg][y][t][16] by lane pair
   float *r0;          // residual of the last refinement step, [npts][PP]
   double *x64;
   double *gam[2], *alpha[2], *beta[2];
@@ -73,12 +75,14 @@ struct MxMember {
   double *r2, *b2;   // per-plane ||r||^2 and ||b||^2, read by the host
   double *part;      // reduction partials
   unsigned *cnt;     // reduction counters
-  int nch;           // plane chunks of 32 (P.PP / 32)
+  int nch;           // plane chunks (P.PP / lp)
+  int lp, lsh;       // planes a chunk and its logarithm
+  int neg;           // element groups of 32 / lp
   int G;             // blocks per chunk of the node kernels
 };
 
 struct MixedWork {
-  int PP = 0, npts = 0, n_inner = 0, M = 0, G = 0;
+  int PP = 0, lp = MX_CH, npts = 0, n_inner = 0, M = 0, G = 0;
   DBuf<double> hcon, b64, x64, Ye64, scal, part;
   DBuf<int> nsolve, active, skip;
   DBuf<unsigned> cnt;
@@ -135,12 +139,13 @@ struct MxItem {
 // Device tables, streams and graphs of a multi-mesh mixed-precision solve.
 // Members are ordered by element order; the members of one order form a
 // class, and every kernel runs once per class over all its members' tiles
-// (element tiles: nel * nch per member; node tiles: G * nch), the classes on
+// (element tiles: neg * nch per member; node tiles: G * nch), the classes on
 // their own streams side by side.
 struct MxBatch {
   struct Class {
     int np = 0, m0 = 0, count = 0;  // order, first member, members
     int te = 0, tn = 0;             // element and node tiles
+    int ep = 1;                     // elements a block holds, at most
     size_t t0 = 0;                  // offset of the 2 (count + 1) tile prefixes
   };
   DBuf<MxMember> mem;
