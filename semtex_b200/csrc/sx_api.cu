@@ -113,6 +113,8 @@ namespace sx {
 
 int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const SystemProvider *prov,
                    cudaStream_t st) {
+  // what this call builds: freed in the stream's order if it gives up early
+  std::vector<std::shared_ptr<System>> built;
   std::vector<System *> to_factor;
   M.sys.clear();
   M.uniq.clear();
@@ -144,11 +146,14 @@ int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const Sy
       found->lambda2 = lam[l];
       found->betak2 = bk2[l];
       found->method = kind;
+      SX_TRY(device_pool(M.mesh->device, &found->pool));
+      built.push_back(found);
+      // enqueued; one wait for all of them below
       if (kind == SX_DIRECT) {
-        SX_TRY(system_build_direct(*found, st));
+        SX_TRY(system_build_direct(*found, st, false));
         if (found->nsolve > 0) to_factor.push_back(found.get());
       } else {
-        SX_TRY(system_build_jacobi(*found, st));
+        SX_TRY(system_build_jacobi(*found, st, false));
       }
     }
     if (std::find(M.uniq.begin(), M.uniq.end(), found) == M.uniq.end()) M.uniq.push_back(found);
@@ -158,15 +163,13 @@ int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const Sy
     SX_TRY(M.dstatus.alloc(1));
     SX_TRY(M.dstatus.zero(st));
   }
-  SX_TRY(factor_batch(to_factor, st));
-  for (System *S : to_factor) {
-    int h = 0;
-    SX_CUDA(cudaMemcpyAsync(&h, S->status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    SX_CUDA(cudaStreamSynchronize(st));
-    if (h & (1 << SX_ERR_NOT_SPD)) {
+  SX_TRY(factor_batch(to_factor, st, false));
+  if (!built.empty()) SX_CUDA(cudaStreamSynchronize(st));
+  for (auto &S : built) {
+    const int rc = system_check_status(*S);
+    if (rc == SX_ERR_NOT_SPD)
       set_error("failed to factor Helmholtz matrix (lambda2=%g, betak2=%g)", S->lambda2, S->betak2);
-      return SX_ERR_NOT_SPD;
-    }
+    SX_TRY(rc);
   }
   return SX_OK;
 }
@@ -180,6 +183,7 @@ static int modal_build(sx_mesh m, int base_mode, int num_modes, const double *la
   *out = nullptr;
   std::unique_ptr<sx_modal_s> M(new sx_modal_s());
   M->mesh = m;
+  M->device = m->device;
   M->base_mode = base_mode;
   M->num_modes = num_modes;
   M->method = method;
@@ -206,7 +210,18 @@ extern "C" int sx_modal_create_ex(sx_mesh m, int base_mode, int num_modes, const
 }
 
 extern "C" int sx_modal_destroy(sx_modal s) {
+  if (!s) return SX_OK;
+  // the systems' memory is freed stream-ordered: work the caller enqueued
+  // with them (on any stream) must finish first, and what the pool does not
+  // keep goes back to the device before this returns
+  int dev = -1;
+  cudaGetDevice(&dev);
+  const int home = s->device;
+  if (home != dev) cudaSetDevice(home);
+  cudaDeviceSynchronize();
   delete s;
+  cudaStreamSynchronize(nullptr);
+  if (home != dev) cudaSetDevice(dev);
   return SX_OK;
 }
 
@@ -449,8 +464,9 @@ static int direct_batched(sx_modal_s *s, DirectBatch &B, const std::vector<Group
     modes.push_back(g.mode);
   }
   SX_TRY(reserve_ws(*s, planes));
-  const bool same = B.exec && B.key[0] == d_u && B.key[1] == d_f && B.key[2] == d_bc && B.key[3] == s->rhs.p &&
-                    B.key[4] == s->Fb.p && B.nz == nz && B.stride == plane_stride && B.modes == modes;
+  const bool same = !B.jobs.empty() && B.key[0] == d_u && B.key[1] == d_f && B.key[2] == d_bc &&
+                    B.key[3] == s->rhs.p && B.key[4] == s->Fb.p && B.nz == nz && B.stride == plane_stride &&
+                    B.modes == modes;
   const MeshView M = s->mesh->view();
   if (!same || !s->use_graphs) {
     B.reset();
@@ -468,10 +484,24 @@ static int direct_batched(sx_modal_s *s, DirectBatch &B, const std::vector<Group
     B.sc = s->sched((int)jobs.size());
     B.jobs = jobs;
     B.modes = modes;
-    if (!s->use_graphs) return direct_solve_jobs(M, B.djobs.p, jobs, st, B.sc, &B.launches);
+    B.key[0] = d_u;
+    B.key[1] = d_f;
+    B.key[2] = d_bc;
+    B.key[3] = s->rhs.p;
+    B.key[4] = s->Fb.p;
+    B.nz = nz;
+    B.stride = plane_stride;
+    // enqueued as it is: a program that solves once does not pay for a graph
+    return direct_solve_jobs(M, B.djobs.p, jobs, st, B.sc, &B.launches);
+  }
+  if (!B.exec) {  // the second call with these arguments: captured, and replayed from here on
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SX_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone)  // the caller's own capture takes the launches themselves
+      return direct_solve_jobs(M, B.djobs.p, B.jobs, st, B.sc, &B.launches);
     cudaGraph_t g = nullptr;
     SX_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    const int rc = direct_solve_jobs(M, B.djobs.p, jobs, st, B.sc, &B.launches);
+    const int rc = direct_solve_jobs(M, B.djobs.p, B.jobs, st, B.sc, &B.launches);
     const cudaError_t ce = cudaStreamEndCapture(st, &g);
     if (rc != SX_OK) {
       if (g) cudaGraphDestroy(g);
@@ -481,13 +511,6 @@ static int direct_batched(sx_modal_s *s, DirectBatch &B, const std::vector<Group
     const cudaError_t ie = cudaGraphInstantiate(&B.exec, g, 0);
     cudaGraphDestroy(g);
     SX_CUDA(ie);
-    B.key[0] = d_u;
-    B.key[1] = d_f;
-    B.key[2] = d_bc;
-    B.key[3] = s->rhs.p;
-    B.key[4] = s->Fb.p;
-    B.nz = nz;
-    B.stride = plane_stride;
   }
   SX_CUDA(cudaGraphLaunch(B.exec, st));
   return SX_OK;

@@ -56,6 +56,21 @@ void gll_tables(int np, std::vector<double> &z, std::vector<double> &w, std::vec
     if (s_ != SX_OK) return s_; \
   } while (0)
 
+// The stream-ordered pool that meshes and modal systems of a device live in,
+// and giving back what the current device's pool keeps but does not use.
+int device_pool(int device, cudaMemPool_t *out);
+void device_pool_trim();
+
+// An allocation, tried again without the pool's idle memory when it fails.
+template <typename F>
+cudaError_t or_trimmed(F &&f) {
+  cudaError_t e = f();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  device_pool_trim();
+  return f();
+}
+
 // Device buffer with RAII release.
 // alloc()/upload() use cudaMalloc (long-lived data); alloc_on()/upload_on()
 // use the stream-ordered allocator on a stream, so releasing a temporary
@@ -84,7 +99,7 @@ struct DBuf {
   int alloc_on(size_t count, cudaStream_t s) {
     release();
     if (count == 0) count = 1;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&p), count * sizeof(T), s);
+    const cudaError_t e = or_trimmed([&]() { return cudaMallocAsync(reinterpret_cast<void **>(&p), count * sizeof(T), s); });
     if (e != cudaSuccess) {
       p = nullptr;
       set_error("cudaMallocAsync(%zu bytes): %s", count * sizeof(T), cudaGetErrorString(e));
@@ -103,7 +118,7 @@ struct DBuf {
   int alloc(size_t count) {
     release();
     if (count == 0) count = 1;
-    cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    const cudaError_t e = or_trimmed([&]() { return cudaMalloc(&p, count * sizeof(T)); });
     if (e != cudaSuccess) {
       p = nullptr;
       set_error("cudaMalloc(%zu bytes): %s", count * sizeof(T), cudaGetErrorString(e));
@@ -120,7 +135,8 @@ struct DBuf {
     if (!pool) return free_on_s ? alloc_on(count, s) : alloc(count);
     release();
     if (count == 0) count = 1;
-    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), count * sizeof(T), pool, s);
+    const cudaError_t e =
+        or_trimmed([&]() { return cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), count * sizeof(T), pool, s); });
     if (e != cudaSuccess) {
       p = nullptr;
       set_error("cudaMallocFromPoolAsync(%zu bytes): %s", count * sizeof(T), cudaGetErrorString(e));

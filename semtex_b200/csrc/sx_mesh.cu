@@ -288,18 +288,19 @@ int mesh_kratio(const sx_mesh_desc *d, double *out) {
 
 }  // namespace sx
 
-// Device memory of meshes comes from a stream-ordered pool of their own
-// (one per device), so that dropping a mesh frees its memory without the
-// device-wide synchronisation of cudaFree (a server drops one per request
-// while other requests run), and creating one waits for nothing but its own
-// copies.  Up to MESH_POOL_KEEP bytes of freed mesh memory stay mapped for
-// the next mesh.
-constexpr uint64_t MESH_POOL_KEEP = uint64_t(4) << 30;
+// Device memory of meshes and of the systems a modal object builds comes from
+// a stream-ordered pool of their own (one per device), so that making and
+// dropping them costs no device-wide synchronisation per buffer (a server
+// drops a mesh per request while other requests run; a program that builds
+// systems for one solve makes and frees five buffers a mode).  Up to
+// POOL_KEEP bytes of freed memory stay mapped for the next ones.
+constexpr uint64_t POOL_KEEP = uint64_t(4) << 30;
 
-static int mesh_pool(int device, cudaMemPool_t *out) {
-  static std::mutex mu;
-  static std::map<int, cudaMemPool_t> pools;
-  std::lock_guard<std::mutex> lk(mu);
+static std::mutex pool_mu;
+static std::map<int, cudaMemPool_t> pools;
+
+int sx::device_pool(int device, cudaMemPool_t *out) {
+  std::lock_guard<std::mutex> lk(pool_mu);
   auto it = pools.find(device);
   if (it == pools.end()) {
     cudaMemPoolProps props = {};
@@ -309,7 +310,7 @@ static int mesh_pool(int device, cudaMemPool_t *out) {
     props.location.id = device;
     cudaMemPool_t pool = nullptr;
     SX_CUDA(cudaMemPoolCreate(&pool, &props));
-    uint64_t keep = MESH_POOL_KEEP;
+    uint64_t keep = POOL_KEEP;
     SX_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
     it = pools.emplace(device, pool).first;
   }
@@ -317,12 +318,20 @@ static int mesh_pool(int device, cudaMemPool_t *out) {
   return SX_OK;
 }
 
+void sx::device_pool_trim() {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  std::lock_guard<std::mutex> lk(pool_mu);
+  auto it = pools.find(dev);
+  if (it != pools.end()) cudaMemPoolTrimTo(it->second, 0);
+}
+
 // The pool and a private stream for one mesh's uploads.
 struct MeshUpload {
   cudaMemPool_t pool = nullptr;
   cudaStream_t s = nullptr;
   int begin(int device) {
-    SX_TRY(mesh_pool(device, &pool));
+    SX_TRY(device_pool(device, &pool));
     SX_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     return SX_OK;
   }

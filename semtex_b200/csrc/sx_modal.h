@@ -41,6 +41,7 @@ struct DirectBatch {
 
 struct sx_modal_s {
   sx_mesh_s *mesh = nullptr;
+  int device = 0;
   int base_mode = 0, num_modes = 0, method = SX_DIRECT;
   std::vector<std::shared_ptr<sx::System>> sys;   // per local mode
   std::vector<std::shared_ptr<sx::System>> uniq;  // distinct systems
