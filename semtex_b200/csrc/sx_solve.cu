@@ -18,6 +18,7 @@
 //                 (src/field.cpp:1022-1040)
 #include "sx_internal.h"
 #include "sx_kernels.cuh"
+#include "sx_ptx.cuh"
 #include "sx_solve.cuh"
 
 namespace sx {
@@ -26,41 +27,48 @@ namespace sx {
 // Element forcing and condensation
 // ---------------------------------------------------------------------------
 
-// One block of ELEM_WARPS warps per (element, job); both planes of the job in
-// one pass, so the element's hbi block is read once per job.  Warp w owns
-// rows b = w, w + ELEM_WARPS, ... of hbi (hbi hii^-1), its lanes the row's
-// NI columns: the whole block is loaded into registers, coalesced and
-// evict-first (it is not read again before the band sweeps have streamed
-// the factor through L2), before anything else, so that it arrives while
-// the forcing and the element operator are computed.  The geometric factors
-// of the operator are read only for elements that hold essential nodes.
-constexpr int ELEM_WARPS = 4;
+// One block of RHS_THREADS threads per (element, job); both planes of the job
+// in one pass, so the element's hbi block (hbi hii^-1, NE x NI) is read once
+// per job.  It goes to shared memory by 16-byte asynchronous copies issued
+// before anything else, so that it arrives while the forcing and the element
+// operator are computed; four neighbouring threads then share a row, so that a
+// row's sum takes two shuffles.  The geometric factors of the operator are
+// read only for elements that hold essential nodes.
+//   HBM bounds it: the block's bytes.  Against a warp a row, its loads held in
+// registers across the operator: 32 systems of 1024 elements of order 8 218 ->
+// 145 us (3.9 TB/s), 12 of 4096 of order 10 495 -> 415 us, 20 of 851 of order
+// 7 110 -> 54 us.
+constexpr int RHS_THREADS = 128;
 
 template <int NP>
-__global__ void __launch_bounds__(ELEM_WARPS * 32) k_rhs_elem(MeshView M, const Job *__restrict__ jobs) {
-  constexpr int NN = NP * NP, NE = 4 * (NP - 1), NI = NN - NE;
-  constexpr int NT = ELEM_WARPS * 32, RW = (NE + ELEM_WARPS - 1) / ELEM_WARPS, QL = (NI + 31) / 32;
-  const Job J = jobs[blockIdx.y];
-  const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+constexpr size_t rhs_smem() {
+  return (size_t)(4 * (NP - 1)) * (NP * NP - 4 * (NP - 1)) * sizeof(double);
+}
+
+template <int NP>
+__global__ void __launch_bounds__(RHS_THREADS) k_rhs_elem(MeshView M, const Job *__restrict__ jobs) {
+  constexpr int NN = NP * NP, NE = 4 * (NP - 1), NI = NN - NE, NT = RHS_THREADS;
+  const Job &J = jobs[blockIdx.y];
+  const int e = blockIdx.x, tid = threadIdx.x;
+  extern __shared__ __align__(16) double H[];  // hbi hii^-1, row-major
+  {
+    const double *hbi = J.hbi + (size_t)e * NE * NI;
+    for (int i = tid; i < NE * NI / 2; i += NT) cp_async16_cg(H + 2 * i, hbi + 2 * i);
+    cp_async_commit();
+  }
   const int P = J.P;
-  const double *hbi = J.hbi + (size_t)e * NE * NI;
-  double h[RW][QL];
-#pragma unroll
-  for (int k = 0; k < RW; k++)
-#pragma unroll
-    for (int j = 0; j < QL; j++) {
-      const int b = w + ELEM_WARPS * k, q = lane + 32 * j;
-      h[k][j] = (b < NE && q < NI) ? __ldcs(hbi + b * NI + q) : 0.0;
-    }
+  const size_t fs = (size_t)J.fstride;
   __shared__ double F[2][NN], Fe[2][NN];
   __shared__ double D[NN], Q[4][NN], u[NN], R[NN], S[NN], T[NN];
   __shared__ int emap[NN];
   const size_t eo = (size_t)e * NN;
+  double *const f = J.f + eo;
   const bool masked = M.emask[e] != 0;
   for (int i = tid; i < NN; i += NT) {
     emap[i] = M.emap[i];
     const double q8 = M.Q8[eo + i];
-    for (int p = 0; p < P; p++) F[p][i] = q8 * J.f[(size_t)p * J.fstride + eo + i];
+    F[0][i] = q8 * f[i];
+    F[1][i] = P > 1 ? q8 * f[fs + i] : 0.0;
   }
   if (masked) {
     // f <- M f + H g: the operator applied to the element's essential values
@@ -86,37 +94,41 @@ __global__ void __launch_bounds__(ELEM_WARPS * 32) k_rhs_elem(MeshView M, const 
   }
   __syncthreads();
   // boundary-first element ordering, negated: f <- -(M f + H g)
-  for (int a = tid; a < NN; a += NT)
-    for (int p = 0; p < P; p++) Fe[p][a] = -F[p][emap[a]];
-  __syncthreads();
-  // F_b -= (hbi hii^-1) F_i: row b of the block against the interior values
-#pragma unroll
-  for (int k = 0; k < RW; k++) {
-    const int b = w + ELEM_WARPS * k;
-    double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-    for (int j = 0; j < QL; j++) {
-      const int q = lane + 32 * j;
-      if (q < NI) {
-        s0 += h[k][j] * Fe[0][NE + q];
-        if (P > 1) s1 += h[k][j] * Fe[1][NE + q];
-      }
-    }
-    s0 = warp_sum(s0);
-    if (P > 1) s1 = warp_sum(s1);
-    if (lane == 0 && b < NE) {
-      const double v0 = Fe[0][b] - s0;
-      J.Fb[(size_t)e * NE + b] = v0;
-      J.f[eo + b] = v0;
-      if (P > 1) {
-        const double v1 = Fe[1][b] - s1;
-        J.Fb[((size_t)M.nel + e) * NE + b] = v1;
-        J.f[(size_t)J.fstride + eo + b] = v1;
-      }
+  for (int a = tid; a < NN; a += NT) {
+    const int n = emap[a];
+    const double v0 = -F[0][n], v1 = -F[1][n];
+    Fe[0][a] = v0;
+    Fe[1][a] = v1;
+    if (a >= NE) {
+      f[a] = v0;
+      if (P > 1) f[fs + a] = v1;
     }
   }
-  for (int i = NE + tid; i < NN; i += NT)
-    for (int p = 0; p < P; p++) J.f[(size_t)p * J.fstride + eo + i] = Fe[p][i];
+  cp_async_wait_all();
+  __syncthreads();
+  // F_b -= (hbi hii^-1) F_i: row b of the block against the interior values
+  const int s = tid & 3;
+  for (int b0 = 0; b0 < NE; b0 += NT / 4) {
+    const int b = b0 + (tid >> 2);
+    double s0 = 0.0, s1 = 0.0;
+    if (b < NE) {
+      const double *h = H + b * NI;
+#pragma unroll 4
+      for (int q = s; q < NI; q += 4) {
+        s0 = fma(h[q], Fe[0][NE + q], s0);
+        s1 = fma(h[q], Fe[1][NE + q], s1);
+      }
+    }
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+    if (s < P && b < NE) {  // thread 0 of the four stores plane 0, thread 1 plane 1
+      const double v = Fe[s][b] - (s == 0 ? s0 : s1);
+      J.Fb[((size_t)s * M.nel + e) * NE + b] = v;
+      f[s * fs + b] = v;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -228,7 +240,7 @@ template <int NP>
 static void launch_elem(const MeshView &M, const Job *djobs, int njobs, bool rhs, cudaStream_t st) {
   dim3 grid(M.nel, njobs);
   if (rhs)
-    k_rhs_elem<NP><<<grid, ELEM_WARPS * 32, 0, st>>>(M, djobs);
+    k_rhs_elem<NP><<<grid, RHS_THREADS, rhs_smem<NP>(), st>>>(M, djobs);
   else
     k_backsub<NP><<<grid, back_threads<NP>(), 0, st>>>(M, djobs);
 }
@@ -246,6 +258,9 @@ static void dispatch_elem(const MeshView &M, const Job *djobs, int njobs, bool r
 
 int prepare_direct_kernels(const MeshView &M) {
   if (M.np < 3 || M.np > 12) return SX_ERR_UNSUPPORTED;
+  // the one order whose block and work arrays exceed 48 KB together
+  if (M.np == 12)
+    SX_CUDA(cudaFuncSetAttribute(k_rhs_elem<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rhs_smem<12>()));
   return prepare_band_kernels();
 }
 
