@@ -95,7 +95,18 @@ static_assert(NEAR + 1 == DEPTH, "the ranks' one wait a step covers their younge
 
 // Blocks in a CTA's window: every block a step multiplies (j <= J), and
 // those whose arrival a rank waits for before it reuses a partial's slot.
-__host__ __device__ __forceinline__ int window_blocks(int J) { return max(J, DEPTH) + 2; }
+// Bands of more than WINDOW_MAX - 2 tiles a block column do not fit beside a
+// ring of tiles: the WIDE kernel keeps the most recent WIDE_WINDOW blocks and
+// reads older ones from the right-hand sides' array through L2.  The D_k then
+// follow the forward sweep, which still needs that array's z_k.  Two systems,
+// 16 CTAs each (full window / WIDE): 103 blocks of 102 tiles 0.56 / 0.62 ms,
+// 121 of 120 tiles 1.28 / 0.79 (one tile in flight beside the full window).
+constexpr int WINDOW_MAX = 112, WIDE_WINDOW = 64;
+__host__ __device__ __forceinline__ int full_window(int J) { return max(J, DEPTH) + 2; }
+__host__ __device__ __forceinline__ int window_blocks(int J) {
+  return full_window(J) > WINDOW_MAX ? WIDE_WINDOW : full_window(J);
+}
+static bool wide_band(int J) { return full_window(J) > WINDOW_MAX; }
 
 // Doubles of the warps' sums and the leader's partial sums (see the kernel).
 __host__ __device__ __forceinline__ int red_doubles(int C) {
@@ -110,13 +121,32 @@ struct TileRegs {
   double2 a[RPW], z[RPW];
 };
 template <bool FWD>
-__device__ __forceinline__ void tile_load(TileRegs &r, const double *T, const double *z, int w, int lane) {
-  const double2 *t2 = reinterpret_cast<const double2 *>(T) + w * RPW * (NB / 2) + lane;
+__device__ __forceinline__ void block_load(TileRegs &r, const double *z, int w, int lane) {
   const double2 *z2 = reinterpret_cast<const double2 *>(z) + (FWD ? w * RPW : lane);
 #pragma unroll
   for (int i = 0; i < (FWD ? RPW : 2); i++) r.z[i] = z2[FWD ? i : i * (NB / 2)];
+}
+// The same from the right-hand sides' array (z0, z1: the planes' block; a lone
+// plane stands in for both, and what it gives the second is never stored).
+template <bool FWD>
+__device__ __forceinline__ void block_load_l2(TileRegs &r, const double *z0, const double *z1, int w, int lane) {
+  if (FWD) {
+#pragma unroll
+    for (int i = 0; i < RPW; i++) r.z[i] = make_double2(__ldcg(z0 + w * RPW + i), __ldcg(z1 + w * RPW + i));
+  } else {
+    r.z[0] = __ldcg(reinterpret_cast<const double2 *>(z0) + lane);
+    r.z[1] = __ldcg(reinterpret_cast<const double2 *>(z1) + lane);
+  }
+}
+__device__ __forceinline__ void rows_load(TileRegs &r, const double *T, int w, int lane) {
+  const double2 *t2 = reinterpret_cast<const double2 *>(T) + w * RPW * (NB / 2) + lane;
 #pragma unroll
   for (int i = 0; i < RPW; i++) r.a[i] = t2[i * (NB / 2)];
+}
+template <bool FWD>
+__device__ __forceinline__ void tile_load(TileRegs &r, const double *T, const double *z, int w, int lane) {
+  block_load<FWD>(r, z, w, lane);
+  rows_load(r, T, w, lane);
 }
 // Forward: acc (two columns, two planes) += T^T z; backward: acc (the rows, two
 // planes) += this lane's columns of T times z.
@@ -204,6 +234,7 @@ using Bwd = std::false_type;
 
 }  // namespace
 
+template <bool WIDE>
 __global__ void __launch_bounds__(SWP_THREADS, 1)
     k_band_sweep(const Job *__restrict__ jobs, int C, int S, int Wmax, int Q) {
   const int rank = (int)cluster_ctarank();
@@ -219,7 +250,8 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
   double *red = zwin + (size_t)Wmax * VEC;
   double *pbuf = red + SWP_WARPS * RED;
   double *vd = red + red_doubles(C);                            // D_k^T z_k
-  uint64_t *full = reinterpret_cast<uint64_t *>(vd + VEC);      // S
+  double *zd = vd + VEC;                                        // WIDE: z_k of a D_k
+  uint64_t *full = reinterpret_cast<uint64_t *>(zd + (WIDE ? VEC : 0));  // S
   uint64_t *empty = full + S;                                   // S
   uint64_t *zbar = empty + S;                                   // Wmax
   uint64_t *pbar = zbar + Wmax;                                 // D
@@ -253,59 +285,69 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
   if (w == SWP_WARPS) {
     // ---- the copying warp: every tile this CTA reads, in its order of use
     cluster_arrive();  // the barrier between the sweeps: nothing to wait for here
-    if (lane == 0) {
-      long long n = 0;  // tiles issued
-      int slot = 0;
-      uint32_t use = 0;  // times the ring has gone round
-      bool stop = false;
-      auto issue = [&](const double *src) {
-        if (stop) return;
-        if (use > 0) {
-          if (!mbar_wait_tx(&empty[slot], (use - 1) & 1, lim)) *aborted = 1;
-          if (*aborted) {
-            stop = true;
-            return;
-          }
+    long long n = 0;  // tiles issued
+    int slot = 0;
+    uint32_t use = 0;  // times the ring has gone round
+    bool stop = false;
+    auto issue = [&](const double *src) {
+      if (stop) return;
+      if (use > 0) {
+        if (!mbar_wait_tx(&empty[slot], (use - 1) & 1, lim)) *aborted = 1;
+        if (*aborted) {
+          stop = true;
+          return;
         }
-        mbar_arrive_expect_tx(&full[slot], (uint32_t)(TSZ * sizeof(double)));
-        bulk_g2s(ring + (size_t)slot * TSZ, src, (uint32_t)(TSZ * sizeof(double)), &full[slot]);
-        n++;
-        if (++slot == S) {
-          slot = 0;
-          use++;
-        }
-      };
-      const size_t J1 = J + 1;
-      auto off = [&](int t, int j) {  // tile j of step t
-        return Jb.tiles + ((size_t)(t < nblk ? t : 2 * nblk - 1 - t + j) * J1 + j) * TSZ;
-      };
-      int cnt = 0;
+      }
+      mbar_arrive_expect_tx(&full[slot], (uint32_t)(TSZ * sizeof(double)));
+      bulk_g2s(ring + (size_t)slot * TSZ, src, (uint32_t)(TSZ * sizeof(double)), &full[slot]);
+      n++;
+      if (++slot == S) {
+        slot = 0;
+        use++;
+      }
+    };
+    const size_t J1 = J + 1;
+    auto off = [&](int t, int j) {  // tile j of step t
+      return Jb.tiles + ((size_t)(t < nblk ? t : 2 * nblk - 1 - t + j) * J1 + j) * TSZ;
+    };
+    auto diag = [&](int k) { issue(Jb.dinv + (size_t)k * TSZ); };
+    int cnt = 0, jm = tab.jmax(0), dm = 0;  // dm: block t - DLAG modulo C - 1
+    auto steps = [&](int t0, int t1) {
       if (rank == 0) {
-        int jm = tab.jmax(0);
-        for (int t = 0; t < T && !stop; t++) {
+        for (int t = t0; t < t1 && !stop; t++) {
           if (jm >= 1) issue(off(t, 1));
-          if (C == 1 && t < nblk) issue(Jb.dinv + (size_t)t * TSZ);
+          if (!WIDE && C == 1 && t < nblk) diag(t);
           jm = tab.jmax(t + 1);
           cnt = own_count(own, len, cnt, jm);
           for (int i = cnt - 1; i >= 0; i--) issue(off(t + 1, own[i]));
           for (int j = min(jm, NEAR); j >= 2; j--) issue(off(t + 1, j));
         }
       } else {
-        int dm = 0;  // block t - DLAG modulo C - 1
-        for (int t = 0; t < T && !stop; t++) {
-          if (t >= DLAG && t < nblk) {
-            if (dm == rank - 1) issue(Jb.dinv + (size_t)(t - DLAG) * TSZ);
+        for (int t = t0; t < t1 && !stop; t++) {
+          if (!WIDE && t >= DLAG && t < nblk) {
+            if (dm == rank - 1) diag(t - DLAG);
             if (++dm == C - 1) dm = 0;
           }
           cnt = own_count(own, len, cnt, tab.jmax(t));
           for (int i = cnt - 1; i >= 0; i--) issue(off(t, own[i]));
-          if (t == nblk - 1)
+          if (!WIDE && t == nblk - 1)
             for (int k = max(0, nblk - DLAG); k < nblk; k++) {
-              if (dm == rank - 1) issue(Jb.dinv + (size_t)k * TSZ);
+              if (dm == rank - 1) diag(k);
               if (++dm == C - 1) dm = 0;
             }
         }
       }
+    };
+    if (WIDE) {  // the D_k between the sweeps, each CTA its share
+      if (lane == 0) steps(0, nblk);
+      __syncwarp();
+      cluster_wait();
+      cluster_arrive();
+      if (lane == 0)
+        for (int k = rank; k < nblk; k += C) diag(k);
+    }
+    if (lane == 0) {
+      steps(WIDE ? nblk : 0, T);
       // the copies still in flight (none unless the sweep was given up)
       for (int s = 0; s < S && s < n; s++) {
         const uint32_t u = s < slot ? use : use - 1;  // the slot's last use
@@ -352,13 +394,21 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
 #pragma unroll
     for (int i = 0; i < 2 * RPW; i++) acc[i] = 0.0;
   };
-  // acc += tile j of a step whose window slot is bs times the block solved j
-  // steps before it, which the caller knows to be in the window
-  auto tile = [&](auto F, int j, int bs) {
+  // acc += tile j of step t, whose window slot is bs, times the block solved j
+  // steps before it, which the caller knows to be there
+  auto tile = [&](auto F, int j, int bs, int t) {
     const int zs = bs - j < 0 ? bs - j + W : bs - j;
     TileRegs r;
-    await_tile();
-    tile_load<decltype(F)::value>(r, ring + (size_t)cs * TSZ, zwin + (size_t)zs * VEC, w, lane);
+    if (WIDE && j > W) {
+      const int so = t - j;
+      const double *z0 = Jb.rhs + (size_t)(so < nblk ? so : T - 1 - so) * NB;
+      block_load_l2<decltype(F)::value>(r, z0, P > 1 ? z0 + Jb.rhs_stride : z0, w, lane);
+      await_tile();
+      rows_load(r, ring + (size_t)cs * TSZ, w, lane);
+    } else {
+      await_tile();
+      tile_load<decltype(F)::value>(r, ring + (size_t)cs * TSZ, zwin + (size_t)zs * VEC, w, lane);
+    }
     release();
     tile_fma<decltype(F)::value>(r, acc);
   };
@@ -381,13 +431,13 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
     return ((q[0] + q[RED]) + (q[2 * RED] + q[3 * RED])) + o;
   };
   auto none = []() { return 0.0; };
-  // w_k = D_k D_k^T z_k from the window slot zs, into rhs
-  auto apply_d = [&](int k, int zs, int par) {
+  // w_k = D_k D_k^T z_k, z in the order of a forward sweep, into rhs
+  auto apply_d = [&](int k, const double *z, int par) {
     clear();
     TileRegs r;
     await_tile();
     const double *t = ring + (size_t)cs * TSZ;
-    tile_load<true>(r, t, zwin + (size_t)zs * VEC, w, lane);
+    tile_load<true>(r, t, z, w, lane);
     tile_fma<true>(r, acc);
     const double v = lane_sum(reduce(Fwd(), par, none));
     if (q4 == 0) vd[pb] = v;
@@ -404,6 +454,18 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
     __syncwarp();
     cluster_arrive();
     cluster_wait();
+  };
+
+  // WIDE: the D_k of this CTA's share, once every z_k is in rhs
+  auto wide_diags = [&]() {
+    if constexpr (WIDE) {
+      for (int k = rank; k < nblk; k += C) {
+        if (q4 == 0) zd[pf] = ep < P ? __ldcg(gx + (size_t)k * NB) : 0.0;
+        bar_sync(1, SWP_WARPS * 32);
+        apply_d(k, zd, 0);
+      }
+      between_sweeps();
+    }
   };
 
   clear();
@@ -424,7 +486,7 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
     auto step = [&](auto F, int t) {
       const int e2 = tab.entry(t + 2);
       const bool parts = C > 1 && mbar_test_cta(&pbar[ps], pp);  // the ranks' partial sums are here
-      if (jm >= 1) tile(F, 1, bs);
+      if (jm >= 1) tile(F, 1, bs, t);
       const double s = reduce(F, t & 1, [&]() {
         double o = 0.0;
         if (C > 1) {
@@ -437,6 +499,11 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
       const double z = b - lane_sum(s);
       const int zo = bs * VEC + (decltype(F)::value ? pf : pb);
       if (q4 == 0) zwin[zo] = z;
+      if (WIDE) {  // in rhs before any rank can know the block is there, whichever lane tells it
+        if (q4 == 0 && ep < P) gx[(size_t)(decltype(F)::value ? t : T - 1 - t) * NB] = z;
+        __threadfence();
+        __syncwarp();
+      }
       if (C > 1 && !dead) {
 #pragma unroll
         for (int i = 0; i < NTO; i++)
@@ -447,11 +514,11 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
         mbar_arrive_expect_tx(&pbar[ps], (C - 1) * VEC * sizeof(double));
       // the next step's right-hand side (the first backward one is read after the barrier)
       const int tn = t + 1;
-      if (!decltype(F)::value && q4 == 0 && ep < P) gx[(size_t)(T - 1 - t) * NB] = z;
+      if (!WIDE && !decltype(F)::value && q4 == 0 && ep < P) gx[(size_t)(T - 1 - t) * NB] = z;
       if (tn < T && tn != nblk && ep < P) b = __ldcg(gx + (size_t)(tn < nblk ? tn : T - 1 - tn) * NB);
       bar_sync(1, SWP_WARPS * 32);
       clear();
-      if (C == 1 && decltype(F)::value) apply_d(t, bs, t & 1);
+      if (!WIDE && C == 1 && decltype(F)::value) apply_d(t, zwin + (size_t)bs * VEC, t & 1);
       if (++bs == W) {
         bs = 0;
         bp ^= 1u;
@@ -464,12 +531,13 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
       e1 = e2;
       if (len > 0) {
         cnt = own_count(own, len, cnt, jm);
-        for (int i = cnt - 1; i >= 0; i--) tile(F, own[i], bs);
+        for (int i = cnt - 1; i >= 0; i--) tile(F, own[i], bs, tn);
       }
-      for (int j = min(jm, NEAR); j >= 2; j--) tile(F, j, bs);
+      for (int j = min(jm, NEAR); j >= 2; j--) tile(F, j, bs, tn);
     };
     for (int t = 0; t < nblk; t++) step(Fwd(), t);
     between_sweeps();
+    wide_diags();
     if (nblk > 0 && ep < P) b = __ldcg(gx + (size_t)(nblk - 1) * NB);
     for (int t = nblk; t < T; t++) step(Bwd(), t);
   } else {
@@ -494,12 +562,12 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
         wait(&zbar[bs], bp ^ 1u);
         if (!dead) mbar_arrive_expect_tx(&zbar[bs], VEC * sizeof(double));
       }
-      if (decltype(F)::value && t >= DLAG) {
+      if (!WIDE && decltype(F)::value && t >= DLAG) {
         if (dm == rank - 1) {
           uint32_t par;
           const int zs = slot_back(DLAG, par);
           wait(&zbar[zs], par);
-          apply_d(t - DLAG, zs, t & 1);
+          apply_d(t - DLAG, zwin + (size_t)zs * VEC, t & 1);
         }
         if (++dm == C - 1) dm = 0;
       }
@@ -514,12 +582,13 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
         const int zs = slot_back(D, par);
         wait(&zbar[zs], par);
         waited = true;
+        if (WIDE) __threadfence();  // the leader's stores to rhs before it
       };
       cnt = own_count(own, len, cnt, jm);
       for (int i = cnt - 1; i >= 0; i--) {
         const int j = own[i];
         if (j <= D) wait_block();
-        tile(F, j, bs);
+        tile(F, j, bs, t);
       }
       const double s = lane_sum(reduce(F, t & 1, none));
       wait_block();
@@ -533,16 +602,18 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
       if (++ps == D) ps = 0;
     };
     for (int t = 0; t < nblk; t++) step(Fwd(), t);
-    for (int k = max(0, nblk - DLAG); k < nblk; k++) {
-      if (dm == rank - 1) {
-        uint32_t par;
-        const int zs = slot_back(nblk - k, par);
-        wait(&zbar[zs], par);
-        apply_d(k, zs, nblk & 1);  // not the buffer that step nblk - 1 may still be reading
+    if (!WIDE)
+      for (int k = max(0, nblk - DLAG); k < nblk; k++) {
+        if (dm == rank - 1) {
+          uint32_t par;
+          const int zs = slot_back(nblk - k, par);
+          wait(&zbar[zs], par);
+          apply_d(k, zwin + (size_t)zs * VEC, nblk & 1);  // not the buffer that step nblk - 1 may still be reading
+        }
+        if (++dm == C - 1) dm = 0;
       }
-      if (++dm == C - 1) dm = 0;
-    }
     between_sweeps();
+    wide_diags();
     for (int t = nblk; t < T; t++) step(Bwd(), t);
     // every block the leader sent has landed before this CTA leaves
     for (int back = min(W, T); back >= 1; back--) {
@@ -563,10 +634,14 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
   }
 }
 
-static size_t sweep_smem(int C, int S, int Wmax) {
-  return sizeof(double) * ((size_t)S * TSZ + ((size_t)Wmax + 1) * VEC + red_doubles(C)) +
-         sizeof(uint64_t) * (2 * S + Wmax + DEPTH) + ((sizeof(unsigned short) * (Wmax + 1) + 15) & ~(size_t)15);
+// J: the most tiles a block column of the launch; W: its largest window.
+static size_t sweep_smem(int C, int S, int J, int W) {
+  return sizeof(double) * ((size_t)S * TSZ + ((size_t)W + 1 + wide_band(J)) * VEC + red_doubles(C)) +
+         sizeof(uint64_t) * (2 * S + W + DEPTH) + ((sizeof(unsigned short) * (J + 1) + 15) & ~(size_t)15);
 }
+
+using SweepKernel = void (*)(const Job *, int, int, int, int);
+static SweepKernel sweep_kernel(int J) { return wide_band(J) ? k_band_sweep<true> : k_band_sweep<false>; }
 
 // Dynamic shared memory available to the sweep kernel: the opt-in limit
 // minus its static shared memory.
@@ -576,17 +651,18 @@ static int smem_optin() {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes a;
-    cudaFuncGetAttributes(&a, k_band_sweep);
-    v = optin - (int)a.sharedSizeBytes;
+    cudaFuncAttributes a, b;
+    cudaFuncGetAttributes(&a, k_band_sweep<false>);
+    cudaFuncGetAttributes(&b, k_band_sweep<true>);
+    v = optin - (int)std::max(a.sharedSizeBytes, b.sharedSizeBytes);
   }
   return v;
 }
 
 // The deepest ring of at most smax tiles that fits (0: none).
-static int fit_stages(int C, int smax, int Wmax) {
+static int fit_stages(int C, int smax, int J, int W) {
   int S = std::max(1, std::min(smax, BAND_STAGES_MAX));
-  while (S > 0 && sweep_smem(C, S, Wmax) > (size_t)smem_optin()) S--;
+  while (S > 0 && sweep_smem(C, S, J, W) > (size_t)smem_optin()) S--;
   return S;
 }
 
@@ -595,21 +671,23 @@ int band_sweep_jobs(const Job *djobs, const std::vector<Job> &hjobs, const BandS
   const int C = sc.C;
   const int nj = (int)hjobs.size();
   if (nj == 0) return SX_OK;
-  int maxP = 0, Wmax = 0;
+  // one wide band makes it the WIDE kernel for all, which takes any band
+  int maxP = 0, J = 0, Wmax = 0;
   for (const Job &j : hjobs) {
     maxP = std::max(maxP, j.P);
+    J = std::max(J, j.J);
     Wmax = std::max(Wmax, window_blocks(j.J));
   }
   if (maxP > 2) return SX_ERR_UNSUPPORTED;
-  const int S = fit_stages(C, sc.S, Wmax);
+  const int S = fit_stages(C, sc.S, J, Wmax);
   if (S < 1) {
-    set_error("band sweep needs %zu B of shared memory (limit %d)", sweep_smem(C, 1, Wmax), smem_optin());
+    set_error("band sweep needs %zu B of shared memory (limit %d)", sweep_smem(C, 1, J, Wmax), smem_optin());
     return SX_ERR_UNSUPPORTED;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C * nj, 1, 1);
   cfg.blockDim = dim3(SWP_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = sweep_smem(C, S, Wmax);
+  cfg.dynamicSmemBytes = sweep_smem(C, S, J, Wmax);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -618,14 +696,16 @@ int band_sweep_jobs(const Job *djobs, const std::vector<Job> &hjobs, const BandS
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  SX_CUDA(cudaLaunchKernelEx(&cfg, k_band_sweep, djobs, C, S, Wmax, std::max(sc.Q, 0)));
+  SX_CUDA(cudaLaunchKernelEx(&cfg, sweep_kernel(J), djobs, C, S, Wmax, std::max(sc.Q, 0)));
   return SX_OK;
 }
 
 int prepare_band_kernels() {
   const int limit = smem_optin();
-  SX_CUDA(cudaFuncSetAttribute(k_band_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
-  SX_CUDA(cudaFuncSetAttribute(k_band_sweep, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  for (SweepKernel k : {(SweepKernel)k_band_sweep<false>, (SweepKernel)k_band_sweep<true>}) {
+    SX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+    SX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  }
   return SX_OK;
 }
 
@@ -638,12 +718,12 @@ int default_lead(int C, int) {
 }
 
 // Clusters of C CTAs (ring of S tiles) that can be resident at once.
-static int resident_clusters(int C, int S, int Wmax) {
+static int resident_clusters(int C, int S, int J) {
   if (S < 1) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
   cfg.blockDim = dim3(SWP_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = sweep_smem(C, S, Wmax);
+  cfg.dynamicSmemBytes = sweep_smem(C, S, J, window_blocks(J));
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C;
@@ -652,7 +732,7 @@ static int resident_clusters(int C, int S, int Wmax) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_band_sweep, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, sweep_kernel(J), &cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -660,8 +740,7 @@ static int resident_clusters(int C, int S, int Wmax) {
 }
 
 int band_active_clusters(int C, int J, int smax) {
-  const int W = window_blocks(J);
-  return resident_clusters(C, fit_stages(C, smax, W), W);
+  return resident_clusters(C, fit_stages(C, smax, J, window_blocks(J)), J);
 }
 
 // Cluster size C <= cmax and ring depth for nj systems of J tiles a block
