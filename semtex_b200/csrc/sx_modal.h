@@ -92,6 +92,9 @@ struct sx_modal_s {
   ~sx_modal_s();
 };
 
+// Parallel branches of a batch's captured direct solve, at most.
+constexpr int BATCH_BRANCHES = 16;
+
 // A multi-mesh batch (sx_batch_solve): the mixed-precision tables and
 // graphs, and the direct solve whose band sweeps cover every member.
 struct sx_batch_s {
@@ -107,6 +110,9 @@ struct sx_batch_s {
                                 // changes from batch to batch, enqueues directly)
   cudaStream_t own = nullptr, aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  std::vector<cudaStream_t> branch;    // the direct graph's parallel branches, used while it is captured
+  std::vector<cudaEvent_t> branch_ev;  // their fork, and a join each
+  int reserve_branches(size_t n);
   ~sx_batch_s();
 };
 
