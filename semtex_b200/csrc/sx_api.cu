@@ -115,7 +115,7 @@ int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const Sy
                    cudaStream_t st) {
   // what this call builds: freed in the stream's order if it gives up early
   std::vector<std::shared_ptr<System>> built;
-  std::vector<System *> to_factor;
+  std::vector<System *> direct, to_factor;
   M.sys.clear();
   M.uniq.clear();
   for (int l = 0; l < M.num_modes; l++) {
@@ -148,13 +148,11 @@ int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const Sy
       found->method = kind;
       SX_TRY(device_pool(M.mesh->device, &found->pool));
       built.push_back(found);
-      // enqueued; one wait for all of them below
-      if (kind == SX_DIRECT) {
-        SX_TRY(system_build_direct(*found, st, false));
-        if (found->nsolve > 0) to_factor.push_back(found.get());
-      } else {
+      // enqueued, the DIRECT ones together below; one wait for all of them
+      if (kind == SX_DIRECT)
+        direct.push_back(found.get());
+      else
         SX_TRY(system_build_jacobi(*found, st, false));
-      }
     }
     if (std::find(M.uniq.begin(), M.uniq.end(), found) == M.uniq.end()) M.uniq.push_back(found);
     M.sys.push_back(found);
@@ -163,6 +161,9 @@ int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const Sy
     SX_TRY(M.dstatus.alloc(1));
     SX_TRY(M.dstatus.zero(st));
   }
+  SX_TRY(systems_build_direct(direct, st));
+  for (System *S : direct)
+    if (S->nsolve > 0) to_factor.push_back(S);
   SX_TRY(factor_batch(to_factor, st, false));
   if (!built.empty()) SX_CUDA(cudaStreamSynchronize(st));
   for (auto &S : built) {

@@ -1,7 +1,7 @@
 // sx_factor.cu -- GPU set-up of a DIRECT or JACPCG system (MatrixSys).
 //
 // DIRECT (src/matrix.cpp:175-274):
-//   1. k_elem_condense: one CTA per element builds the elemental Helmholtz
+//   1. k_elem_condense: one CTA per element and system builds the elemental Helmholtz
 //      matrix in edge-major order (Element::HelmholtzRow,
 //      src/element.cpp:1439-1509), inverts the interior block (the reference
 //      uses getrf+getri, src/element.cpp:212-216; hii is SPD here so
@@ -35,28 +35,47 @@ namespace sx {
 // Element matrix + static condensation
 // ---------------------------------------------------------------------------
 
-// smem (doubles): D nn | Q1..Q4 4nn | hbb next^2 | hbi next*nint | hii nint^2 |
-// t next*nint | colk nint ; ints: emap nn
-static size_t condense_smem_np(int np) {
-  const size_t nn = (size_t)np * np, ne = 4 * (size_t)(np - 1), ni = nn - ne;
-  return sizeof(double) * (5 * nn + ne * ne + 2 * ne * ni + ni * ni + ni) + sizeof(int) * nn + 16;
-}
-static size_t condense_smem(const MeshView &M) { return condense_smem_np(M.np); }
+// One system of a batched build: every launch covers all of them (blockIdx.y).
+struct BuildDesc {
+  double hCon;
+  double *hbi, *hii, *hbb, *tiles;
+  int *status;
+  int nsolve, nblk, J;
+};
 
-__global__ void k_elem_condense(MeshView M, double hCon, double *__restrict__ hbi_out,
-                                double *__restrict__ hii_out, double *__restrict__ hbb_out,
-                                int *status) {
+// Shared rows are PI doubles apart (odd: row and column walks are free of bank
+// conflicts).
+template <int NP>
+struct Condense {
+  static constexpr int NN = NP * NP, NE = 4 * (NP - 1), NI = NN - NE, PI = NI | 1;
+  static constexpr int AE = (NE + 15) / 16, AI = (NI + 15) / 16;  // rows of a thread: ty, ty + 16, ...
+  static constexpr int WORK = 5 * NN > NI * PI ? 5 * NN : NI * PI;
+  // hbi | t | D, Q1..Q4 and later hii | pivot row and column, two buffers each
+  static constexpr size_t smem = sizeof(double) * (2 * (size_t)NE * PI + WORK + 4 * 16 * AI);
+  static constexpr int blocks = NP <= 8 ? 4 : NP <= 11 ? 2 : 1;  // an SM: shared memory and registers
+};
+
+// The element's matrix and its condensation, one block of 16 x 16 threads per
+// (element, system).  Thread (ty, tx) keeps the entries (ty + 16 a, tx + 16 b)
+// of hii and of hbb in registers: the Gauss-Jordan steps exchange the pivot row
+// and column through shared memory (one barrier a step, two buffers), and the
+// two products that follow reuse each value they read AE or AI times.  What
+// bounded the form before this (entries in shared memory, an index division and
+// four shared-memory accesses per entry and step) was instruction issue: ten
+// systems of 851 elements of order 7, 1.52 ms in ten launches -> 0.56 ms in one.
+template <int NP>
+__global__ void __launch_bounds__(256, Condense<NP>::blocks)
+    k_elem_condense(MeshView M, const BuildDesc *__restrict__ desc) {
+  using C = Condense<NP>;
+  constexpr int NN = C::NN, NE = C::NE, NI = C::NI, PI = C::PI, AE = C::AE, AI = C::AI;
+  const BuildDesc B = desc[blockIdx.y];
   extern __shared__ double sm[];
-  const int np = M.np, nn = M.npnp, next = M.next, nint = M.nint;
-  const int e = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
-  double *D = sm, *Q1 = D + nn, *Q2 = Q1 + nn, *Q3 = Q2 + nn, *Q4 = Q3 + nn;
-  double *hbb = Q4 + nn, *hbi = hbb + next * next, *hii = hbi + next * nint;
-  double *t = hii + nint * nint, *colk = t + next * nint;
-  int *emap = (int *)(colk + nint);
-  __shared__ int bad;
-  if (tid == 0) bad = 0;
-  const size_t eo = (size_t)e * nn;
-  for (int i = tid; i < nn; i += nt) {
+  double *hbi = sm, *t = hbi + NE * PI, *hii = t + NE * PI, *rowb = hii + C::WORK, *colb = rowb + 2 * 16 * AI;
+  double *D = hii, *Q1 = D + NN, *Q2 = Q1 + NN, *Q3 = Q2 + NN, *Q4 = Q3 + NN;  // until the inverse is there
+  __shared__ int emap[NN];
+  const int e = blockIdx.x, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const size_t eo = (size_t)e * NN;
+  for (int i = tid; i < NN; i += 256) {
     D[i] = M.D[i];
     Q1[i] = M.Q1[eo + i];
     Q2[i] = M.Q2[eo + i];
@@ -66,123 +85,190 @@ __global__ void k_elem_condense(MeshView M, double hCon, double *__restrict__ hb
   }
   __syncthreads();
   const bool q3 = M.hasQ3[e];
-  // Entry H[(i,j),(m,n)] of the elemental matrix, accumulated in the order
-  // of HelmholtzRow: Q1 term, Q2 term, the two Q3 terms, then Q4*hCon.
-  for (int idx = tid; idx < nn * nn; idx += nt) {
-    const int a = idx / nn, b = idx - a * nn;
-    if (a >= next && b < next) continue;
+  // Entry H[(i,j),(m,n)] of the elemental matrix in edge-major order,
+  // accumulated in the order of HelmholtzRow: Q1 term, Q2 term, the two Q3
+  // terms, then Q4*hCon.
+  auto entry = [&](int a, int b) {
     const int r = emap[a], c = emap[b];
-    const int i = r / np, j = r - i * np, m = c / np, n = c - m * np;
+    const int i = r / NP, j = r - i * NP, m = c / NP, n = c - m * NP;
     double h = 0.0;
     if (m == i) {
       double s = 0.0;
-      for (int q = 0; q < np; q++) s += Q1[i * np + q] * (D[q * np + j] * D[q * np + n]);
+#pragma unroll
+      for (int q = 0; q < NP; q++) s += Q1[i * NP + q] * (D[q * NP + j] * D[q * NP + n]);
       h = s;
     }
     if (n == j) {
       double s = 0.0;
-      for (int p = 0; p < np; p++) s += Q2[p * np + j] * (D[p * np + i] * D[p * np + m]);
+#pragma unroll
+      for (int p = 0; p < NP; p++) s += Q2[p * NP + j] * (D[p * NP + i] * D[p * NP + m]);
       h += s;
     }
     if (q3) {
-      h += Q3[i * np + n] * D[n * np + j] * D[i * np + m];
-      h += Q3[m * np + j] * D[j * np + n] * D[m * np + i];
+      h += Q3[i * NP + n] * D[n * NP + j] * D[i * NP + m];
+      h += Q3[m * NP + j] * D[j * NP + n] * D[m * NP + i];
     }
-    if (m == i && n == j) h += Q4[i * np + j] * hCon;
-    if (a < next) {
-      if (b < next)
-        hbb[a * next + b] = h;
-      else
-        hbi[a * nint + (b - next)] = h;
-    } else {
-      hii[(a - next) * nint + (b - next)] = h;
+    if (m == i && n == j) h += Q4[i * NP + j] * B.hCon;
+    return h;
+  };
+  double hb[AE][AE], v[AI][AI];
+#pragma unroll
+  for (int a = 0; a < AE; a++) {
+    const int r = ty + 16 * a;
+#pragma unroll
+    for (int b = 0; b < AE; b++) hb[a][b] = r < NE && tx + 16 * b < NE ? entry(r, tx + 16 * b) : 0.0;
+#pragma unroll
+    for (int b = 0; b < AI; b++) {
+      const int c = tx + 16 * b;
+      if (r < NE && c < NI) hbi[r * PI + c] = entry(r, NE + c);
     }
   }
-  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < AI; a++)
+#pragma unroll
+    for (int b = 0; b < AI; b++)
+      v[a][b] = ty + 16 * a < NI && tx + 16 * b < NI ? entry(NE + ty + 16 * a, NE + tx + 16 * b) : 0.0;
   // In-place Gauss-Jordan inverse of the SPD interior block.
-  for (int k = 0; k < nint; k++) {
-    const double p = hii[k * nint + k];
-    for (int i = tid; i < nint; i += nt) colk[i] = hii[i * nint + k];
-    // a zero (or NaN) pivot: hii is singular (src/element.cpp:212-216); a
-    // negative one: hii, a principal block of H, is not positive definite,
-    // so neither is H -- the reference's getrf/getri go on with an
-    // indefinite hii and its dpbtrf then fails (src/matrix.cpp:259-261)
-    if (tid == 0) bad |= (p < 0.0) ? 2 : (!(p > 0.0) ? 1 : 0);
-    __syncthreads();
-    const double rp = (p != 0.0 && p == p) ? 1.0 / p : 1.0;
-    for (int j = tid; j < nint; j += nt) hii[k * nint + j] = ((j == k) ? 1.0 : hii[k * nint + j]) * rp;
-    __syncthreads();
-    for (int idx = tid; idx < nint * nint; idx += nt) {
-      const int i = idx / nint, j = idx - i * nint;
-      if (i == k) continue;
-      const double v = (j == k) ? 0.0 : hii[idx];
-      hii[idx] = v - colk[i] * hii[k * nint + j];
+  int bad = 0;
+#pragma unroll
+  for (int ka = 0; ka < AI; ka++) {
+    for (int kk = 0; kk < 16; kk++) {
+      const int k = 16 * ka + kk;
+      if (k >= NI) break;
+      double *rk = rowb + (k & 1) * 16 * AI, *ck = colb + (k & 1) * 16 * AI;
+      if (ty == kk)
+#pragma unroll
+        for (int b = 0; b < AI; b++) rk[tx + 16 * b] = v[ka][b];
+      if (tx == kk)
+#pragma unroll
+        for (int a = 0; a < AI; a++) ck[ty + 16 * a] = v[a][ka];
+      __syncthreads();
+      const double p = rk[k];
+      // a zero (or NaN) pivot: hii is singular (src/element.cpp:212-216); a
+      // negative one: hii, a principal block of H, is not positive definite,
+      // so neither is H -- the reference's getrf/getri go on with an
+      // indefinite hii and its dpbtrf then fails (src/matrix.cpp:259-261)
+      bad |= (p < 0.0) ? 2 : (!(p > 0.0) ? 1 : 0);
+      const double rp = (p != 0.0 && p == p) ? 1.0 / p : 1.0;
+      double x[AI], y[AI];
+#pragma unroll
+      for (int b = 0; b < AI; b++) x[b] = (tx + 16 * b == k ? 1.0 : rk[tx + 16 * b]) * rp;
+#pragma unroll
+      for (int a = 0; a < AI; a++) y[a] = ck[ty + 16 * a];
+#pragma unroll
+      for (int a = 0; a < AI; a++)
+#pragma unroll
+        for (int b = 0; b < AI; b++)
+          v[a][b] = ty + 16 * a == k ? x[b] : (tx + 16 * b == k ? 0.0 : v[a][b]) - y[a] * x[b];
     }
-    __syncthreads();
   }
-  // t = hbi * hii^-1 ; hbb -= t * hbi^T
-  for (int idx = tid; idx < next * nint; idx += nt) {
-    const int b = idx / nint, c = idx - b * nint;
-    double s = 0.0;
-    for (int q = 0; q < nint; q++) s += hbi[b * nint + q] * hii[q * nint + c];
-    t[idx] = s;
+  // every thread is past its reads of D and Q (the barriers above; NI >= 1)
+#pragma unroll
+  for (int a = 0; a < AI; a++)
+#pragma unroll
+    for (int b = 0; b < AI; b++)
+      if (ty + 16 * a < NI && tx + 16 * b < NI) hii[(ty + 16 * a) * PI + tx + 16 * b] = v[a][b];
+  __syncthreads();
+  // t = hbi * hii^-1
+  {
+    double s[AE][AI];
+#pragma unroll
+    for (int a = 0; a < AE; a++)
+#pragma unroll
+      for (int b = 0; b < AI; b++) s[a][b] = 0.0;
+    for (int q = 0; q < NI; q++) {
+      double x[AE], y[AI];
+#pragma unroll
+      for (int a = 0; a < AE; a++) x[a] = hbi[min(ty + 16 * a, NE - 1) * PI + q];
+#pragma unroll
+      for (int b = 0; b < AI; b++) y[b] = hii[q * PI + min(tx + 16 * b, NI - 1)];
+#pragma unroll
+      for (int a = 0; a < AE; a++)
+#pragma unroll
+        for (int b = 0; b < AI; b++) s[a][b] += x[a] * y[b];
+    }
+#pragma unroll
+    for (int a = 0; a < AE; a++)
+#pragma unroll
+      for (int b = 0; b < AI; b++)
+        if (ty + 16 * a < NE && tx + 16 * b < NI) t[(ty + 16 * a) * PI + tx + 16 * b] = s[a][b];
   }
   __syncthreads();
-  for (int idx = tid; idx < next * next; idx += nt) {
-    const int b = idx / next, b2 = idx - b * next;
-    double s = 0.0;
-    for (int q = 0; q < nint; q++) s += t[b * nint + q] * hbi[b2 * nint + q];
-    hbb[idx] -= s;
+  // hbb -= t * hbi^T
+  double *oh = B.hbb + (size_t)e * NE * NE;
+  {
+    double s[AE][AE];
+#pragma unroll
+    for (int a = 0; a < AE; a++)
+#pragma unroll
+      for (int b = 0; b < AE; b++) s[a][b] = 0.0;
+    for (int q = 0; q < NI; q++) {
+      double x[AE], y[AE];
+#pragma unroll
+      for (int a = 0; a < AE; a++) {
+        x[a] = t[min(ty + 16 * a, NE - 1) * PI + q];
+        y[a] = hbi[min(tx + 16 * a, NE - 1) * PI + q];
+      }
+#pragma unroll
+      for (int a = 0; a < AE; a++)
+#pragma unroll
+        for (int b = 0; b < AE; b++) s[a][b] += x[a] * y[b];
+    }
+#pragma unroll
+    for (int a = 0; a < AE; a++)
+#pragma unroll
+      for (int b = 0; b < AE; b++) {
+        const int r = ty + 16 * a, c = tx + 16 * b;
+        if (r < NE && c < NE) oh[r * NE + c] = hb[a][b] - s[a][b];
+      }
   }
-  __syncthreads();
-  double *ob = hbi_out + (size_t)e * next * nint;
-  for (int i = tid; i < next * nint; i += nt) ob[i] = t[i];
-  double *oi = hii_out + (size_t)e * nint * nint;
+  double *ob = B.hbi + (size_t)e * NE * NI;
+  for (int o = tid; o < NE * NI; o += 256) ob[o] = t[(o / NI) * PI + o % NI];
+  double *oi = B.hii + (size_t)e * NI * NI;
   // column-major, (r, c) at c * nint + r: the back-substitution's threads
   // own rows and read a column per step
-  for (int o = tid; o < nint * nint; o += nt) {
-    const int c = o / nint, r = o - c * nint;
-    oi[o] = hii[r * nint + c];
-  }
-  double *oh = hbb_out + (size_t)e * next * next;
-  for (int i = tid; i < next * next; i += nt) oh[i] = hbb[i];
+  for (int o = tid; o < NI * NI; o += 256) oi[o] = hii[(o % NI) * PI + o / NI];
   if (tid == 0 && bad)
-    atomicOr(status, ((bad & 1) ? 1 << SX_ERR_SINGULAR_HII : 0) | ((bad & 2) ? 1 << SX_ERR_NOT_SPD : 0));
+    atomicOr(B.status, ((bad & 1) ? 1 << SX_ERR_SINGULAR_HII : 0) | ((bad & 2) ? 1 << SX_ERR_NOT_SPD : 0));
 }
 
 // ---------------------------------------------------------------------------
 // Band assembly into tiles
 // ---------------------------------------------------------------------------
 
-__global__ void k_band_identity_pad(double *tiles, int J, int nsolve, int nblk) {
-  const int g = nsolve + blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= nblk * NB) return;
+// Identity rows past the last solve node (fewer than NB), and the status word.
+__global__ void k_band_init(const BuildDesc *__restrict__ desc) {
+  const BuildDesc B = desc[blockIdx.y];
+  if (threadIdx.x == 0) *B.status = 0;
+  const int g = B.nsolve + threadIdx.x;
+  if (g >= B.nblk * NB) return;
   const int b = g / NB, r = g - b * NB;
-  tiles[((size_t)b * (J + 1)) * TSZ + (size_t)r * LDT + r] = 1.0;
+  B.tiles[((size_t)b * (B.J + 1)) * TSZ + (size_t)r * LDT + r] = 1.0;
 }
 
-__global__ void k_band_add(MeshView M, const int *__restrict__ elems, const double *__restrict__ hbb,
-                           double *tiles, int J, int nsolve, int *status) {
+__global__ void k_band_add(MeshView M, const int *__restrict__ elems, const BuildDesc *__restrict__ desc) {
+  const BuildDesc B = desc[blockIdx.y];
   const int e = elems[blockIdx.x];
   const int next = M.next, kd = M.nband - 1;
   const int *bt = M.btog + (size_t)e * next;
-  const double *h = hbb + (size_t)e * next * next;
+  const double *h = B.hbb + (size_t)e * next * next;
   for (int idx = threadIdx.x; idx < next * next; idx += blockDim.x) {
     const int i = idx / next, k = idx - i * next;
     const int m = bt[i], n = bt[k];
-    if (m < nsolve && n < nsolve && n >= m) {
+    if (m < B.nsolve && n < B.nsolve && n >= m) {
       if (n - m > kd) {
-        atomicOr(status, 1 << SX_ERR_BAND);
+        atomicOr(B.status, 1 << SX_ERR_BAND);
         continue;
       }
-      tiles[tile_addr(m, n, J)] += h[idx];
+      B.tiles[tile_addr(m, n, B.J)] += h[idx];
     }
   }
 }
 
 // Mixed::augmentSC in boundary order (one thread: tiny, order-preserving).
-__global__ void k_band_mixed(MeshView M, double *tiles, int J, int nsolve) {
-  if (threadIdx.x || blockIdx.x) return;
+__global__ void k_band_mixed(MeshView M, const BuildDesc *__restrict__ desc) {
+  if (threadIdx.x) return;
+  const BuildDesc B = desc[blockIdx.y];
   const int np = M.np, nm = np - 1;
   for (int b = 0; b < M.nbound; b++) {
     if (M.b_kind[b] != SX_BC_MIXED) continue;
@@ -192,10 +278,10 @@ __global__ void k_band_mixed(MeshView M, double *tiles, int J, int nsolve) {
     const double *area = M.b_area + (size_t)b * np;
     for (int i = 0; i < nm; i++) {
       const int k = bmap[side * nm + i];
-      if (k < nsolve) tiles[tile_addr(k, k, J)] += K * area[i];
+      if (k < B.nsolve) B.tiles[tile_addr(k, k, B.J)] += K * area[i];
     }
     const int i = (side == 3) ? bmap[0] : bmap[side * nm + nm];
-    if (i < nsolve) tiles[tile_addr(i, i, J)] += K * area[nm];
+    if (i < B.nsolve) B.tiles[tile_addr(i, i, B.J)] += K * area[nm];
   }
 }
 
@@ -608,51 +694,92 @@ int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync, boo
   return SX_OK;
 }
 
-int system_build_direct(System &S, cudaStream_t st, bool sync) {
-  sx_mesh_s &Mh = *S.mesh;
-  const MeshView M = Mh.view();
-  const double hCon = S.betak2 + S.lambda2;
+template <int NP>
+static int launch_condense(const MeshView &M, const BuildDesc *d, int ns, cudaStream_t st) {
+  // the kernel's shared-memory limit is a per-function setting, the same for
+  // every caller of this order
+  SX_CUDA(cudaFuncSetAttribute(k_elem_condense<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)Condense<NP>::smem));
+  k_elem_condense<NP><<<dim3(M.nel, ns), 256, Condense<NP>::smem, st>>>(M, d);
+  SX_CUDA(cudaGetLastError());
+  return SX_OK;
+}
+
+static int condense(const MeshView &M, const BuildDesc *d, int ns, cudaStream_t st) {
+  switch (M.np) {
+#define SX_CASE(n) \
+  case n: return launch_condense<n>(M, d, ns, st);
+    SX_CASE(3) SX_CASE(4) SX_CASE(5) SX_CASE(6) SX_CASE(7) SX_CASE(8) SX_CASE(9) SX_CASE(10)
+    SX_CASE(11) SX_CASE(12)
+#undef SX_CASE
+    default: return SX_ERR_UNSUPPORTED;
+  }
+}
+
+// The temporary condensed matrices of the systems built together are kept
+// below this many bytes (64 systems of a large mesh would take several GB), or
+// to one system's where not even that is free.
+constexpr size_t BUILD_TEMP = size_t(1) << 30;
+
+// Sizes, and the memory that stays.
+static int system_reserve_direct(System &S, cudaStream_t st) {
+  const sx_mesh_s &Mh = *S.mesh;
   S.singular = (S.lambda2 + S.betak2) < EPSSP && (Mh.nglobal - Mh.nsolve) == 0 && !Mh.mixed;
   S.nsolve = S.singular ? Mh.nsolve - 1 : Mh.nsolve;
-  const int kd = Mh.nband - 1;
   S.nblk = (S.nsolve + NB - 1) / NB;
-  S.J = (kd + NB - 1) / NB;
+  S.J = (Mh.nband - 1 + NB - 1) / NB;
   if (S.status.p == nullptr) SX_TRY(S.status.alloc_in(1, S.pool, st));
-  SX_TRY(S.status.zero(st));
   SX_TRY(S.hbi.alloc_in((size_t)Mh.nel * Mh.next * Mh.nint, S.pool, st));
   SX_TRY(S.hii.alloc_in((size_t)Mh.nel * Mh.nint * Mh.nint, S.pool, st));
-  DBuf<double> hbb;
-  SX_TRY(hbb.alloc_in((size_t)Mh.nel * Mh.next * Mh.next, S.pool, st, true));
-  const size_t smem = condense_smem(M);
-  // the kernel's shared-memory limit is a per-function setting: set it once,
-  // for the largest order, so that builds of different orders on other host
-  // threads never lower it under this launch
-  static std::once_flag attr_once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(attr_once, []() {
-    attr_err = cudaFuncSetAttribute(k_elem_condense, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)condense_smem_np(NP_MAX));
-  });
-  SX_CUDA(attr_err);
-  k_elem_condense<<<Mh.nel, 256, smem, st>>>(M, hCon, S.hbi.p, S.hii.p, hbb.p, S.status.p);
-  SX_CUDA(cudaGetLastError());
-  const size_t ntiles = (size_t)std::max(S.nblk, 1) * (S.J + 1);
-  SX_TRY(S.tiles.alloc_in(ntiles * TSZ, S.pool, st));
+  const size_t nb = (size_t)std::max(S.nblk, 1);
+  SX_TRY(S.tiles.alloc_in(nb * (S.J + 1) * TSZ, S.pool, st));
   SX_TRY(S.tiles.zero(st));
-  SX_TRY(S.dinv.alloc_in((size_t)std::max(S.nblk, 1) * TSZ, S.pool, st));
-  SX_TRY(S.dinv.zero(st));
-  if (S.nsolve > 0) {
-    const int npad = S.nblk * NB - S.nsolve;
-    if (npad > 0) k_band_identity_pad<<<(npad + 127) / 128, 128, 0, st>>>(S.tiles.p, S.J, S.nsolve, S.nblk);
+  return S.dinv.alloc_in(nb * TSZ, S.pool, st);  // k_potrf writes every block's tile in full
+}
+
+int systems_build_direct(const std::vector<System *> &systems, cudaStream_t st) {
+  for (System *S : systems) SX_TRY(system_reserve_direct(*S, st));
+  for (size_t s0 = 0, s1; s0 < systems.size(); s0 = s1) {
+    sx_mesh_s &Mh = *systems[s0]->mesh;
+    const MeshView M = Mh.view();
+    const size_t nh = (size_t)Mh.nel * Mh.next * Mh.next;
+    const size_t most = std::max<size_t>(1, BUILD_TEMP / (nh * 8));
+    s1 = s0;
+    while (s1 < systems.size() && s1 - s0 < most && systems[s1]->mesh == &Mh) s1++;
+    DBuf<double> hbb;
+    int rc = hbb.alloc_in(nh * (s1 - s0), systems[s0]->pool, st, true);
+    if (rc == SX_ERR_NOMEM && s1 - s0 > 1) {
+      s1 = s0 + 1;
+      rc = hbb.alloc_in(nh, systems[s0]->pool, st, true);
+    }
+    SX_TRY(rc);
+    const int ns = (int)(s1 - s0);
+    std::vector<BuildDesc> hd(ns);
+    bool any = false;
+    for (int i = 0; i < ns; i++) {
+      System &S = *systems[s0 + i];
+      any |= S.nsolve > 0;
+      hd[i] = BuildDesc{S.betak2 + S.lambda2, S.hbi.p, S.hii.p,  hbb.p + nh * i, S.tiles.p,
+                        S.status.p,           S.nsolve, S.nblk, S.J};
+    }
+    DBuf<BuildDesc> dd;
+    SX_TRY(dd.upload_on(hd.data(), hd.size(), st));
+    k_band_init<<<dim3(1, ns), NB, 0, st>>>(dd.p);
+    SX_TRY(condense(M, dd.p, ns, st));
+    if (!any) continue;
     for (size_t c = 0; c + 1 < Mh.colour_ptr.size(); c++) {
       const int n = Mh.colour_ptr[c + 1] - Mh.colour_ptr[c];
-      if (n > 0)
-        k_band_add<<<n, 256, 0, st>>>(M, Mh.dcolour_elmt.p + Mh.colour_ptr[c], hbb.p, S.tiles.p, S.J,
-                                      S.nsolve, S.status.p);
+      if (n > 0) k_band_add<<<dim3(n, ns), 256, 0, st>>>(M, Mh.dcolour_elmt.p + Mh.colour_ptr[c], dd.p);
     }
-    if (Mh.mixed) k_band_mixed<<<1, 1, 0, st>>>(M, S.tiles.p, S.J, S.nsolve);
+    if (Mh.mixed) k_band_mixed<<<dim3(1, ns), 32, 0, st>>>(M, dd.p);
     SX_CUDA(cudaGetLastError());
   }
+  return SX_OK;
+}
+
+int system_build_direct(System &S, cudaStream_t st, bool sync) {
+  const std::vector<System *> one(1, &S);
+  SX_TRY(systems_build_direct(one, st));
   if (!sync) return SX_OK;
   SX_CUDA(cudaStreamSynchronize(st));
   SX_TRY(check_status(S.status));

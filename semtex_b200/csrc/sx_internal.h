@@ -282,6 +282,8 @@ struct System {
 // caller synchronises st (or records an event) and then calls
 // system_check_status.
 int system_build_direct(System &S, cudaStream_t st, bool sync = true);
+// Several systems, each launch over all that share a mesh; enqueued only.
+int systems_build_direct(const std::vector<System *> &systems, cudaStream_t st);
 int system_build_jacobi(System &S, cudaStream_t st, bool sync = true);
 int system_build_jacobi_diag(System &S, cudaStream_t st, bool sync = true);
 int system_check_status(System &S);

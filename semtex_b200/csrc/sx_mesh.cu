@@ -321,6 +321,7 @@ int sx::device_pool(int device, cudaMemPool_t *out) {
 void sx::device_pool_trim() {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) return;
+  cudaDeviceSynchronize();  // what was freed in stream order becomes idle
   std::lock_guard<std::mutex> lk(pool_mu);
   auto it = pools.find(dev);
   if (it != pools.end()) cudaMemPoolTrimTo(it->second, 0);
