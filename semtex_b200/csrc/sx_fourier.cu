@@ -11,8 +11,9 @@
 //   inverse (sign = -1): x_j = X_0 + (-1)^j X_{nz/2} + 2 sum_{k=1}^{nz/2-1}
 //     Re(X_k exp(+2 pi i j k / nz)), unscaled, so that inverse(forward(x))
 //     = x.
-// Lengths 2, 4, ..., 64 (config 2 uses 64): one pass, k_z_fwd / k_z_inv;
-// 128, 256, 512: one pass through shared memory, k_z_fwd_s / k_z_inv_s.
+// Lengths 2, 4, ..., 64 (config 2 uses 64): one pass, k_z_fwd / k_z_inv; the
+// other lengths up to 512: one pass through shared memory, k_z_fwd_any /
+// k_z_inv_any (256: k_z_fwd_s / k_z_inv_s).
 // A thread holds one point's whole z-line in registers: the real transform
 // of length N is a complex FFT of length M = N/2 on z_m = x_2m + i x_2m+1
 // (radix-2, decimation in time, every index a compile-time constant), then
@@ -87,7 +88,7 @@ bool factors_235(int n) {
 
 // exp(-2 pi i t / TWN), t = 0 .. TWN/2, from the host's cos / sin in FP64;
 // a length-L stage uses t = j * (TWN / L).
-constexpr int TWN = 512;
+constexpr int TWN = 256;
 __constant__ double c_twr[TWN / 2 + 1], c_twi[TWN / 2 + 1];
 
 static int ensure_twiddles() {
@@ -227,8 +228,7 @@ __global__ void __launch_bounds__(128) k_z_inv(double *__restrict__ data, int np
   }
 }
 
-// Lengths 128, 256, 512: a block of eight warps takes 32 points (lane =
-// point); the half-length complex sequence z (length M = N/2) of each point
+// Length 256: a block of eight warps takes 32 points (lane = point); the half-length complex sequence z (length M = N/2) of each point
 // lies in shared memory, Zr/Zi[m][32], in natural order.  The complex FFT
 // of length M = M1 M2 runs in four steps with m = M2 m1 + m2 and
 // k = k1 + M1 k2: (1) the M2 FFTs of length M1 over m1, each a warp's, in
@@ -404,6 +404,474 @@ static int launch_smem(double *d, int npts, long long stride, int sign, cudaStre
   return SX_OK;
 }
 
+// ---------------------------------------------------------------------------
+// every other even length up to ZN_MAX with prime factors 2, 3, 5
+// ---------------------------------------------------------------------------
+//
+// The complex FFT of length M = N / 2 of 32 points (lane = point) in two or
+// three in-place stages over shared memory, Zr/Zi[row][32] (the decimation in
+// frequency of Gentleman & Sande 1966, mixed radix): a stage of radix R over
+// sub-sequences of length n = R L takes rows j, j + L, ... of a sub-sequence
+// into registers, a warp each, transforms them, multiplies output k by
+// W_n^(j k) and puts it back at row j + k L; the next stage works on the R
+// sub-sequences of length L.  X_K ends at the row whose mixed-radix digits are
+// K's, reversed.
+//   What bounds it is HBM (a field is read and written once), so the stages
+// next to global memory skip the shared-memory trip: forward, the first stage
+// reads its rows from the planes; inverse, the last one writes its outputs to
+// them.  The real-to-complex split needs rows k and M - k together and stays
+// on the shared-memory side.  A block holds PG groups of 32 points, so that a
+// short M still gives every warp a sub-transform.
+//   Measured (forward / inverse, L2 flushed; before: cuFFT's batched transform
+// into a workspace and a packing pass, or for 128 and 512 one radix-2 four-step
+// kernel pair with a load and a store pass of its own): 24 x 495,616 points
+// 98/99 -> 50/60 us, 96 x 82,944 75/73 -> 44/46, 120 x 82,944 86/88 -> 54/58,
+// 128 x 495,616 261/283 -> 241/276, 240 x 82,944 185/201 -> 110/124,
+// 512 x 82,944 290/375 -> 220/321.
+constexpr int ZN_MAX = 512, ZST = 5;
+
+// exp(-2 pi i t / N), t = 0 .. N / 2, and the stages: a kernel parameter, so
+// that warp-uniform reads are constant-cache broadcasts and nothing is kept
+// on the device between calls.
+struct ZPlan235 {
+  double c[ZN_MAX / 2 + 1], s[ZN_MAX / 2 + 1];
+  int N, M, PG, nst, radix[ZST];
+};
+
+// W_N^t (conjugated for the inverse), 0 <= t < N.
+template <bool INV>
+__device__ __forceinline__ void zw(const ZPlan235 &Z, int t, double &wr, double &wi) {
+  const int h = Z.M;
+  const bool neg = t >= h;
+  const int i = neg ? t - h : t;
+  wr = neg ? -Z.c[i] : Z.c[i];
+  wi = (neg != INV) ? -Z.s[i] : Z.s[i];
+}
+
+// DFT of length R in registers, natural order in and out, unscaled.
+template <int R, bool INV>
+struct Dft;
+template <bool INV>
+struct Dft<2, INV> {
+  static __device__ __forceinline__ void run(const ZPlan235 &, double (&re)[2], double (&im)[2]) {
+    const double ar = re[0], ai = im[0];
+    re[0] += re[1];
+    im[0] += im[1];
+    re[1] = ar - re[1];
+    im[1] = ai - im[1];
+  }
+};
+template <bool INV>
+struct Dft<4, INV> {
+  static __device__ __forceinline__ void run(const ZPlan235 &, double (&re)[4], double (&im)[4]) {
+    const double ar = re[0] + re[2], ai = im[0] + im[2], br = re[0] - re[2], bi = im[0] - im[2];
+    const double cr = re[1] + re[3], ci = im[1] + im[3];
+    const double dr = INV ? im[3] - im[1] : im[1] - im[3];  // -+ i (x1 - x3)
+    const double di = INV ? re[1] - re[3] : re[3] - re[1];
+    re[0] = ar + cr;
+    im[0] = ai + ci;
+    re[1] = br + dr;
+    im[1] = bi + di;
+    re[2] = ar - cr;
+    im[2] = ai - ci;
+    re[3] = br - dr;
+    im[3] = bi - di;
+  }
+};
+template <bool INV>
+struct Dft<8, INV> {
+  static __device__ __forceinline__ void run(const ZPlan235 &Z, double (&re)[8], double (&im)[8]) {
+    constexpr double H = 0.70710678118654752440;  // cos(pi / 4)
+    double er[4] = {re[0], re[2], re[4], re[6]}, ei[4] = {im[0], im[2], im[4], im[6]};
+    double orr[4] = {re[1], re[3], re[5], re[7]}, oi[4] = {im[1], im[3], im[5], im[7]};
+    Dft<4, INV>::run(Z, er, ei);
+    Dft<4, INV>::run(Z, orr, oi);
+    // W_8^k O_k: (1 -+ i) / sqrt 2, -+ i, (-1 -+ i) / sqrt 2
+    const double ar = INV ? H * (orr[1] - oi[1]) : H * (orr[1] + oi[1]);
+    const double ai = INV ? H * (oi[1] + orr[1]) : H * (oi[1] - orr[1]);
+    const double br = INV ? -oi[2] : oi[2], bi = INV ? orr[2] : -orr[2];
+    const double cr = INV ? -H * (orr[3] + oi[3]) : H * (oi[3] - orr[3]);
+    const double ci = INV ? H * (orr[3] - oi[3]) : -H * (orr[3] + oi[3]);
+    orr[1] = ar;
+    oi[1] = ai;
+    orr[2] = br;
+    oi[2] = bi;
+    orr[3] = cr;
+    oi[3] = ci;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      re[k] = er[k] + orr[k];
+      im[k] = ei[k] + oi[k];
+      re[k + 4] = er[k] - orr[k];
+      im[k + 4] = ei[k] - oi[k];
+    }
+  }
+};
+template <bool INV>
+struct Dft<3, INV> {
+  static __device__ __forceinline__ void run(const ZPlan235 &, double (&re)[3], double (&im)[3]) {
+    constexpr double S = INV ? 0.86602540378443864676 : -0.86602540378443864676;  // -+ sin(2 pi / 3)
+    const double tr = re[1] + re[2], ti = im[1] + im[2], dr = S * (re[1] - re[2]), di = S * (im[1] - im[2]);
+    const double mr = re[0] - 0.5 * tr, mi = im[0] - 0.5 * ti;
+    re[0] += tr;
+    im[0] += ti;
+    re[1] = mr - di;
+    im[1] = mi + dr;
+    re[2] = mr + di;
+    im[2] = mi - dr;
+  }
+};
+template <bool INV>
+struct Dft<5, INV> {
+  static __device__ __forceinline__ void run(const ZPlan235 &, double (&re)[5], double (&im)[5]) {
+    constexpr double C1 = 0.30901699437494742410, C2 = -0.80901699437494742410;  // cos(2 pi / 5), cos(4 pi / 5)
+    constexpr double S1 = INV ? 0.95105651629515357212 : -0.95105651629515357212;
+    constexpr double S2 = INV ? 0.58778525229247312917 : -0.58778525229247312917;
+    const double ar = re[1] + re[4], ai = im[1] + im[4], br = re[2] + re[3], bi = im[2] + im[3];
+    const double cr = re[1] - re[4], ci = im[1] - im[4], dr = re[2] - re[3], di = im[2] - im[3];
+    const double pr = re[0] + C1 * ar + C2 * br, pi = im[0] + C1 * ai + C2 * bi;
+    const double qr = re[0] + C2 * ar + C1 * br, qi = im[0] + C2 * ai + C1 * bi;
+    const double ur = S1 * cr + S2 * dr, ui = S1 * ci + S2 * di;
+    const double vr = S2 * cr - S1 * dr, vi = S2 * ci - S1 * di;
+    re[0] += ar + br;
+    im[0] += ai + bi;
+    re[1] = pr - ui;
+    im[1] = pi + ur;
+    re[4] = pr + ui;
+    im[4] = pi - ur;
+    re[2] = qr - vi;
+    im[2] = qi + vr;
+    re[3] = qr + vi;
+    im[3] = qi - vr;
+  }
+};
+// R = A B: A-point transforms of every B-th value, twiddles, B-point ones.
+template <int A, int B, bool INV>
+struct DftAB {
+  static constexpr int R = A * B;
+  static __device__ __forceinline__ void run(const ZPlan235 &Z, double (&re)[R], double (&im)[R]) {
+    const int u = Z.N / R;
+#pragma unroll
+    for (int b = 0; b < B; b++) {
+      double x[A], y[A];
+#pragma unroll
+      for (int a = 0; a < A; a++) {
+        x[a] = re[a * B + b];
+        y[a] = im[a * B + b];
+      }
+      Dft<A, INV>::run(Z, x, y);
+#pragma unroll
+      for (int k = 0; k < A; k++) {
+        if (b * k == 0) {
+          re[k * B + b] = x[k];
+          im[k * B + b] = y[k];
+        } else {
+          double wr, wi;
+          zw<INV>(Z, b * k * u, wr, wi);
+          re[k * B + b] = x[k] * wr - y[k] * wi;
+          im[k * B + b] = x[k] * wi + y[k] * wr;
+        }
+      }
+    }
+    double ur[R], ui[R];
+#pragma unroll
+    for (int k = 0; k < A; k++) {
+      double x[B], y[B];
+#pragma unroll
+      for (int b = 0; b < B; b++) {
+        x[b] = re[k * B + b];
+        y[b] = im[k * B + b];
+      }
+      Dft<B, INV>::run(Z, x, y);
+#pragma unroll
+      for (int l = 0; l < B; l++) {
+        ur[k + A * l] = x[l];
+        ui[k + A * l] = y[l];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+      re[q] = ur[q];
+      im[q] = ui[q];
+    }
+  }
+};
+template <bool INV> struct Dft<6, INV> : DftAB<2, 3, INV> {};
+template <bool INV> struct Dft<9, INV> : DftAB<3, 3, INV> {};
+template <bool INV> struct Dft<10, INV> : DftAB<2, 5, INV> {};
+template <bool INV> struct Dft<12, INV> : DftAB<4, 3, INV> {};
+template <bool INV> struct Dft<15, INV> : DftAB<3, 5, INV> {};
+template <bool INV> struct Dft<16, INV> : DftAB<4, 4, INV> {};
+constexpr int Z_RADIX[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+
+// One stage of radix R over sub-sequences of length n: the block's tasks go
+// round its warps.  FROM: the rows come from the planes (forward's first
+// stage); TO: the outputs go to the planes (inverse's last).
+template <int R, bool INV>
+__device__ __forceinline__ void z_stage(const ZPlan235 &Z, double *Zr, double *Zi, int n, bool from, bool to,
+                                        int before, double *data, int npts, long long stride) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int L = n / R, per = Z.M / R, u = Z.N / n;
+  for (int idx = w; idx < Z.PG * per; idx += nw) {
+    const int g = idx / per, o = idx - g * per, sb = o / L, j = o - sb * L;
+    const int p = (blockIdx.x * Z.PG + g) * 32 + lane, row = sb * n + j;
+    const bool ok = p < npts;
+    double *zr = Zr + (size_t)g * Z.M * 32 + lane, *zi = Zi + (size_t)g * Z.M * 32 + lane;
+    double re[R], im[R];
+    if (from) {
+#pragma unroll
+      for (int q = 0; q < R; q++) {
+        const double *d = data + (long long)(2 * (row + q * L)) * stride + p;
+        re[q] = ok ? d[0] : 0.0;
+        im[q] = ok ? d[stride] : 0.0;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < R; q++) {
+        re[q] = zr[(row + q * L) * 32];
+        im[q] = zi[(row + q * L) * 32];
+      }
+    }
+    Dft<R, INV>::run(Z, re, im);
+    if (to) {
+      // L = 1: output k is X_K with K's last digit k and the others sb's,
+      // reversed; z_m = x_2m + i x_2m+1
+      int K = 0, v = sb, weight = before;
+      for (int st = Z.nst - 2; st >= 0; st--) {
+        weight /= Z.radix[st];
+        K += (v % Z.radix[st]) * weight;
+        v /= Z.radix[st];
+      }
+      if (ok) {
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+          double *d = data + (long long)(2 * (K + k * before)) * stride + p;
+          d[0] = 2.0 * re[k];
+          d[stride] = 2.0 * im[k];
+        }
+      }
+      continue;
+    }
+    zr[row * 32] = re[0];
+    zi[row * 32] = im[0];
+#pragma unroll
+    for (int k = 1; k < R; k++) {
+      double wr, wi;
+      zw<INV>(Z, j * k * u, wr, wi);
+      zr[(row + k * L) * 32] = re[k] * wr - im[k] * wi;
+      zi[(row + k * L) * 32] = re[k] * wi + im[k] * wr;
+    }
+  }
+  __syncthreads();
+}
+
+template <int RMAX, bool INV>
+__device__ __forceinline__ void z_stages(const ZPlan235 &Z, double *Zr, double *Zi, double *data, int npts,
+                                         long long stride) {
+  int n = Z.M, before = 1;  // before: the product of the earlier stages' radices
+  for (int st = 0; st < Z.nst; st++) {
+    const int R = Z.radix[st];
+    const bool from = !INV && st == 0, to = INV && st == Z.nst - 1;
+    switch (R) {
+#define SX_ZCASE(r)                                                                                  \
+  case r:                                                                                            \
+    if constexpr (r <= RMAX) z_stage<r, INV>(Z, Zr, Zi, n, from, to, before, data, npts, stride);     \
+    break;
+      SX_ZCASE(2) SX_ZCASE(3) SX_ZCASE(4) SX_ZCASE(5) SX_ZCASE(6) SX_ZCASE(8)
+      SX_ZCASE(9) SX_ZCASE(10) SX_ZCASE(12) SX_ZCASE(15) SX_ZCASE(16)
+#undef SX_ZCASE
+    }
+    n /= R;
+    before *= R;
+  }
+}
+
+// The row of X_K after the stages.
+__device__ __forceinline__ int z_row(const ZPlan235 &Z, int K) {
+  int row = 0, n = Z.M;
+  for (int st = 0; st < Z.nst; st++) {
+    const int R = Z.radix[st];
+    n /= R;
+    row += (K % R) * n;
+    K /= R;
+  }
+  return row;
+}
+
+template <int NT, int MINB, int RMAX>
+__global__ void __launch_bounds__(NT, MINB) k_z_fwd_any(const __grid_constant__ ZPlan235 Z, double *__restrict__ data,
+                                                        int npts, long long stride, double scale) {
+  extern __shared__ __align__(16) double zs[];
+  __shared__ short rowt[ZN_MAX / 2];
+  const int M = Z.M;
+  double *Zr = zs, *Zi = zs + (size_t)Z.PG * M * 32;
+  for (int k = threadIdx.x; k < M; k += NT) rowt[k] = (short)z_row(Z, k);
+  z_stages<RMAX, false>(Z, Zr, Zi, data, npts, stride);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = M / 2 + 1;
+  for (int idx = w; idx < Z.PG * per; idx += NT / 32) {
+    const int g = idx / per, k = idx - g * per, p = (blockIdx.x * Z.PG + g) * 32 + lane;
+    if (p >= npts) continue;
+    const double *zr = Zr + (size_t)g * M * 32 + lane, *zi = Zi + (size_t)g * M * 32 + lane;
+    double *d = data + p;
+    if (k == 0) {
+      const double a = zr[0], b = zi[0];
+      d[0] = (a + b) * scale;
+      d[stride] = (a - b) * scale;
+      continue;
+    }
+    // X_k from Z_k and conj Z_{M-k}; and X_{M-k} from the same pair
+    const int kk = M - k, rk = rowt[k] * 32, rkk = rowt[kk] * 32;
+    const double ar = zr[rk], ai = zi[rk], br = zr[rkk], bi = zi[rkk];
+    const double er = 0.5 * (ar + br), ei = 0.5 * (ai - bi);    // E_k; E_{M-k} is its conjugate
+    const double orr = 0.5 * (ai + bi), oi = -0.5 * (ar - br);  // O_k
+    double wr, wi;
+    zw<false>(Z, k, wr, wi);
+    const double tr = orr * wr - oi * wi, ti = orr * wi + oi * wr;  // W^k O_k
+    d[(2 * k) * stride] = (er + tr) * scale;
+    d[(2 * k + 1) * stride] = (ei + ti) * scale;
+    if (k != kk) {  // X_{M-k} = conj(E_k - W^k O_k)
+      d[(2 * kk) * stride] = (er - tr) * scale;
+      d[(2 * kk + 1) * stride] = (ti - ei) * scale;
+    }
+  }
+}
+
+template <int NT, int MINB, int RMAX>
+__global__ void __launch_bounds__(NT, MINB) k_z_inv_any(const __grid_constant__ ZPlan235 Z, double *__restrict__ data,
+                                                        int npts, long long stride) {
+  extern __shared__ __align__(16) double zs[];
+  const int M = Z.M;
+  double *Zr = zs, *Zi = zs + (size_t)Z.PG * M * 32;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = M / 2 + 1;
+#pragma unroll 2
+  for (int idx = w; idx < Z.PG * per; idx += NT / 32) {
+    const int g = idx / per, k = idx - g * per, p = (blockIdx.x * Z.PG + g) * 32 + lane;
+    const bool ok = p < npts;
+    double *zr = Zr + (size_t)g * M * 32 + lane, *zi = Zi + (size_t)g * M * 32 + lane;
+    const double *d = data + p;
+    if (k == 0) {
+      const double x0 = ok ? d[0] : 0.0, xm = ok ? d[stride] : 0.0;
+      zr[0] = 0.5 * (x0 + xm);
+      zi[0] = 0.5 * (x0 - xm);
+      continue;
+    }
+    // E_k = (X_k + conj X_{M-k}) / 2, O_k = (X_k - conj X_{M-k}) conj(W^k) / 2,
+    // Z_k = E_k + i O_k and Z_{M-k} = conj(E_k) + i conj(O_k)
+    const int kk = M - k;
+    const double ar = ok ? d[(2 * k) * stride] : 0.0, ai = ok ? d[(2 * k + 1) * stride] : 0.0;
+    const double br = ok ? d[(2 * kk) * stride] : 0.0, bi = ok ? d[(2 * kk + 1) * stride] : 0.0;
+    const double er = 0.5 * (ar + br), ei = 0.5 * (ai - bi), dr = 0.5 * (ar - br), di = 0.5 * (ai + bi);
+    double wr, wi;
+    zw<true>(Z, k, wr, wi);
+    const double orr = dr * wr - di * wi, oi = dr * wi + di * wr;
+    zr[k * 32] = er - oi;
+    zi[k * 32] = ei + orr;
+    if (k != kk) {
+      zr[kk * 32] = er + oi;
+      zi[kk * 32] = orr - ei;
+    }
+  }
+  __syncthreads();
+  z_stages<RMAX, true>(Z, Zr, Zi, data, npts, stride);
+}
+
+// Splits M into at most `depth` radices of Z_RADIX, none above rmax, in
+// descending order; false when it cannot.
+static bool z_factor(int M, int depth, int rmax, int *radix, int *nst) {
+  if (M == 1) {
+    *nst = 0;
+    return true;
+  }
+  if (depth == 0) return false;
+  for (int R : Z_RADIX)
+    if (R <= rmax && M % R == 0 && z_factor(M / R, depth - 1, R, radix + 1, nst)) {
+      radix[0] = R;
+      ++*nst;
+      return true;
+    }
+  return false;
+}
+
+// Threads, blocks an SM, the largest radix and the rows of 32 points a block
+// may hold.  The blocks wait for memory in turn, so what counts is how many
+// share an SM: four at 64 registers and 48 KB, which radices up to 10 allow.
+// Lengths that one radix of up to 12 transforms (M <= 12) take it at three
+// blocks an SM (nz = 24: 48 / 61 us for one stage, 71 / 73 for two); from M =
+// 111 on shared memory allows three, from 145 on one block, then of 16 warps
+// with radices up to 16 (nz = 512: 216 / 311 us, 257 / 322 with radices up to 8
+// in 32 warps).
+struct ZVariant {
+  int threads, blocks, rmax, rows;
+};
+static const ZVariant &z_variant(int M) {
+  static const ZVariant small = {256, 3, 12, 144}, mid = {256, 4, 10, 110}, large = {256, 3, 10, 144},
+                        whole = {512, 1, 16, ZN_MAX / 2};
+  return M <= 12 ? small : M <= mid.rows ? mid : M <= large.rows ? large : whole;
+}
+
+// The plan of a length (host data, made once per length).
+static const ZPlan235 &z_plan(int nz) {
+  static std::mutex mu;
+  static std::map<int, ZPlan235> plans;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = plans.find(nz);
+  if (it != plans.end()) return it->second;
+  ZPlan235 &Z = plans[nz];
+  Z.N = nz;
+  Z.M = nz / 2;
+  const long double pi = 3.14159265358979323846264338327950288L;
+  for (int t = 0; t <= Z.M; t++) {
+    Z.c[t] = (double)cosl(2 * pi * t / nz);
+    Z.s[t] = (double)-sinl(2 * pi * t / nz);
+    if (4 * t == nz) Z.c[t] = 0.0;  // exact at the quarter and half turns
+    if (4 * t == nz) Z.s[t] = -1.0;
+    if (2 * t == nz) Z.s[t] = 0.0;
+  }
+  const ZVariant &v = z_variant(Z.M);
+  // the fewest stages, and of those the smallest largest radix
+  Z.nst = 0;
+  for (int depth = 1; depth <= ZST && Z.nst == 0; depth++)
+    for (int i = (int)(sizeof(Z_RADIX) / sizeof(int)) - 1; i >= 0 && Z.nst == 0; i--)
+      if (Z_RADIX[i] <= v.rmax && !z_factor(Z.M, depth, Z_RADIX[i], Z.radix, &Z.nst)) Z.nst = 0;
+  // enough groups that the longest stage's sub-transforms fill eight warps
+  const int per = Z.M / Z.radix[0];
+  Z.PG = std::max(1, std::min((8 + per - 1) / per, v.rows / Z.M));
+  return Z;
+}
+
+template <int NT, int MINB, int RMAX>
+static int launch_rows(const ZPlan235 &Z, int rows, double *d, int npts, long long stride, int sign,
+                       cudaStream_t st) {
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [&]() {
+    attr = cudaFuncSetAttribute((k_z_fwd_any<NT, MINB, RMAX>), cudaFuncAttributeMaxDynamicSharedMemorySize, rows * 512);
+    if (attr == cudaSuccess)
+      attr = cudaFuncSetAttribute((k_z_inv_any<NT, MINB, RMAX>), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  rows * 512);
+  });
+  SX_CUDA(attr);
+  const int grid = (npts + 32 * Z.PG - 1) / (32 * Z.PG);
+  const size_t smem = (size_t)Z.PG * Z.M * 512;
+  if (sign == 1)
+    k_z_fwd_any<NT, MINB, RMAX><<<grid, NT, smem, st>>>(Z, d, npts, stride, 1.0 / Z.N);
+  else
+    k_z_inv_any<NT, MINB, RMAX><<<grid, NT, smem, st>>>(Z, d, npts, stride);
+  SX_CUDA(cudaGetLastError());
+  return SX_OK;
+}
+
+static int launch_any(double *d, int nz, int npts, long long stride, int sign, cudaStream_t st) {
+  const ZPlan235 &Z = z_plan(nz);
+  const ZVariant &v = z_variant(Z.M);
+  if (v.blocks == 4) return launch_rows<256, 4, 10>(Z, v.rows, d, npts, stride, sign, st);
+  if (v.rmax == 12) return launch_rows<256, 3, 12>(Z, v.rows, d, npts, stride, sign, st);
+  if (v.blocks == 3) return launch_rows<256, 3, 10>(Z, v.rows, d, npts, stride, sign, st);
+  return launch_rows<512, 1, 16>(Z, v.rows, d, npts, stride, sign, st);
+}
+
 template <int N>
 static void launch_reg(double *d, int npts, long long stride, int sign, cudaStream_t st) {
   const int grid = (npts + 127) / 128;
@@ -478,17 +946,15 @@ extern "C" int sx_transform_z(double *d_data, int nz, int plane_stride, int npts
     SX_CUDA(cudaGetLastError());
     return SX_OK;
   }
-  if (nz <= TWN && (nz & (nz - 1)) == 0) {
+  if (nz <= ZN_MAX) {
     // one pass through shared memory, enqueued without waiting
-    SX_TRY(ensure_twiddles());
-    cudaStream_t st = (cudaStream_t)stream;
-    switch (nz) {
-      case 128: SX_TRY(launch_smem<128>(d_data, npts, plane_stride, sign, st)); break;
-      case 256: SX_TRY(launch_smem<256>(d_data, npts, plane_stride, sign, st)); break;
-      default: SX_TRY(launch_smem<512>(d_data, npts, plane_stride, sign, st)); break;
+    if (nz == 256) {  // the radix-2 four-step kernels: 243 / 281 us on 248,000 points, the others' 281 / 328
+      SX_TRY(ensure_twiddles());
+      SX_TRY(launch_smem<256>(d_data, npts, plane_stride, sign, (cudaStream_t)stream));
+      SX_CUDA(cudaGetLastError());
+      return SX_OK;
     }
-    SX_CUDA(cudaGetLastError());
-    return SX_OK;
+    return launch_any(d_data, nz, npts, plane_stride, sign, (cudaStream_t)stream);
   }
   const CufftApi &api = cufft_api();
   if (!api.ok) {

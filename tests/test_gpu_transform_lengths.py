@@ -1,0 +1,42 @@
+"""sx_transform_z at every length it takes up to 512, and two beyond (the
+library path): one stage and several, each kernel variant's largest and
+smallest block, ragged point counts and padded planes; against numpy's FFT of
+the same packing in 64 bits.  Tolerance: the FFT's error grows as log2(nz)
+roundings, 2^-53 each; 1e-14 of the largest value is about eight times that."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _lengths():
+    out = []
+    for n in range(2, 513, 2):
+        m = n
+        for f in (2, 3, 5):
+            while m % f == 0:
+                m //= f
+        if m == 1:
+            out.append(n)
+    return out + [540, 768]
+
+
+@pytest.mark.parametrize("nz", _lengths())
+def test_transform_every_length(nz):
+    import torch
+    import semtex_b200 as sx
+    for npts, stride in ((1, 1), (77, 80), (300, 301)):
+        x = np.random.default_rng(nz + npts).standard_normal((nz, stride))
+        d = torch.tensor(x, device="cuda")
+        sx.transform_z(d.data_ptr(), nz, stride, npts, +1)
+        X = d.cpu().numpy()
+        F = np.fft.rfft(x[:, :npts], axis=0) / nz
+        want = np.empty((nz, npts))
+        want[0], want[1] = F[0].real, F[nz // 2].real
+        want[2::2], want[3::2] = F[1:nz // 2].real, F[1:nz // 2].imag
+        assert np.abs(X[:, :npts] - want).max() <= 1e-14 * np.abs(want).max()
+        assert np.array_equal(X[:, npts:], x[:, npts:])
+        sx.transform_z(d.data_ptr(), nz, stride, npts, -1)
+        back = d.cpu().numpy()
+        assert np.abs(back[:, :npts] - x[:, :npts]).max() <= 1e-14 * np.abs(x).max()
+        assert np.array_equal(back[:, npts:], x[:, npts:])
