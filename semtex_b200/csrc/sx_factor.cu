@@ -12,10 +12,10 @@
 //      (deterministic; src/matrix.cpp:236-241).  Mixed-BC diagonal terms
 //      follow in boundary order (Mixed::augmentSC, src/condition.cpp:347-381).
 //   3. Tiled right-looking banded Cholesky, A = U^T U (LAPACK dpbtrf "U",
-//      src/matrix.cpp:259): per block column k, k_potrf factors the diagonal
-//      tile and forms its inverse, k_trsm forms the off-diagonal tiles of
-//      block row k, k_update applies the trailing rank-nb update inside the
-//      band.  All systems of a batch share each launch.
+//      src/matrix.cpp:259): per block column k, k_trsm forms the off-diagonal
+//      tiles of block row k, k_update applies the trailing rank-nb update
+//      inside the band and factors the next diagonal tile.  All systems of a
+//      batch share each launch.
 //      What is kept is the block LDL^T form of the same factor: the diagonal
 //      tiles U_kk, their inverses D_k, and off the diagonal U_kk^-1 U(k, k+i)
 //      in place of U(k, k+i), so that the sweeps' block-column chains carry
@@ -353,21 +353,21 @@ __device__ __forceinline__ void mma_zero(MmaAcc &acc) {
     for (int n = 0; n < 4; n++) acc.v[m][n][0] = acc.v[m][n][1] = 0.0;
 }
 
-// T -= acc at this thread's result elements (one subtraction each, after
+// R = T - acc at this thread's result elements (one subtraction each, after
 // the whole product: the order of the reference's blocked update, C - A^T B
-// with the product formed first).
-__device__ __forceinline__ void mma_sub_store(double *T, const MmaAcc &acc) {
+// with the product formed first); R of row pitch LD.
+template <int LD>
+__device__ __forceinline__ void mma_sub_to(double *R, const double *T, const MmaAcc &acc) {
   int r0, c0, g, t;
   mma_coords(r0, c0, g, t);
 #pragma unroll
   for (int m = 0; m < 2; m++)
 #pragma unroll
-    for (int n = 0; n < 4; n++)
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        double *c = &T[(r0 + 8 * m + g) * LDT + c0 + 8 * n + 2 * t + q];
-        *c = *c - acc.v[m][n][q];
-      }
+    for (int n = 0; n < 4; n++) {
+      const int r = r0 + 8 * m + g, c = c0 + 8 * n + 2 * t;
+      const double2 v = *reinterpret_cast<const double2 *>(&T[r * LDT + c]);
+      *reinterpret_cast<double2 *>(&R[r * LD + c]) = make_double2(v.x - acc.v[m][n][0], v.y - acc.v[m][n][1]);
+    }
 }
 
 // Stores this thread's result elements into a tile of row pitch LD.
@@ -394,11 +394,11 @@ __device__ __forceinline__ void mma_block8(double &d0, double &d1, const double 
     mma_f64(d0, d1, TRANS ? A[(l + t) * LDM + r + g] : A[(r + g) * LDM + l + t], B[(l + t) * LDM + c + g]);
 }
 
-// Factor the diagonal tile of block column k, A = U^T U (upper), and form
-// D_k = U^-1: one CTA of eight warps per system, the serial link between the
-// block columns of a factorisation (one system leaves the rest of the chip
-// idle meanwhile).  What bounds it is the chain of 64 pivots, so the pivots'
-// steps stay in registers:
+// Factor the diagonal tile of block column k, A = U^T U (upper), staged in
+// shared memory (pitch LDM), and form D_k = U^-1 (X, zeroed by the caller
+// before its last barrier): one CTA of eight warps per system, the serial
+// link between the block columns of a factorisation.  What bounds it is the
+// chain of 64 pivots, so the pivots' steps stay in registers:
 //   Cholesky by panels of 16 rows.  A warp holds the panel's 16 diagonal
 //   columns in its lower lanes and 16 columns to the right in its upper ones,
 //   16 rows a lane; pivot c is lane c's, every warp factors the diagonal block
@@ -410,19 +410,9 @@ __device__ __forceinline__ void mma_block8(double &d0, double &d1, const double 
 //   on the tensor cores.
 // Measured (10 systems side by side): 78 -> 18.6 us a block column against one
 // block barrier and a square root and division in every thread per pivot.
-__global__ void __launch_bounds__(256) k_potrf(const SysDesc *__restrict__ sys, int k) {
-  const SysDesc S = sys[blockIdx.x];
-  if (k >= S.nblk) return;
+__device__ __forceinline__ void factor_diag(const SysDesc &S, int k, double *A, double *X, double *rinv) {
   constexpr int PW = 16, NP4 = NB / PW;  // panel width, panels
-  extern __shared__ __align__(16) double smp[];
-  double *A = smp, *X = smp + NB * LDM, *rinv = X + NB * LDM;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
-  double *T = S.tiles + ((size_t)k * (S.J + 1)) * TSZ;
-  tile_stage_mma(A, T);
-  cp_async_commit();
-  for (int idx = tid; idx < NB * LDM; idx += 256) X[idx] = 0.0;
-  cp_async_wait_all();
-  __syncthreads();
   bool bad = false;
   for (int p = 0; p < NP4; p++) {
     const int c0 = p * PW, right = NP4 - 1 - p;  // 16-column groups right of the panel
@@ -504,7 +494,7 @@ __global__ void __launch_bounds__(256) k_potrf(const SysDesc *__restrict__ sys, 
       __syncthreads();
     }
   }
-  double *D = S.dinv + (size_t)k * TSZ;
+  double *T = S.tiles + ((size_t)k * (S.J + 1)) * TSZ, *D = S.dinv + (size_t)k * TSZ;
   for (int idx = tid; idx < NB * NB; idx += 256) {
     const int i = idx / NB, j = idx % NB;
     T[idx] = j < i ? 0.0 : A[i * LDM + j];
@@ -550,24 +540,42 @@ __global__ void __launch_bounds__(256, 3) k_trsm(const SysDesc *__restrict__ sys
 // subtracted from the target tile once: accumulating into the target
 // instead moved an ill-conditioned mode's solution 170 times further from
 // LAPACK's (1.3e-12 -> 2.2e-10 relative, config 5's pressure mode 1).
-__global__ void __launch_bounds__(256, 3) k_update(const SysDesc *__restrict__ sys, int k,
+//
+// The CTA of pair (1, 1) holds the diagonal tile of block column k + 1 when
+// its update is done, and factors it on the spot (k = -1: block column 0,
+// which nothing updates): the pivots' chain runs under the other pairs'
+// products and the block column is a launch and a tile's way to memory and
+// back shorter.  Blocks count the systems first, so that every system's chain
+// starts with the launch.  Ten systems of 171 block columns built and solved:
+// 11.1 -> 10.1 ms against a launch of its own for the diagonal tiles.
+__global__ void __launch_bounds__(256, 3) k_update(const SysDesc *__restrict__ sys, int ns, int k,
                                                    const int2 *__restrict__ pairs) {
-  const SysDesc S = sys[blockIdx.y];
-  const int2 pr = pairs[blockIdx.x];
+  const SysDesc S = sys[blockIdx.x % ns];
+  const int2 pr = pairs[blockIdx.x / ns];
   const int i = pr.x, j = pr.y;
-  if (k >= S.nblk || j > S.J || k + j >= S.nblk || (S.jb && j > S.jb[k])) return;
+  const bool prod = k >= 0 && j <= S.J && !(S.jb && j > S.jb[k]);
+  if (k + j >= S.nblk || !(prod || j == 1)) return;
   extern __shared__ __align__(16) double smt[];
   double *A = smt, *B = A + NB * LDM;
   double *Ct = S.tiles + ((size_t)(k + j) * (S.J + 1) + (j - i)) * TSZ;
-  tile_stage_mma(A, S.row + (size_t)(i - 1) * TSZ);
-  tile_stage_mma(B, S.row + (size_t)(j - 1) * TSZ);
-  cp_async_commit();
   MmaAcc acc;
   mma_zero(acc);
-  cp_async_wait_all();
-  __syncthreads();
-  mma_tile<true>(acc, A, B);
-  mma_sub_store(Ct, acc);
+  if (prod) {
+    tile_stage_mma(A, S.row + (size_t)(i - 1) * TSZ);
+    if (i != j) tile_stage_mma(B, S.row + (size_t)(j - 1) * TSZ);
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();
+    mma_tile<true>(acc, A, i == j ? A : B);
+  }
+  if (j > 1) {
+    mma_sub_to<LDT>(Ct, Ct, acc);
+    return;
+  }
+  mma_sub_to<LDM>(B, Ct, acc);
+  __syncthreads();  // the products have been read
+  for (int idx = threadIdx.x; idx < NB * LDM; idx += 256) A[idx] = 0.0;
+  factor_diag(S, k + 1, B, A, B + NB * LDM);
 }
 
 // ---------------------------------------------------------------------------
@@ -671,23 +679,19 @@ int factor_batch(std::vector<System *> &systems, cudaStream_t st, bool sync, boo
   DBuf<SysDesc> dd;
   SX_TRY(dd.upload_on(hd.data(), hd.size(), st));
   std::vector<int2> pairs;
-  for (int j = 1; j <= maxJ; j++)
+  for (int j = 1; j <= std::max(maxJ, 1); j++)
     for (int i = 1; i <= j; i++) pairs.push_back(make_int2(i, j));
   DBuf<int2> dpairs;
-  if (!pairs.empty()) SX_TRY(dpairs.upload_on(pairs.data(), pairs.size(), st));
+  SX_TRY(dpairs.upload_on(pairs.data(), pairs.size(), st));
   const size_t smm = 2 * NB * LDM * sizeof(double), sm2 = (2 * NB * LDM + NB) * sizeof(double);
-  SX_CUDA(cudaFuncSetAttribute(k_potrf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
   SX_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm));
-  SX_CUDA(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm));
+  SX_CUDA(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
   const int ns = (int)systems.size();
-  for (int k = 0; k < maxblk; k++) {
-    k_potrf<<<ns, 256, sm2, st>>>(dd.p, k);
-    const int m = rowmax[k];
-    if (m > 0) {
-      // pairs are listed by j, so those with j <= m come first
-      k_trsm<<<dim3(m, ns), 256, smm, st>>>(dd.p, k, scaled);
-      k_update<<<dim3((unsigned)(m * (m + 1) / 2), ns), 256, smm, st>>>(dd.p, k, dpairs.p);
-    }
+  for (int k = -1; k < maxblk - 1; k++) {
+    const int m = k < 0 ? 0 : rowmax[k];
+    if (m > 0) k_trsm<<<dim3(m, ns), 256, smm, st>>>(dd.p, k, scaled);
+    // pairs are listed by j, so those with j <= m come first
+    k_update<<<(unsigned)(ns * std::max(1, m * (m + 1) / 2)), 256, sm2, st>>>(dd.p, ns, k, dpairs.p);
   }
   SX_CUDA(cudaGetLastError());
   if (sync) SX_CUDA(cudaStreamSynchronize(st));
@@ -734,7 +738,7 @@ static int system_reserve_direct(System &S, cudaStream_t st) {
   const size_t nb = (size_t)std::max(S.nblk, 1);
   SX_TRY(S.tiles.alloc_in(nb * (S.J + 1) * TSZ, S.pool, st));
   SX_TRY(S.tiles.zero(st));
-  return S.dinv.alloc_in(nb * TSZ, S.pool, st);  // k_potrf writes every block's tile in full
+  return S.dinv.alloc_in(nb * TSZ, S.pool, st);  // factor_diag writes every block's tile in full
 }
 
 int systems_build_direct(const std::vector<System *> &systems, cudaStream_t st) {
