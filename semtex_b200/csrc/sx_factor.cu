@@ -353,21 +353,59 @@ __device__ __forceinline__ void mma_zero(MmaAcc &acc) {
     for (int n = 0; n < 4; n++) acc.v[m][n][0] = acc.v[m][n][1] = 0.0;
 }
 
-// R = T - acc at this thread's result elements (one subtraction each, after
+// T -= acc at this thread's result elements (one subtraction each, after
 // the whole product: the order of the reference's blocked update, C - A^T B
-// with the product formed first); R of row pitch LD.
-template <int LD>
-__device__ __forceinline__ void mma_sub_to(double *R, const double *T, const MmaAcc &acc) {
+// with the product formed first).
+__device__ __forceinline__ void mma_sub(double *T, const MmaAcc &acc) {
   int r0, c0, g, t;
   mma_coords(r0, c0, g, t);
 #pragma unroll
   for (int m = 0; m < 2; m++)
 #pragma unroll
     for (int n = 0; n < 4; n++) {
-      const int r = r0 + 8 * m + g, c = c0 + 8 * n + 2 * t;
-      const double2 v = *reinterpret_cast<const double2 *>(&T[r * LDT + c]);
-      *reinterpret_cast<double2 *>(&R[r * LD + c]) = make_double2(v.x - acc.v[m][n][0], v.y - acc.v[m][n][1]);
+      double2 *q = reinterpret_cast<double2 *>(&T[(r0 + 8 * m + g) * LDT + c0 + 8 * n + 2 * t]);
+      const double2 v = *q;
+      *q = make_double2(v.x - acc.v[m][n][0], v.y - acc.v[m][n][1]);
     }
+}
+
+// C -= A^T A over the staged tiles, in the 8 x 8 blocks of the upper triangle:
+// a block row a warp (N blocks, the last N of the row), long and short rows
+// paired on a scheduler.  The same sums as mma_tile and mma_sub.
+template <int N>
+__device__ __forceinline__ void syrk_row(double *C, const double *A) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  constexpr int R = NB - 8 * N;  // first row, and first column
+  double v[N][2];
+#pragma unroll
+  for (int n = 0; n < N; n++) v[n][0] = v[n][1] = 0.0;
+#pragma unroll 4
+  for (int l0 = 0; l0 < NB; l0 += 4) {
+    const double *q = A + (l0 + t) * LDM + R + g;
+    double b[N];
+#pragma unroll
+    for (int n = 0; n < N; n++) b[n] = q[8 * n];
+#pragma unroll
+    for (int n = 0; n < N; n++) mma_f64(v[n][0], v[n][1], b[0], b[n]);
+  }
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    double2 *q = reinterpret_cast<double2 *>(&C[(R + g) * LDM + R + 8 * n + 2 * t]);
+    const double2 c = *q;
+    *q = make_double2(c.x - v[n][0], c.y - v[n][1]);
+  }
+}
+__device__ __forceinline__ void syrk_sub(double *C, const double *A) {
+  switch (threadIdx.x >> 5) {
+    case 0: return syrk_row<8>(C, A);
+    case 1: return syrk_row<7>(C, A);
+    case 2: return syrk_row<6>(C, A);
+    case 3: return syrk_row<5>(C, A);
+    case 4: return syrk_row<1>(C, A);
+    case 5: return syrk_row<2>(C, A);
+    case 6: return syrk_row<3>(C, A);
+    case 7: return syrk_row<4>(C, A);
+  }
 }
 
 // Stores this thread's result elements into a tile of row pitch LD.
@@ -395,51 +433,73 @@ __device__ __forceinline__ void mma_block8(double &d0, double &d1, const double 
 }
 
 // Factor the diagonal tile of block column k, A = U^T U (upper), staged in
-// shared memory (pitch LDM), and form D_k = U^-1 (X, zeroed by the caller
-// before its last barrier): one CTA of eight warps per system, the serial
-// link between the block columns of a factorisation.  What bounds it is the
-// chain of 64 pivots, so the pivots' steps stay in registers:
+// shared memory (pitch LDM), and form D_k = U^-1 in X: one CTA of eight warps
+// per system, the serial link between the block columns of a factorisation.
+// What bounds it is the chain of 64 pivots, so the pivots' steps stay in
+// registers:
 //   Cholesky by panels of 16 rows.  A warp holds the panel's 16 diagonal
 //   columns in its lower lanes and 16 columns to the right in its upper ones,
-//   16 rows a lane; pivot c is lane c's, every warp factors the diagonal block
-//   (the same numbers), and the columns to the right follow in the same
-//   instructions, with one shuffle per element of the pivot row and no
-//   barrier.  The trailing tile is then updated on the FP64 tensor cores.
+//   16 rows a lane.  Pivots go by fours: every lane takes the 4 x 4 diagonal
+//   block by shuffles and factors it (the same numbers), so that the chain
+//   from pivot to pivot is a square root and two products, then solves its own
+//   column's four rows and takes them out of the rows below, with one shuffle
+//   per element of the pivot rows, all independent.  The trailing tile is then
+//   updated on the FP64 tensor cores.
 //   Inverse: the four 16 x 16 diagonal blocks by back-substitution, a lane a
 //   column, then [A B; 0 C]^-1 = [A^-1, -A^-1 B C^-1; 0, C^-1] at 16 and 32
 //   on the tensor cores.
-// Measured (10 systems side by side): 78 -> 18.6 us a block column against one
-// block barrier and a square root and division in every thread per pivot.
+// Cycles of a diagonal tile (10 systems, other tiles being updated beside it):
+// 36,600 with one pivot a step -> 29,300; a factorisation of theirs with its
+// solve 10.1 -> 9.4 ms.
 __device__ __forceinline__ void factor_diag(const SysDesc &S, int k, double *A, double *X, double *rinv) {
-  constexpr int PW = 16, NP4 = NB / PW;  // panel width, panels
+  constexpr int PW = 16, NP4 = NB / PW, MB = 4;  // panel width, panels, pivots a step
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
   bool bad = false;
   for (int p = 0; p < NP4; p++) {
     const int c0 = p * PW, right = NP4 - 1 - p;  // 16-column groups right of the panel
-    if (w < max(1, right)) {
-      const int j = lane & (PW - 1);
-      const bool diag = lane < PW || right == 0;
-      const int col = diag ? c0 + j : c0 + PW * (w + 1) + j;
-      double a[PW];
+    const int j = lane & (PW - 1);
+    const bool busy = w < max(1, right), diag = lane < PW || right == 0;
+    const int col = diag ? c0 + j : c0 + PW * (w + 1) + j;
+    const bool mine = diag ? w == 0 && lane < PW : true;
+    double a[PW];
+    if (busy)
 #pragma unroll
       for (int i = 0; i < PW; i++) a[i] = A[(c0 + i) * LDM + col];
+    __syncthreads();  // every warp has the diagonal columns
+    if (busy) {
 #pragma unroll
-      for (int c = 0; c < PW; c++) {
-        double d = __shfl_sync(0xffffffffu, a[c], c);
-        if (!(d > 0.0)) {
-          bad = true;
-          d = 1.0;
+      for (int c = 0; c < PW; c += MB) {
+        double d[MB][MB], u[MB];  // d: the rows of U in the block, above its diagonal
+#pragma unroll
+        for (int k = 0; k < MB; k++)
+#pragma unroll
+          for (int i = 0; i <= k; i++) d[i][k] = __shfl_sync(0xffffffffu, a[c + i], c + k);
+#pragma unroll
+        for (int m = 0; m < MB; m++) {
+          const double x = d[m][m], r = rsqrt(x);
+          bad |= !(x > 0.0);  // (the NaN that follow stay in this factor)
+#pragma unroll
+          for (int k = m + 1; k < MB; k++) d[m][k] *= r;
+#pragma unroll
+          for (int i = m + 1; i < MB; i++)
+#pragma unroll
+            for (int k = i; k < MB; k++) d[i][k] = fma(-d[m][i], d[m][k], d[i][k]);
+          double v = a[c + m];
+#pragma unroll
+          for (int l = 0; l < m; l++) v = fma(-d[l][m], u[l], v);
+          u[m] = v * r;
+          const double q = x * r;  // sqrt(x), with one Newton step
+          if (mine) {
+            const int row = c + m;
+            A[(c0 + row) * LDM + col] = !diag || j > row ? u[m] : j == row ? fma(0.5 * r, fma(-q, q, x), q) : 0.0;
+          }
+          if (w == 0 && lane == 0) rinv[c0 + c + m] = r;
         }
-        const double r = rsqrt(d), u = a[c] * r;
 #pragma unroll
-        for (int i = c + 1; i < PW; i++) a[i] = fma(-__shfl_sync(0xffffffffu, u, i), u, a[i]);
-        const double q = d * r;  // sqrt(d), with one Newton step
-        a[c] = diag && j == c ? fma(0.5 * r, fma(-q, q, d), q) : u;
-        if (w == 0 && lane == 0) rinv[c0 + c] = r;
+        for (int i = c + MB; i < PW; i++)
+#pragma unroll
+          for (int m = 0; m < MB; m++) a[i] = fma(-__shfl_sync(0xffffffffu, u[m], i), u[m], a[i]);
       }
-      if (diag ? w == 0 && lane < PW : true)
-#pragma unroll
-        for (int i = 0; i < PW; i++) A[(c0 + i) * LDM + col] = diag && i > j ? 0.0 : a[i];
     }
     __syncthreads();
     // A(r, c) -= sum over the panel's rows of U(l, r) U(l, c), r <= c
@@ -495,10 +555,12 @@ __device__ __forceinline__ void factor_diag(const SysDesc &S, int k, double *A, 
     }
   }
   double *T = S.tiles + ((size_t)k * (S.J + 1)) * TSZ, *D = S.dinv + (size_t)k * TSZ;
-  for (int idx = tid; idx < NB * NB; idx += 256) {
-    const int i = idx / NB, j = idx % NB;
-    T[idx] = j < i ? 0.0 : A[i * LDM + j];
-    D[idx] = j < i ? 0.0 : X[i * LDM + j];
+  for (int idx = tid; idx < NB * NB / 2; idx += 256) {
+    const int i = idx / (NB / 2), j = 2 * (idx % (NB / 2));
+    const double2 u = *reinterpret_cast<const double2 *>(&A[i * LDM + j]);
+    const double2 x = *reinterpret_cast<const double2 *>(&X[i * LDM + j]);
+    reinterpret_cast<double2 *>(T)[idx] = make_double2(j < i ? 0.0 : u.x, j + 1 < i ? 0.0 : u.y);
+    reinterpret_cast<double2 *>(D)[idx] = make_double2(j < i ? 0.0 : x.x, j + 1 < i ? 0.0 : x.y);
   }
   if (bad && lane == 0) atomicOr(S.status, 1 << SX_ERR_NOT_SPD);
 }
@@ -547,8 +609,11 @@ __global__ void __launch_bounds__(256, 3) k_trsm(const SysDesc *__restrict__ sys
 // products and the block column is a launch and a tile's way to memory and
 // back shorter.  Blocks count the systems first, so that every system's chain
 // starts with the launch.  Ten systems of 171 block columns built and solved:
-// 11.1 -> 10.1 ms against a launch of its own for the diagonal tiles.
-__global__ void __launch_bounds__(256, 3) k_update(const SysDesc *__restrict__ sys, int ns, int k,
+// 11.1 -> 10.1 ms against a launch of its own for the diagonal tiles.  Two
+// blocks an SM: the pivots need the registers (at three 11.9 ms for 9.4), and
+// large launches lose nothing (12 systems of 1,206 block columns 258 ms, 268
+// at three before).
+__global__ void __launch_bounds__(256, 2) k_update(const SysDesc *__restrict__ sys, int ns, int k,
                                                    const int2 *__restrict__ pairs) {
   const SysDesc S = sys[blockIdx.x % ns];
   const int2 pr = pairs[blockIdx.x / ns];
@@ -558,24 +623,26 @@ __global__ void __launch_bounds__(256, 3) k_update(const SysDesc *__restrict__ s
   extern __shared__ __align__(16) double smt[];
   double *A = smt, *B = A + NB * LDM;
   double *Ct = S.tiles + ((size_t)(k + j) * (S.J + 1) + (j - i)) * TSZ;
-  MmaAcc acc;
-  mma_zero(acc);
-  if (prod) {
-    tile_stage_mma(A, S.row + (size_t)(i - 1) * TSZ);
-    if (i != j) tile_stage_mma(B, S.row + (size_t)(j - 1) * TSZ);
+  if (j == 1) {
+    tile_stage_mma(B, Ct);
+    if (prod) tile_stage_mma(A, S.row);
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-    mma_tile<true>(acc, A, i == j ? A : B);
-  }
-  if (j > 1) {
-    mma_sub_to<LDT>(Ct, Ct, acc);
+    if (prod) syrk_sub(B, A);
+    __syncthreads();
+    factor_diag(S, k + 1, B, A, B + NB * LDM);
     return;
   }
-  mma_sub_to<LDM>(B, Ct, acc);
-  __syncthreads();  // the products have been read
-  for (int idx = threadIdx.x; idx < NB * LDM; idx += 256) A[idx] = 0.0;
-  factor_diag(S, k + 1, B, A, B + NB * LDM);
+  tile_stage_mma(A, S.row + (size_t)(i - 1) * TSZ);
+  if (i != j) tile_stage_mma(B, S.row + (size_t)(j - 1) * TSZ);
+  cp_async_commit();
+  MmaAcc acc;
+  mma_zero(acc);
+  cp_async_wait_all();
+  __syncthreads();
+  mma_tile<true>(acc, A, i == j ? A : B);
+  mma_sub(Ct, acc);
 }
 
 // ---------------------------------------------------------------------------
