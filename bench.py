@@ -282,12 +282,12 @@ TILE_BYTES = 64 * 64 * 8   # one 64 x 64 band tile as stored
 
 
 def envelope_sweep_bytes(mesh, m, modes_planes):
-    """Bytes the two sweeps move: per system and sweep, the factor tiles
-    inside the envelope (the tiles above each diagonal tile, and the diagonal
-    inverse) once, and each right-hand side read and written."""
+    """Bytes the two sweeps move: per system, the factor tiles inside the
+    envelope above the diagonal tiles once a sweep, the diagonal inverses
+    once, and each right-hand side read and written a sweep."""
     above, _ = mesh.envelope()
-    tiles = int(above.sum()) + len(above)
-    return sum(2 * tiles * TILE_BYTES + 2 * 2 * P * m.nsolve * 8 for P in modes_planes)
+    tiles = 2 * int(above.sum()) + len(above)
+    return sum(tiles * TILE_BYTES + 2 * 2 * P * m.nsolve * 8 for P in modes_planes)
 
 
 def run_ours(args, rank, world):

@@ -703,7 +703,7 @@ extern "C" int sx_modal_autotune(sx_modal s, double *d_u, const double *d_f, con
   double best_t = INFINITY;
   bool best_ok = false;
   int trials = 0, rc = SX_OK;
-  // one candidate: three solves (the first captures the graphs), the faster
+  // one candidate: three solves (the first two may capture graphs), the faster
   // of the last two; kept when it converges and beats the best so far
   auto trial = [&](const Cand &c) {
     s->forced_cluster = c.sc.C;
