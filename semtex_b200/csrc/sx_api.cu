@@ -1,4 +1,5 @@
 // sx_api.cu -- C ABI: ModalMatrixSys and Field::solve replacements.
+#include <atomic>
 #include <cmath>
 #include <cstring>
 
@@ -13,6 +14,11 @@ using namespace sx;
 // ---------------------------------------------------------------------------
 // sx_modal_s
 // ---------------------------------------------------------------------------
+
+unsigned long long sx_modal_s::next_serial() {
+  static std::atomic<unsigned long long> n{0};
+  return ++n;
+}
 
 BandSched sx_modal_s::sched(int nj) {
   int J = 1;
@@ -38,6 +44,7 @@ BandSched sx_modal_s::sched(int nj) {
 }
 
 void sx_modal_s::rebind(sx_mesh_s *m, int base, int nmodes, int meth, std::vector<std::shared_ptr<System>> s) {
+  serial = next_serial();
   mesh = m;
   base_mode = base;
   num_modes = nmodes;
@@ -1049,7 +1056,7 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
     int planes = 0;
     for (auto &g : q.gd) planes += g.P;
     SX_TRY(reserve_ws(*q.s, planes));
-    key_ptr(key, q.s);
+    key.push_back((long long)q.s->serial);
     key_ptr(key, q.u);
     key_ptr(key, q.f);
     key_ptr(key, q.bc);
@@ -1253,7 +1260,7 @@ extern "C" int sx_batch_solve(sx_batch b, int count, const sx_modal *modals, dou
       it.stride = q.stride;
       item_of[i] = (int)items.size();
       items.push_back(it);
-      key_ptr(key, q.s);
+      key.push_back((long long)q.s->serial);
       key_ptr(key, q.u);
       key_ptr(key, q.f);
       key_ptr(key, q.bc);

@@ -40,6 +40,12 @@ struct DirectBatch {
 }  // namespace sx
 
 struct sx_modal_s {
+  // Names this object and its set of systems for as long as the process runs
+  // (rebind takes a new one): what is kept between calls under an object's
+  // address is kept under this too, since a later object, and its buffers, may
+  // be given the same addresses.
+  unsigned long long serial = next_serial();
+  static unsigned long long next_serial();
   sx_mesh_s *mesh = nullptr;
   int device = 0;
   int base_mode = 0, num_modes = 0, method = SX_DIRECT;
@@ -99,10 +105,10 @@ constexpr int BATCH_BRANCHES = 16;
 // graphs, and the direct solve whose band sweeps cover every member.
 struct sx_batch_s {
   sx::MxBatch mixed;
-  std::vector<long long> mkey;  // members and buffers the mixed tables were built for
+  std::vector<long long> mkey;  // members (by serial) and buffers the mixed tables were built for
   sx::DBuf<sx::Job> djobs;      // every member's direct jobs, member by member
   std::vector<sx::Job> jobs;
-  std::vector<long long> dkey;  // members and buffers the direct graph was captured for
+  std::vector<long long> dkey;  // members (by serial) and buffers the direct graph was captured for
   cudaGraphExec_t dexec = nullptr;
   int dlaunches = 0;
   sx::BandSched sc;
