@@ -395,11 +395,14 @@ __global__ void __launch_bounds__(SWP_THREADS, 1)
     for (int i = 0; i < 2 * RPW; i++) acc[i] = 0.0;
   };
   // acc += tile j of step t, whose window slot is bs, times the block solved j
-  // steps before it, which the caller knows to be there
+  // steps before it, which the caller knows to be there.
   auto tile = [&](auto F, int j, int bs, int t) {
     const int zs = bs - j < 0 ? bs - j + W : bs - j;
     TileRegs r;
-    if (WIDE && j > W) {
+    // (block t - W's slot is the one block t is stored to, and backward the
+    // leader meets no barrier between a warp's read and another's store: it
+    // too is read from there)
+    if (WIDE && j >= W) {
       const int so = t - j;
       const double *z0 = Jb.rhs + (size_t)(so < nblk ? so : T - 1 - so) * NB;
       block_load_l2<decltype(F)::value>(r, z0, P > 1 ? z0 + Jb.rhs_stride : z0, w, lane);

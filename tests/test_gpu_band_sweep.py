@@ -71,13 +71,15 @@ def test_wide_band_equals_narrow(sx):
     new = np.arange(narrow.nglobal)
     new[:narrow.nsolve] = np.random.default_rng(8).permutation(narrow.nsolve)
     wide = dataclasses.replace(narrow, btog=new[narrow.btog].astype(np.int32), nband=narrow.nsolve)
-    assert (wide.nsolve - 1) // 64 > 100  # beyond the window
+    assert -(-(wide.nband - 1) // 64) > 110  # tiles a block column: beyond the window
     f = torch.tensor(np.random.default_rng(3).standard_normal((nz, narrow.nplane)), device="cuda")
     sols = []
-    for m, cases in ((narrow, ((0, 0),)), (wide, ((0, 0), (1, 0), (2, 2), (7, 1)))):
+    # the last two leave the leader the tile 64 block columns back, whose block's
+    # place in the window is the next one stored to, and little after it
+    for m, cases in ((narrow, ((0, 0),)), (wide, ((0, 0), (1, 0), (2, 2), (7, 1), (2, 31), (3, 62)))):
         S = sx.ModalMatrixSys(sx.Mesh(m), num_modes=2, method=sx.DIRECT, lambda2_modes=lam, betak2_modes=np.zeros(2))
         for cluster, lead in cases:
-            S.tune(band_cluster=cluster, band_lead=lead)
+            S.tune(band_cluster=cluster, band_stages=4 if lead > 2 else 0, band_lead=lead)
             fd, u = f.clone(), torch.zeros_like(f)
             S.solve_batched(u.data_ptr(), fd.data_ptr(), 0, nz, m.nplane, sx.FP64)
             torch.cuda.synchronize()
