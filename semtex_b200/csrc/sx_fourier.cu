@@ -386,21 +386,24 @@ __global__ void __launch_bounds__(ZW * 32, 3) k_z_inv_s(double *__restrict__ dat
   }
 }
 
+// A kernel's limit on dynamic shared memory is a setting of the current
+// device's copy of it, so every launch sets it (to the same value: callers do
+// not disturb one another).
+template <typename K>
+static cudaError_t dynamic_smem(K *kernel, int bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 template <int N>
 static int launch_smem(double *d, int npts, long long stride, int sign, cudaStream_t st) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, []() {
-    attr = cudaFuncSetAttribute(k_z_fwd_s<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem(N));
-    if (attr == cudaSuccess)
-      attr = cudaFuncSetAttribute(k_z_inv_s<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem(N));
-  });
-  SX_CUDA(attr);
   const int grid = (npts + 31) / 32;
-  if (sign == 1)
+  if (sign == 1) {
+    SX_CUDA(dynamic_smem(k_z_fwd_s<N>, (int)zsmem(N)));
     k_z_fwd_s<N><<<grid, ZW * 32, zsmem(N), st>>>(d, npts, stride, 1.0 / N);
-  else
+  } else {
+    SX_CUDA(dynamic_smem(k_z_inv_s<N>, (int)zsmem(N)));
     k_z_inv_s<N><<<grid, ZW * 32, zsmem(N), st>>>(d, npts, stride);
+  }
   return SX_OK;
 }
 
@@ -844,21 +847,15 @@ static const ZPlan235 &z_plan(int nz) {
 template <int NT, int MINB, int RMAX>
 static int launch_rows(const ZPlan235 &Z, int rows, double *d, int npts, long long stride, int sign,
                        cudaStream_t st) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [&]() {
-    attr = cudaFuncSetAttribute((k_z_fwd_any<NT, MINB, RMAX>), cudaFuncAttributeMaxDynamicSharedMemorySize, rows * 512);
-    if (attr == cudaSuccess)
-      attr = cudaFuncSetAttribute((k_z_inv_any<NT, MINB, RMAX>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  rows * 512);
-  });
-  SX_CUDA(attr);
   const int grid = (npts + 32 * Z.PG - 1) / (32 * Z.PG);
   const size_t smem = (size_t)Z.PG * Z.M * 512;
-  if (sign == 1)
+  if (sign == 1) {
+    SX_CUDA(dynamic_smem(k_z_fwd_any<NT, MINB, RMAX>, rows * 512));
     k_z_fwd_any<NT, MINB, RMAX><<<grid, NT, smem, st>>>(Z, d, npts, stride, 1.0 / Z.N);
-  else
+  } else {
+    SX_CUDA(dynamic_smem(k_z_inv_any<NT, MINB, RMAX>, rows * 512));
     k_z_inv_any<NT, MINB, RMAX><<<grid, NT, smem, st>>>(Z, d, npts, stride);
+  }
   SX_CUDA(cudaGetLastError());
   return SX_OK;
 }
