@@ -169,7 +169,11 @@ SX_API int sx_modal_status(sx_modal modal);
 /* Device memory held by the modal system (factors, element matrices). */
 SX_API unsigned long long sx_modal_device_bytes(sx_modal modal);
 /* Band factor of local mode m, in LAPACK "U" band storage
- * (ldab = nband, veclib/lapack.h:107-108): nsolve*nband doubles. */
+ * (ldab = nband, veclib/lapack.h:107-108): nsolve*nband doubles.  The
+ * factor is held in another form, so the system is assembled and factored
+ * again for the call, in as much device memory as it takes; where that is not
+ * free, U is formed from the resident factor on the host, to a few roundings.
+ * Any device may be current. */
 SX_API int sx_modal_band(sx_modal modal, int m, double *ab, int *nsolve, int *singular);
 
 /* ---- solve: replaces Field::solve (src/field.cpp:509-725) ----------------

@@ -217,19 +217,27 @@ extern "C" int sx_modal_create_ex(sx_mesh m, int base_mode, int num_modes, const
   return modal_build(m, base_mode, num_modes, lambda2, betak2, method, out);
 }
 
+// The given device is current while this lives.
+struct OnDevice {
+  int was = -1, now;
+  explicit OnDevice(int dev) : now(dev) {
+    cudaGetDevice(&was);
+    if (was != now) cudaSetDevice(now);
+  }
+  ~OnDevice() {
+    if (was != now) cudaSetDevice(was);
+  }
+};
+
 extern "C" int sx_modal_destroy(sx_modal s) {
   if (!s) return SX_OK;
   // the systems' memory is freed stream-ordered: work the caller enqueued
   // with them (on any stream) must finish first, and what the pool does not
   // keep goes back to the device before this returns
-  int dev = -1;
-  cudaGetDevice(&dev);
-  const int home = s->device;
-  if (home != dev) cudaSetDevice(home);
+  OnDevice home(s->device);
   cudaDeviceSynchronize();
   delete s;
   cudaStreamSynchronize(nullptr);
-  if (home != dev) cudaSetDevice(dev);
   return SX_OK;
 }
 
@@ -239,7 +247,10 @@ extern "C" int sx_modal_band(sx_modal s, int m, double *ab, int *nsolve, int *si
   if (nsolve) *nsolve = S.nsolve;
   if (singular) *singular = S.singular ? 1 : 0;
   if (S.method != SX_DIRECT) return SX_ERR_ARG;
-  if (ab) SX_TRY(system_band_export(S, ab));
+  if (ab) {
+    OnDevice home(s->device);  // the export builds the system again, where it lives
+    SX_TRY(system_band_export(S, ab));
+  }
   return SX_OK;
 }
 

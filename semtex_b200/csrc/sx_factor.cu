@@ -908,12 +908,9 @@ int system_build_jacobi_diag(System &S, cudaStream_t st, bool sync) {
   return SX_OK;
 }
 
-// The factor U in LAPACK "U" band storage, ldab = nband.  The resident tiles
-// hold it scaled, and U_kk times a scaled tile would give rounding noise where
-// U is exactly zero: the system is assembled and factored once more, keeping U.
-int system_band_export(const System &S, double *ab) {
-  const sx_mesh_s &Mh = *S.mesh;
-  const int nband = Mh.nband, kd = nband - 1;
+// The factor's tiles with U itself off the diagonal.  The resident ones hold
+// U_kk^-1 U(k, k+i): the system is assembled and factored once more, keeping U.
+static int tiles_refactored(const System &S, std::vector<double> &t) {
   System X;
   X.mesh = S.mesh;
   X.lambda2 = S.lambda2;
@@ -922,8 +919,40 @@ int system_band_export(const System &S, double *ab) {
   SX_TRY(system_build_direct(X, 0));
   std::vector<System *> one(1, &X);
   if (X.nsolve > 0) SX_TRY(factor_batch(one, 0, true, false));
-  std::vector<double> t((size_t)X.tiles.n);
+  t.resize(X.tiles.n);
   SX_CUDA(cudaMemcpy(t.data(), X.tiles.p, t.size() * 8, cudaMemcpyDeviceToHost));
+  return SX_OK;
+}
+
+// The same from the resident tiles, U_kk times each on the host: U to a few
+// roundings (noise where it is exactly zero inside a tile), but no device
+// memory.
+static int tiles_unscaled(const System &S, std::vector<double> &t) {
+  t.resize(S.tiles.n);
+  SX_CUDA(cudaMemcpy(t.data(), S.tiles.p, t.size() * 8, cudaMemcpyDeviceToHost));
+  const sx_mesh_s &Mh = *S.mesh;
+  const size_t col = (size_t)(S.J + 1) * TSZ;
+  for (int k = 0; k < S.nblk; k++)
+    for (int j = 1; j <= std::min(std::min(S.J, k), Mh.env[k]); j++) {
+      const double *U = &t[(size_t)(k - j) * col];
+      double *T = &t[(size_t)k * col + (size_t)j * TSZ];
+      for (int r = 0; r < NB; r++) {  // U_kk is upper triangular: row r takes rows r and below
+        double row[NB] = {};
+        for (int l = r; l < NB; l++)
+          for (int c = 0; c < NB; c++) row[c] += U[r * LDT + l] * T[l * LDT + c];
+        std::memcpy(T + r * LDT, row, sizeof(row));
+      }
+    }
+  return SX_OK;
+}
+
+// The factor U in LAPACK "U" band storage, ldab = nband.
+int system_band_export(const System &S, double *ab) {
+  const int nband = S.mesh->nband, kd = nband - 1;
+  std::vector<double> t;
+  int rc = tiles_refactored(S, t);
+  if (rc == SX_ERR_NOMEM) rc = tiles_unscaled(S, t);  // no room for the system a second time
+  SX_TRY(rc);
   std::memset(ab, 0, sizeof(double) * (size_t)S.nsolve * nband);
   for (int n = 0; n < S.nsolve; n++)
     for (int m = std::max(0, n - kd); m <= n; m++) ab[(size_t)n * nband + kd + m - n] = t[tile_addr(m, n, S.J)];
