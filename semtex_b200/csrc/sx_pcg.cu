@@ -325,12 +325,12 @@ int pcg_solve_job(const MeshView &M, const System &S, PcgWork &W, const Job &job
     }
     if (i == step_max) rc = SX_WARN_STEP_LIMIT;
     // kernels enqueued for this plane: RHS + initial residual (10, + 3 range
-    // zeroings when there are essential nodes, + 1 for BC values), 9 (+1)
-    // per iteration body, 1 to unpack
+    // zeroings when there are essential nodes), 9 (+1) per iteration body, 1
+    // to unpack
     if (launches) {
       const int zr = nzero > 0 ? 1 : 0;
       const int bodies = (i == step_max) ? i - 1 : i;
-      *launches += 10 + 3 * zr + (bc ? 1 : 0) + bodies * (9 + zr) + 1;
+      *launches += 10 + 3 * zr + bodies * (9 + zr) + 1;
     }
     k_g2l<<<M.nel, 128, 0, st>>>(M, W.x.p, bc, u);
     SX_CUDA(cudaGetLastError());
