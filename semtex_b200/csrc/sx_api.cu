@@ -1059,7 +1059,10 @@ void key_ptr(std::vector<long long> &k, const void *p) { k.push_back((long long)
 
 // The band Cholesky part of a batch: per member its RHS kernels, then one
 // band-sweep launch over every member's jobs, then per member the interior
-// back-substitution; captured once per member set and buffers.
+// back-substitution.  The first call with given members and buffers enqueues
+// this as it is (a program that solves once does not pay for a graph: 24
+// members with 180 systems 0.98 ms, host time and all, 2.4 when captured at once); the
+// second captures it, and later ones replay the graph.
 static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaStream_t st) {
   std::vector<long long> key;
   for (Part &q : parts) {
@@ -1082,51 +1085,63 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
     key.push_back(-1);
   }
   if (key.empty()) return SX_OK;
-  if (b->dexec && graphs && key == b->dkey) {
+  const bool same = graphs && key == b->dkey;
+  if (same && b->dexec) {
     SX_CUDA(cudaGraphLaunch(b->dexec, st));
     return SX_OK;
   }
-  if (b->dexec) cudaGraphExecDestroy(b->dexec);
-  b->dexec = nullptr;
-  b->dkey.clear();
-  std::vector<Job> jobs;
-  std::vector<size_t> j0;
-  int maxJ = 1, forced = 0, fstages = 0, flead = -1;
-  for (Part &q : parts) {
-    j0.push_back(jobs.size());
-    if (q.gd.empty()) continue;
-    const long long bcstride = (long long)std::max(q.s->mesh->nbound, 1) * q.s->mesh->np;
-    int slot = 0;
-    for (auto &g : q.gd) {
-      jobs.push_back(make_job(*q.s, g, slot, q.u, q.f, q.bc, q.stride, bcstride));
-      maxJ = std::max(maxJ, jobs.back().J);
-      slot += g.P;
-    }
-    forced = std::max(forced, q.s->forced_cluster);
-    fstages = std::max(fstages, q.s->forced_stages);
-    flead = std::max(flead, q.s->forced_lead);
-    SX_TRY(prepare_direct_kernels(q.s->mesh->view()));
+  std::vector<size_t> members, j0;  // and each member's first job
+  size_t njobs = 0;
+  for (size_t i = 0; i < parts.size(); i++) {
+    j0.push_back(njobs);
+    njobs += parts[i].gd.size();
+    if (!parts[i].gd.empty()) members.push_back(i);
   }
-  j0.push_back(jobs.size());
-  if (b->djobs.n < jobs.size()) SX_TRY(b->djobs.alloc(jobs.size()));
-  SX_CUDA(cudaMemcpyAsync(b->djobs.p, jobs.data(), jobs.size() * sizeof(Job), cudaMemcpyHostToDevice, st));
-  SX_CUDA(cudaStreamSynchronize(st));
-  b->jobs = jobs;
-  b->sc = BandSched();
-  b->sc.C = forced > 0 ? forced
-                       : pick_cluster((int)jobs.size(), std::min(16, std::max(1, maxJ - 1)), maxJ, &b->sc.S,
-                                      fstages);
-  if (forced > 0 && fstages > 0) b->sc.S = fstages;
-  b->sc.Q = flead >= 0 ? flead : default_lead(b->sc.C, maxJ);
+  j0.push_back(njobs);
+  if (!same) {
+    if (b->dexec) cudaGraphExecDestroy(b->dexec);
+    b->dexec = nullptr;
+    b->dkey.clear();
+    std::vector<Job> jobs;
+    int maxJ = 1, forced = 0, fstages = 0, flead = -1;
+    for (size_t i : members) {
+      Part &q = parts[i];
+      const long long bcstride = (long long)std::max(q.s->mesh->nbound, 1) * q.s->mesh->np;
+      int slot = 0;
+      for (auto &g : q.gd) {
+        jobs.push_back(make_job(*q.s, g, slot, q.u, q.f, q.bc, q.stride, bcstride));
+        maxJ = std::max(maxJ, jobs.back().J);
+        slot += g.P;
+      }
+      forced = std::max(forced, q.s->forced_cluster);
+      fstages = std::max(fstages, q.s->forced_stages);
+      flead = std::max(flead, q.s->forced_lead);
+      SX_TRY(prepare_direct_kernels(q.s->mesh->view()));
+    }
+    if (b->djobs.n < jobs.size()) SX_TRY(b->djobs.alloc(jobs.size()));
+    SX_CUDA(cudaMemcpyAsync(b->djobs.p, jobs.data(), jobs.size() * sizeof(Job), cudaMemcpyHostToDevice, st));
+    SX_CUDA(cudaStreamSynchronize(st));
+    b->jobs = jobs;
+    b->sc = BandSched();
+    b->sc.C = forced > 0 ? forced
+                         : pick_cluster((int)jobs.size(), std::min(16, std::max(1, maxJ - 1)), maxJ, &b->sc.S,
+                                        fstages);
+    if (forced > 0 && fstages > 0) b->sc.S = fstages;
+    b->sc.Q = flead >= 0 ? flead : default_lead(b->sc.C, maxJ);
+    if (graphs) b->dkey = key;
+  }
+  bool capture = same;
+  if (capture) {  // a capture of the caller's own takes the launches themselves
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SX_CUDA(cudaStreamIsCapturing(st, &cap));
+    capture = cap == cudaStreamCaptureStatusNone;
+  }
   // The members' element kernels before and after the sweeps are small and
   // independent: inside a capture they become parallel branches of the graph
   // (24 members of 4 to 144 elements: 813 us a call one after another, 406 as
   // branches).  Enqueued directly, every fork and join would be a call of its
   // own: one after another on st.
-  std::vector<size_t> members;
-  for (size_t i = 0; i < parts.size(); i++)
-    if (!parts[i].gd.empty()) members.push_back(i);
-  const size_t nbr = graphs ? std::min(members.size(), (size_t)BATCH_BRANCHES) : 1;
+  const size_t nbr = capture ? std::min(members.size(), (size_t)BATCH_BRANCHES) : 1;
   SX_TRY(b->reserve_branches(nbr > 1 ? nbr : 0));
   auto each_member = [&](const std::function<int(size_t, cudaStream_t)> &f) -> int {
     if (nbr > 1) {
@@ -1145,10 +1160,10 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
   auto body = [&]() -> int {
     int nl = 0;
     SX_TRY(each_member([&](size_t i, cudaStream_t s) {
-      const std::vector<Job> slice(jobs.begin() + j0[i], jobs.begin() + j0[i + 1]);
+      const std::vector<Job> slice(b->jobs.begin() + j0[i], b->jobs.begin() + j0[i + 1]);
       return direct_rhs_jobs(parts[i].s->mesh->view(), b->djobs.p + j0[i], slice, s, &nl);
     }));
-    SX_TRY(band_sweep_jobs(b->djobs.p, jobs, b->sc, st));
+    SX_TRY(band_sweep_jobs(b->djobs.p, b->jobs, b->sc, st));
     nl++;
     SX_TRY(each_member([&](size_t i, cudaStream_t s) {
       return direct_backsub_jobs(parts[i].s->mesh->view(), b->djobs.p + j0[i], (int)(j0[i + 1] - j0[i]), s, &nl);
@@ -1156,7 +1171,7 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
     b->dlaunches = nl;
     return SX_OK;
   };
-  if (!graphs) return body();
+  if (!capture) return body();
   cudaGraph_t g = nullptr;
   SX_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   const int rc = body();
@@ -1169,7 +1184,6 @@ static int batch_direct(sx_batch b, std::vector<Part> &parts, bool graphs, cudaS
   const cudaError_t ie = cudaGraphInstantiate(&b->dexec, g, 0);
   cudaGraphDestroy(g);
   SX_CUDA(ie);
-  b->dkey = key;
   SX_CUDA(cudaGraphLaunch(b->dexec, st));
   return SX_OK;
 }
