@@ -118,6 +118,15 @@ static bool same_constants(const System &S, double lambda2, double betak2, int m
 
 namespace sx {
 
+// What a band system may take of the pool beyond POOL_KEEP (modal_populate).
+constexpr uint64_t POOL_SPARE = uint64_t(128) << 20;
+
+// Device memory of one band system on a mesh.
+static size_t direct_bytes(const sx_mesh_s &M) {
+  const size_t nblk = std::max((M.nsolve + NB - 1) / NB, 1), J = (M.nband - 1 + NB - 1) / NB;
+  return (nblk * (J + 2) * TSZ + (size_t)M.nel * M.nint * (M.next + M.nint)) * sizeof(double);
+}
+
 int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const SystemProvider *prov,
                    cudaStream_t st) {
   // what this call builds: freed in the stream's order if it gives up early
@@ -153,13 +162,14 @@ int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const Sy
       found->lambda2 = lam[l];
       found->betak2 = bk2[l];
       found->method = kind;
-      SX_TRY(device_pool(M.mesh->device, &found->pool));
       built.push_back(found);
       // enqueued, the DIRECT ones together below; one wait for all of them
-      if (kind == SX_DIRECT)
+      if (kind == SX_DIRECT) {
         direct.push_back(found.get());
-      else
+      } else {
+        SX_TRY(device_pool(M.mesh->device, &found->pool));
         SX_TRY(system_build_jacobi(*found, st, false));
+      }
     }
     if (std::find(M.uniq.begin(), M.uniq.end(), found) == M.uniq.end()) M.uniq.push_back(found);
     M.sys.push_back(found);
@@ -168,6 +178,15 @@ int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const Sy
     SX_TRY(M.dstatus.alloc(1));
     SX_TRY(M.dstatus.zero(st));
   }
+  // Band systems live in the pool while that is the cheaper way to make and
+  // drop them.  From the pool, what is above POOL_KEEP is unmapped at the next
+  // wait and mapped again for the next systems, some 14 ms a GB; by cudaMalloc
+  // and cudaFree a system's five buffers take about 2 ms whatever their size.
+  // Built and dropped (pool / cudaMalloc): 32 systems of 0.17 GB 35 / 98 ms;
+  // 4 of 1.6 GB 100 / 78; 12 of 1.6 GB 340 / 190; 48 of 1.6 GB 1610 / 696; 16
+  // of 6.6 GB 2660 / 1480; at the line, 129 of 0.17 GB, 270 / 271.
+  if (direct.size() * direct_bytes(*M.mesh) <= POOL_KEEP + direct.size() * POOL_SPARE)
+    for (System *S : direct) SX_TRY(device_pool(M.mesh->device, &S->pool));
   SX_TRY(systems_build_direct(direct, st));
   for (System *S : direct)
     if (S->nsolve > 0) to_factor.push_back(S);

@@ -58,6 +58,8 @@ void gll_tables(int np, std::vector<double> &z, std::vector<double> &w, std::vec
 
 // The stream-ordered pool that meshes and modal systems of a device live in,
 // and giving back what the current device's pool keeps but does not use.
+// Up to POOL_KEEP bytes of it stay mapped for the next ones.
+constexpr uint64_t POOL_KEEP = uint64_t(4) << 30;
 int device_pool(int device, cudaMemPool_t *out);
 void device_pool_trim();
 

@@ -294,8 +294,6 @@ int mesh_kratio(const sx_mesh_desc *d, double *out) {
 // drops a mesh per request while other requests run; a program that builds
 // systems for one solve makes and frees five buffers a mode).  Up to
 // POOL_KEEP bytes of freed memory stay mapped for the next ones.
-constexpr uint64_t POOL_KEEP = uint64_t(4) << 30;
-
 static std::mutex pool_mu;
 static std::map<int, cudaMemPool_t> pools;
 
