@@ -160,7 +160,10 @@ SX_API int sx_modal_create(sx_mesh mesh, double lambda2, double beta, int base_m
 /* Same, with an explicit (lambda2, betak2) per local mode. */
 SX_API int sx_modal_create_ex(sx_mesh mesh, int base_mode, int num_modes, const double *lambda2,
                        const double *betak2, int method, sx_modal *out);
-/* ModalMatrixSys::~ModalMatrixSys, src/matrix.cpp:113-130. */
+/* ModalMatrixSys::~ModalMatrixSys, src/matrix.cpp:113-130.  Waits for the
+ * device.  The library keeps at most 4 GB of dropped meshes' and systems'
+ * memory per device for the next ones, and none while the device has less
+ * than 8 GB free. */
 SX_API int sx_modal_destroy(sx_modal modal);
 /* Status of the device work enqueued so far on this system: synchronises
  * the device, returns SX_OK or the first recorded device-side error (e.g.

@@ -253,10 +253,12 @@ extern "C" int sx_modal_destroy(sx_modal s) {
   // the systems' memory is freed stream-ordered: work the caller enqueued
   // with them (on any stream) must finish first, and what the pool does not
   // keep goes back to the device before this returns
-  OnDevice home(s->device);
+  const int device = s->device;
+  OnDevice home(device);
   cudaDeviceSynchronize();
   delete s;
   cudaStreamSynchronize(nullptr);
+  device_pool_release(device);
   return SX_OK;
 }
 

@@ -62,6 +62,10 @@ void gll_tables(int np, std::vector<double> &z, std::vector<double> &w, std::vec
 constexpr uint64_t POOL_KEEP = uint64_t(4) << 30;
 int device_pool(int device, cudaMemPool_t *out);
 void device_pool_trim();
+// Gives back what the pool of `device`, the current one, keeps but does not
+// use if the device has little else free (less than twice POOL_KEEP): there
+// the memory is worth more to other allocators than to the next systems.
+void device_pool_release(int device);
 
 // An allocation, tried again without the pool's idle memory when it fails.
 template <typename F>

@@ -325,6 +325,20 @@ void sx::device_pool_trim() {
   if (it != pools.end()) cudaMemPoolTrimTo(it->second, 0);
 }
 
+void sx::device_pool_release(int device) {
+  constexpr uint64_t WORTH = uint64_t(64) << 20;  // idle memory below this is not looked at
+  std::lock_guard<std::mutex> lk(pool_mu);
+  auto it = pools.find(device);
+  if (it == pools.end()) return;
+  uint64_t reserved = 0, used = 0;
+  if (cudaMemPoolGetAttribute(it->second, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(it->second, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+      reserved < used + WORTH)
+    return;
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr < 2 * POOL_KEEP) cudaMemPoolTrimTo(it->second, 0);
+}
+
 // The pool and a private stream for one mesh's uploads.
 struct MeshUpload {
   cudaMemPool_t pool = nullptr;

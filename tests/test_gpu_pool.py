@@ -60,3 +60,17 @@ for _ in range(2):
     del u, S
     assert free() > before - 64 * MB
 """)
+
+
+def test_nothing_is_kept_while_the_device_is_short():
+    _run("""
+m = rect_mesh(24, 24, 9, jitter=0.1, seed=4)
+mesh = sx.Mesh(m)
+def drop():
+    sx.ModalMatrixSys(mesh, num_modes=10, method=sx.DIRECT, lambda2_modes=np.linspace(1.0, 9.0, 10)).close()
+drop()
+before = free()  # the pool keeps some 600 MB
+hold = torch.empty(torch.cuda.mem_get_info()[0] - (6 << 30), dtype=torch.uint8, device="cuda")
+drop()
+assert free() > before - hold.numel() + 400 * MB  # it kept nothing
+""")
