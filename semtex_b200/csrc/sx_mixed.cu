@@ -418,11 +418,11 @@ __global__ void __launch_bounds__(NP * 32, 2) k_x_constrain(const __grid_constan
   constrain_body<NP, PK>(B, blockIdx.x, blockIdx.y);
 }
 
-template <int NP>
+template <int NP, bool PK>
 __global__ void __launch_bounds__(NP * 32, 2) k_x_constrain_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) constrain_body<NP, true>(sB, t % sB.neg, t / sB.neg);
+  if (tile_member(T, sB, t)) constrain_body<NP, PK>(sB, t % sB.neg, t / sB.neg);
 }
 
 // b = DSS(Ye) + <h,w>, essential tail zero; x = 0, r = b (FP32); per-plane
@@ -472,10 +472,11 @@ __global__ void __launch_bounds__(256) k_x_rhs(const __grid_constant__ MxMember 
   rhs_body<PK>(B, blockIdx.x, blockIdx.y);
 }
 
+template <bool PK>
 __global__ void __launch_bounds__(256) k_x_rhs_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) rhs_body<true>(sB, t % sB.G, t / sB.G);
+  if (tile_member(T, sB, t)) rhs_body<PK>(sB, t % sB.G, t / sB.G);
 }
 
 // ---------------------------------------------------------------------------
@@ -553,6 +554,10 @@ __device__ __forceinline__ float gather_we(const MxMember &B, const float *__res
 // Resident blocks per SM that the register budget is set for (shared memory
 // allows 3 at np <= 9 and 2 at np <= 11).
 constexpr int cg_min_blocks(int np) { return np <= 9 ? 3 : (np <= 11 ? 2 : 1); }
+// The same for blocks of several elements: at low orders the compiler would
+// take twice the registers (121 a thread for 60 at np = 4), and half the
+// blocks would fit.
+constexpr int cg_min_blocks_packed(int np) { return np <= 4 ? 6 : np <= 6 ? 10 - np : cg_min_blocks(np); }
 constexpr long long CG_WAIT_LIMIT = CG_WAIT_DEFAULT;  // clock cycles: about a second
 
 // Cycles the first wait for a block's staged spans may take before the
@@ -849,16 +854,17 @@ __device__ __forceinline__ void cg_body(const MxMember &B, int eg, int y, int it
 }
 
 template <int NP, bool PK>
-__global__ void __launch_bounds__(NP * 32, cg_min_blocks(NP))
+__global__ void __launch_bounds__(NP * 32, PK ? cg_min_blocks_packed(NP) : cg_min_blocks(NP))
     k_cg(const __grid_constant__ MxMember B, int it, int mode) {
   cg_body<NP, PK>(B, blockIdx.x, blockIdx.y, it, mode);
 }
 
-template <int NP>
-__global__ void __launch_bounds__(NP * 32, cg_min_blocks(NP)) k_cg_multi(MxTable T, int it, int mode) {
+template <int NP, bool PK>
+__global__ void __launch_bounds__(NP * 32, PK ? cg_min_blocks_packed(NP) : cg_min_blocks(NP))
+    k_cg_multi(MxTable T, int it, int mode) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) cg_body<NP, true>(sB, t % sB.neg, t / sB.neg, it, mode);
+  if (tile_member(T, sB, t)) cg_body<NP, PK>(sB, t % sB.neg, t / sB.neg, it, mode);
 }
 
 // ---------------------------------------------------------------------------
@@ -913,11 +919,11 @@ __global__ void __launch_bounds__(NP * 32, 2) k_x_op64(const __grid_constant__ M
   op64_body<NP, PK>(B, blockIdx.x, blockIdx.y);
 }
 
-template <int NP>
+template <int NP, bool PK>
 __global__ void __launch_bounds__(NP * 32, 2) k_x_op64_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) op64_body<NP, true>(sB, t % sB.neg, t / sB.neg);
+  if (tile_member(T, sB, t)) op64_body<NP, PK>(sB, t % sB.neg, t / sB.neg);
 }
 
 // r = b - A x (FP64), essential tail zero; the next round's inner solve
@@ -958,10 +964,11 @@ __global__ void __launch_bounds__(256) k_x_res(const __grid_constant__ MxMember 
   res_body<PK>(B, blockIdx.x, blockIdx.y);
 }
 
+template <bool PK>
 __global__ void __launch_bounds__(256) k_x_res_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) res_body<true>(sB, t % sB.G, t / sB.G);
+  if (tile_member(T, sB, t)) res_body<PK>(sB, t % sB.G, t / sB.G);
 }
 
 // u = x at element nodes, essential values from the boundary lines (global2local +
@@ -1010,11 +1017,11 @@ __global__ void __launch_bounds__(256) k_x_unpack(const __grid_constant__ MxMemb
   unpack_body<NP, PK>(B, blockIdx.x, blockIdx.y);
 }
 
-template <int NP>
+template <int NP, bool PK>
 __global__ void __launch_bounds__(256) k_x_unpack_multi(MxTable T) {
   __shared__ MxMember sB;
   int t;
-  if (tile_member(T, sB, t)) unpack_body<NP, true>(sB, t % sB.neg, t / sB.neg);
+  if (tile_member(T, sB, t)) unpack_body<NP, PK>(sB, t % sB.neg, t / sB.neg);
 }
 
 // ---------------------------------------------------------------------------
@@ -1036,10 +1043,12 @@ __global__ void __launch_bounds__(256) k_x_unpack_multi(MxTable T) {
     default: break;                                            \
   }
 
-// Runs the statements with PK_ = whether workspace W's chunks hold fewer than 32 planes.
-#define SX_PK_SWITCH(W, ...)           \
+// Runs the statements with PK_ = whether blocks hold several elements: those of
+// workspace W's chunks, or P says so.
+#define SX_PK_SWITCH(W, ...) SX_PACKED((W).lp < MX_CH, __VA_ARGS__)
+#define SX_PACKED(P, ...)              \
   do {                                 \
-    if ((W).lp < MX_CH) {              \
+    if (P) {                           \
       constexpr bool PK_ = true;       \
       __VA_ARGS__;                     \
     } else {                           \
@@ -1054,17 +1063,44 @@ static int grid_nodes(int npts, int ep) {
   return std::max(1, std::min((npts + 4 * MX_ROWS * ep - 1) / (4 * MX_ROWS * ep), 6 * 148));
 }
 
-// Planes a chunk: 32, 16 or 8, whichever pads nz planes least (the widest on a
-// tie).  The iterations stream whole chunks, so an idle lane costs what a
-// working one does; a narrower chunk reads the element geometry once more for
-// the same planes (16 bytes a node for 8 planes, against 40 bytes a node and
-// plane of vectors).  Measured: 16 planes of 8192 elements of order 10, one
-// solve 15.8 ms in 32-plane chunks, 8.9 ms in 16-plane ones.
-static int chunk_planes(int nz) {
-  int best = MX_CH;
-  for (int lp = MX_CH / 2; lp >= 8; lp /= 2)
-    if ((nz + lp - 1) / lp * lp < (nz + best - 1) / best * best) best = lp;
-  return best;
+// Blocks of an iteration on one member, lp planes a chunk.
+static long long chunk_blocks(int nel, int nz, int lp) {
+  const int ep = MX_CH / lp;
+  return (long long)((nel + ep - 1) / ep) * ((nz + lp - 1) / lp);
+}
+
+// Planes a chunk of the members that are solved together, their iterations
+// side by side on the chip: 32, 16 or 8, whichever makes the fewest blocks of a
+// member (the widest on a tie), if that takes blocks off the fullest SM; 32 for
+// all of them otherwise.  An idle lane costs what a working one does, so fewer
+// blocks are faster once an SM has several to work off, by about the ratio of
+// the blocks.  A block of several elements takes about a tenth longer than one
+// of a single element (three tenths at np <= 4), so on small meshes, which fit
+// the chip either way, it only loses.  One solve at
+// tol 1e-10, always 32 planes / fewest blocks / this rule, us:
+//   np 11, 1920 elements,  2 planes 4470 / 1530 / 1530, 18 planes 4440 / 3810 / 3810
+//   np  9, 1024 elements, 10 planes  990 /  750 /  750, 50 planes 1830 / 1790 / 1830
+//   np  9,  256 elements, 18 planes  440 /  469 /  440
+//   np  8,    4 elements, 24 planes, an iteration  12.0 / 14.9 / 12.0
+//   np  4, 1920 elements, 18 planes  394 /  455 /  394,  2 planes  393 / 276 / 279
+struct ChunkMember {
+  int np, nel, nz;
+};
+static std::vector<int> chunk_planes(const std::vector<ChunkMember> &members) {
+  constexpr int SMS = 148;
+  long long wide = 0;
+  double packed = 0.0;
+  std::vector<int> out;
+  for (const ChunkMember &m : members) {
+    int best = MX_CH;
+    for (int lp = MX_CH / 2; lp >= 8; lp /= 2)
+      if (chunk_blocks(m.nel, m.nz, lp) < chunk_blocks(m.nel, m.nz, best)) best = lp;
+    out.push_back(best);
+    wide += chunk_blocks(m.nel, m.nz, MX_CH);
+    packed += (best == MX_CH ? 1.0 : m.np <= 4 ? 1.3 : 1.1) * (double)chunk_blocks(m.nel, m.nz, best);
+  }
+  if (std::ceil(packed / SMS) >= std::ceil((double)wide / SMS)) out.assign(members.size(), MX_CH);
+  return out;
 }
 
 template <int NP, bool PK>
@@ -1226,10 +1262,10 @@ __global__ void k_x_pce(MeshView M, int nch, int neg, int lp, int Mc, const floa
   }
 }
 
-static int setup(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &groups, int nz, int num_modes,
-                 cudaStream_t st) {
+static int setup(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &groups, int nz, int lp,
+                 int num_modes, cudaStream_t st) {
   const int npts = M.nglobal + M.nel * M.nint;
-  const int lp = chunk_planes(nz), nch = (nz + lp - 1) / lp, PP = nch * lp;
+  const int nch = (nz + lp - 1) / lp, PP = nch * lp;
   const int ep = MX_CH / lp, neg = (M.nel + ep - 1) / ep;
   const int Mc = std::max(1, num_modes);
   {
@@ -1342,7 +1378,7 @@ int mixed_solve(const MeshView &M, MixedWork &W, const std::vector<MxGroup> &gro
     if (W.g_init) cudaGraphExecDestroy(W.g_init);
     if (W.g_round) cudaGraphExecDestroy(W.g_round);
     W.g_init = W.g_round = nullptr;
-    SX_TRY(setup(M, W, groups, nz, num_modes, st));
+    SX_TRY(setup(M, W, groups, nz, chunk_planes({{M.np, M.nel, nz}})[0], num_modes, st));
     int attr_rc = SX_OK;
     SX_PK_SWITCH(W, SX_NP_SWITCH_M(M.np, (attr_rc = set_smem_attrs<N_, PK_>())));
     SX_TRY(attr_rc);
@@ -1462,8 +1498,11 @@ static int per_class(MxBatch &B, cudaStream_t st,
 static int enqueue_init_multi(MxBatch &B, cudaStream_t st, int *nl) {
   *nl = 2 * (int)B.cls.size();
   return per_class(B, st, [&](const MxBatch::Class &c, cudaStream_t s) {
-    SX_NP_SWITCH_M(c.np, (k_x_constrain_multi<N_><<<c.te, N_ * 32, x64_smem(N_), s>>>(class_table(B, c, 0))));
-    k_x_rhs_multi<<<c.tn, 256, 0, s>>>(class_table(B, c, 1));
+    const MxTable Te = class_table(B, c, 0), Tn = class_table(B, c, 1);
+    SX_PACKED(c.ep > 1, {
+      SX_NP_SWITCH_M(c.np, (k_x_constrain_multi<N_, PK_><<<c.te, N_ * 32, x64_smem(N_), s>>>(Te)));
+      k_x_rhs_multi<PK_><<<c.tn, 256, 0, s>>>(Tn);
+    });
     SX_CUDA(cudaGetLastError());
     return SX_OK;
   });
@@ -1473,27 +1512,29 @@ static int enqueue_round_multi(MxBatch &B, int n_inner, bool check_stop, cudaStr
   *nl = (int)B.cls.size() * (n_inner + 3);
   return per_class(B, st, [&](const MxBatch::Class &c, cudaStream_t s) {
     const MxTable Te = class_table(B, c, 0), Tn = class_table(B, c, 1);
-    SX_NP_SWITCH_M(c.np, (k_cg_multi<N_><<<c.te, N_ * 32, cg_smem(N_, c.ep), s>>>(Te, 0, CG_INIT)));
-    for (int it = 0; it < n_inner; it++) {
-      const int mode = (it == n_inner - 1 ? CG_LAST : CG_ITER) | (check_stop ? CG_CHECK_STOP : 0);
-      SX_NP_SWITCH_M(c.np, (k_cg_multi<N_><<<c.te, N_ * 32, cg_smem(N_, c.ep), s>>>(Te, it, mode)));
-    }
-    SX_NP_SWITCH_M(c.np, (k_x_op64_multi<N_><<<c.te, N_ * 32, x64_smem(N_), s>>>(Te)));
-    k_x_res_multi<<<c.tn, 256, 0, s>>>(Tn);
+    SX_PACKED(c.ep > 1, {
+      SX_NP_SWITCH_M(c.np, (k_cg_multi<N_, PK_><<<c.te, N_ * 32, cg_smem(N_, c.ep), s>>>(Te, 0, CG_INIT)));
+      for (int it = 0; it < n_inner; it++) {
+        const int mode = (it == n_inner - 1 ? CG_LAST : CG_ITER) | (check_stop ? CG_CHECK_STOP : 0);
+        SX_NP_SWITCH_M(c.np, (k_cg_multi<N_, PK_><<<c.te, N_ * 32, cg_smem(N_, c.ep), s>>>(Te, it, mode)));
+      }
+      SX_NP_SWITCH_M(c.np, (k_x_op64_multi<N_, PK_><<<c.te, N_ * 32, x64_smem(N_), s>>>(Te)));
+      k_x_res_multi<PK_><<<c.tn, 256, 0, s>>>(Tn);
+    });
     SX_CUDA(cudaGetLastError());
     return SX_OK;
   });
 }
 
-template <int NP>
+template <int NP, bool PK>
 static int set_smem_attrs_multi() {
-  SX_CUDA(cudaFuncSetAttribute(k_x_constrain_multi<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  SX_CUDA(cudaFuncSetAttribute((k_x_constrain_multi<NP, PK>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)x64_smem(NP)));
-  SX_CUDA(cudaFuncSetAttribute(k_x_op64_multi<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  SX_CUDA(cudaFuncSetAttribute((k_x_op64_multi<NP, PK>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)x64_smem(NP)));
-  SX_CUDA(cudaFuncSetAttribute(k_cg_multi<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)cg_smem(NP, MX_EP)));
-  SX_CUDA(cudaFuncSetAttribute(k_cg_multi<NP>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  SX_CUDA(cudaFuncSetAttribute((k_cg_multi<NP, PK>), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)cg_smem(NP, PK ? MX_EP : 1)));
+  SX_CUDA(cudaFuncSetAttribute((k_cg_multi<NP, PK>), cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   return SX_OK;
 }
 
@@ -1518,14 +1559,14 @@ int mixed_solve_multi(std::vector<MxItem> &items, MxBatch &B, bool rebuild, doub
     for (int i = 0; i < n; i++) B.order[i] = i;
     std::stable_sort(B.order.begin(), B.order.end(),
                      [&](int a, int b) { return items[a].M.np < items[b].M.np; });
+    std::vector<ChunkMember> cm;
+    for (int m : B.order) cm.push_back({items[m].M.np, items[m].M.nel, items[m].nz});
+    const std::vector<int> lps = chunk_planes(cm);
     std::vector<MxMember> mem(n);
     size_t ntot = 0;
     for (int m = 0; m < n; m++) {
       MxItem &it = items[B.order[m]];
-      SX_TRY(setup(it.M, *it.W, it.groups, it.nz, it.num_modes, st));
-      int attr_rc = SX_OK;
-      SX_NP_SWITCH_M(it.M.np, (attr_rc = set_smem_attrs_multi<N_>()));
-      SX_TRY(attr_rc);
+      SX_TRY(setup(it.M, *it.W, it.groups, it.nz, lps[m], it.num_modes, st));
       bind_params(it.M, *it.W, it.nz, it.u, it.f, it.bc, it.stride);
       B.noff.push_back(ntot);
       ntot += 2 * (size_t)it.W->PP;
@@ -1557,6 +1598,9 @@ int mixed_solve_multi(std::vector<MxItem> &items, MxBatch &B, bool rebuild, doub
       }
       c.te = te.back();
       c.tn = tn.back();
+      int attr_rc = SX_OK;
+      SX_PACKED(c.ep > 1, SX_NP_SWITCH_M(c.np, (attr_rc = set_smem_attrs_multi<N_, PK_>())));
+      SX_TRY(attr_rc);
       tiles.insert(tiles.end(), te.begin(), te.end());
       tiles.insert(tiles.end(), tn.begin(), tn.end());
     }
@@ -1602,7 +1646,8 @@ int mixed_solve_multi(std::vector<MxItem> &items, MxBatch &B, bool rebuild, doub
   }
   if (rounds > max_refine) rounds = max_refine;
   SX_TRY(per_class(B, st, [&](const MxBatch::Class &c, cudaStream_t s) {
-    SX_NP_SWITCH_M(c.np, (k_x_unpack_multi<N_><<<c.te, 256, 0, s>>>(class_table(B, c, 0))));
+    const MxTable Te = class_table(B, c, 0);
+    SX_PACKED(c.ep > 1, SX_NP_SWITCH_M(c.np, (k_x_unpack_multi<N_, PK_><<<c.te, 256, 0, s>>>(Te))));
     SX_CUDA(cudaGetLastError());
     return SX_OK;
   }));

@@ -1,7 +1,9 @@
 """GPU parity of the mixed form for every way its lanes are filled: 32, 16 or 8
 planes a chunk, one chunk and several, element counts that leave the last
 group of a block short, straight and curved elements side by side, alone and
-in a multi-mesh batch; against the oracle (1e-10, the mixed form's bar)."""
+in a multi-mesh batch; against the oracle (1e-10, the mixed form's bar).
+Blocks hold several elements only where 32 planes a chunk would give an SM more
+of them, so the meshes that are to be packed have more than 148 elements."""
 import numpy as np
 import pytest
 
@@ -49,9 +51,12 @@ def _check(m, nz, f, bc, lam, u):
 
 SIZES = [(1, 1, 1, 5, "D"), (1, 3, 3, 3, "D"), (2, 3, 3, 4, "N"), (8, 5, 1, 12, "D"), (10, 3, 3, 6, "D"),
          (16, 3, 5, 11, "N"), (18, 5, 1, 7, "D"), (24, 3, 3, 9, "N"), (32, 5, 1, 5, "D"), (34, 3, 3, 5, "D")]
+#: 8, 8, 8, 16, 16, 8, 8, 8 planes a chunk, and 16 at the lowest order
+PACKED = [(1, 19, 9, 5, "D"), (2, 19, 9, 4, "N"), (8, 19, 9, 12, "D"), (10, 17, 9, 6, "D"), (16, 17, 11, 11, "N"),
+          (18, 19, 9, 7, "D"), (24, 19, 9, 9, "N"), (34, 13, 13, 5, "D"), (10, 17, 9, 3, "D")]
 
 
-@pytest.mark.parametrize("nz,nx,ny,np_,walls", SIZES)
+@pytest.mark.parametrize("nz,nx,ny,np_,walls", SIZES + PACKED)
 def test_lane_layouts_match_oracle(sx, nz, nx, ny, np_, walls):
     import torch
     m = _mesh(nx, ny, np_, walls)
@@ -66,10 +71,11 @@ def test_lane_layouts_match_oracle(sx, nz, nx, ny, np_, walls):
     _check(m, nz, f, bc, lam, u.cpu().numpy())
 
 
-def test_lane_layouts_in_one_batch(sx):
+@pytest.mark.parametrize("sizes", [SIZES, SIZES + PACKED], ids=["wide", "packed"])
+def test_lane_layouts_in_one_batch(sx, sizes):
     import torch
     B, members, probs = sx.Batch(), [], []
-    for nz, nx, ny, _, walls in SIZES:  # one order: one launch over every layout
+    for nz, nx, ny, _, walls in sizes:  # one order: one launch over every layout
         m = _mesh(nx, ny, 6, walls)
         f, bc, lam = _problem(m, nz, 100 + nz)
         S = sx.ModalMatrixSys(sx.Mesh(m), num_modes=len(lam), method=sx.JACPCG, lambda2_modes=lam,
