@@ -13,7 +13,7 @@
 //     = x.
 // Lengths 2, 4, ..., 64 (config 2 uses 64): one pass, k_z_fwd / k_z_inv; the
 // other lengths up to 512: one pass through shared memory, k_z_fwd_any /
-// k_z_inv_any (256: k_z_fwd_s / k_z_inv_s).
+// k_z_inv_any (256, and 128 on smaller fields: k_z_fwd_s / k_z_inv_s).
 // A thread holds one point's whole z-line in registers: the real transform
 // of length N is a complex FFT of length M = N/2 on z_m = x_2m + i x_2m+1
 // (radix-2, decimation in time, every index a compile-time constant), then
@@ -228,9 +228,10 @@ __global__ void __launch_bounds__(128) k_z_inv(double *__restrict__ data, int np
   }
 }
 
-// Length 256: a block of eight warps takes 32 points (lane = point); the half-length complex sequence z (length M = N/2) of each point
-// lies in shared memory, Zr/Zi[m][32], in natural order.  The complex FFT
-// of length M = M1 M2 runs in four steps with m = M2 m1 + m2 and
+// Lengths 256 and, on smaller fields, 128: a block of eight warps takes 32
+// points (lane = point); the half-length complex sequence z (length M = N/2) of
+// each point lies in shared memory, Zr/Zi[m][32], in natural order.  The
+// complex FFT of length M = M1 M2 runs in four steps with m = M2 m1 + m2 and
 // k = k1 + M1 k2: (1) the M2 FFTs of length M1 over m1, each a warp's, in
 // registers; (2) the twiddles W_M^(m2 k1); (3) the M1 FFTs of length M2
 // over m2, in registers.  Two round trips through shared memory and two
@@ -802,7 +803,7 @@ static bool z_factor(int M, int depth, int rmax, int *radix, int *nst) {
 // share an SM: four at 64 registers and 48 KB, which radices up to 10 allow.
 // Lengths that one radix of up to 12 transforms (M <= 12) take it at three
 // blocks an SM (nz = 24: 48 / 61 us for one stage, 71 / 73 for two); from M =
-// 111 on shared memory allows three, from 145 on one block, then of 16 warps
+// 111 on shared memory allows three; from 145 on one block is taken, of 16 warps
 // with radices up to 16 (nz = 512: 216 / 311 us, 257 / 322 with radices up to 8
 // in 32 warps).
 struct ZVariant {
@@ -868,6 +869,18 @@ static int launch_any(double *d, int nz, int npts, long long stride, int sign, c
   if (v.blocks == 3) return launch_rows<256, 3, 10>(Z, v.rows, d, npts, stride, sign, st);
   return launch_rows<512, 1, 16>(Z, v.rows, d, npts, stride, sign, st);
 }
+
+// Where the radix-2 four-step kernels beat the mixed-radix ones.  At 256 they
+// need one stage less in each direction and fit 3 blocks an SM like them.  At
+// 128 both have two stages: the mixed-radix kernels' stages next to global
+// memory skip a trip through shared memory, which pays once HBM bounds the
+// transform; before that the four-step ones' straight loads come back sooner.
+// Forward / inverse, us, four-step against mixed-radix:
+//   128: 10,000 points 13.1/13.3 and 15.2/15.2, 41,472 25.6/27.5 and 27.8/28.1,
+//        82,944 47.6/50.0 and 47.5/50.0, 200,000 112/124 and 106/119
+//   256: 10,000 points 17.6/19.2 and 24.4/28.7, 82,944 85/98 and 114/142,
+//        200,000 184/221 and 246/318
+static bool four_step_faster(int nz, int npts) { return nz == 256 || (nz == 128 && npts < 80000); }
 
 template <int N>
 static void launch_reg(double *d, int npts, long long stride, int sign, cudaStream_t st) {
@@ -945,9 +958,12 @@ extern "C" int sx_transform_z(double *d_data, int nz, int plane_stride, int npts
   }
   if (nz <= ZN_MAX) {
     // one pass through shared memory, enqueued without waiting
-    if (nz == 256) {  // the radix-2 four-step kernels: 243 / 281 us on 248,000 points, the others' 281 / 328
+    if (four_step_faster(nz, npts)) {
       SX_TRY(ensure_twiddles());
-      SX_TRY(launch_smem<256>(d_data, npts, plane_stride, sign, (cudaStream_t)stream));
+      if (nz == 256)
+        SX_TRY(launch_smem<256>(d_data, npts, plane_stride, sign, (cudaStream_t)stream));
+      else
+        SX_TRY(launch_smem<128>(d_data, npts, plane_stride, sign, (cudaStream_t)stream));
       SX_CUDA(cudaGetLastError());
       return SX_OK;
     }
