@@ -87,3 +87,29 @@ def test_wide_band_equals_narrow(sx):
             sols.append(u)
     for u in sols[1:]:
         assert float((u - sols[0]).norm()) <= 1e-11 * float(sols[0].norm())
+
+
+@pytest.mark.parametrize("nm", [148, 149, 300])
+def test_more_systems_than_sms(sx, nm):
+    """One launch over as many systems as the chip has SMs, and more: the rest
+    wait for a place, in the default schedule and in one of three CTAs a system.
+    Every system against the oracle."""
+    import torch
+
+    from semtex_b200.mesh import rect_mesh
+    m = rect_mesh(5, 4, 7, 0.0, 1.0, 0.0, 1.0, jitter=0.1, seed=4)
+    nz, lam = 2 * nm, np.linspace(40.0, 900.0, nm)
+    f = np.random.default_rng(nm).standard_normal((nz, m.nplane))
+    S = sx.ModalMatrixSys(sx.Mesh(m), num_modes=nm, method=sx.DIRECT, lambda2_modes=lam, betak2_modes=np.zeros(nm))
+    uo, _ = solve_planes(OracleMesh(m), 0.0, 0.0, f, None, lambda2_per_mode=lam)
+    sp = [0] + list(range(2, nz))
+    for cluster in (0, 3):
+        S.tune(band_cluster=cluster)
+        fd = torch.tensor(f, device="cuda")
+        u = torch.zeros_like(fd)
+        torch.cuda.synchronize()
+        S.solve_batched(u.data_ptr(), fd.data_ptr(), 0, nz, m.nplane, sx.FP64)
+        torch.cuda.synchronize()
+        S.status()
+        a, b = u.cpu().numpy()[sp], uo[sp]
+        assert (np.linalg.norm(a - b, axis=1) <= TOL * np.linalg.norm(b, axis=1)).all()

@@ -40,3 +40,25 @@ def test_transform_every_length(nz):
         back = d.cpu().numpy()
         assert np.abs(back[:, :npts] - x[:, :npts]).max() <= 1e-14 * np.abs(x).max()
         assert np.array_equal(back[:, npts:], x[:, npts:])
+
+
+@pytest.mark.parametrize("npts", [79_999, 80_000, 80_033])
+def test_transform_128_on_both_sides_of_its_line(npts):
+    """Length 128 takes other kernels from 80,000 points on."""
+    import torch
+    import semtex_b200 as sx
+    nz = 128
+    x = torch.randn(nz, npts + 6, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    d = x.clone()
+    sx.transform_z(d.data_ptr(), nz, npts + 6, npts, +1)
+    torch.cuda.synchronize()
+    cols = np.r_[0:40, npts - 40:npts]
+    F = np.fft.rfft(x[:, cols].cpu().numpy(), axis=0) / nz
+    want = np.empty((nz, len(cols)))
+    want[0], want[1] = F[0].real, F[nz // 2].real
+    want[2::2], want[3::2] = F[1:nz // 2].real, F[1:nz // 2].imag
+    assert np.abs(d[:, cols].cpu().numpy() - want).max() <= 1e-14 * np.abs(want).max()
+    assert torch.equal(d[:, npts:], x[:, npts:])
+    sx.transform_z(d.data_ptr(), nz, npts + 6, npts, -1)
+    torch.cuda.synchronize()
+    assert float((d - x).abs().max()) <= 1e-14 * float(x.abs().max())
