@@ -674,7 +674,9 @@ int band_sweep_jobs(const Job *djobs, const std::vector<Job> &hjobs, const BandS
   const int C = sc.C;
   const int nj = (int)hjobs.size();
   if (nj == 0) return SX_OK;
-  // one wide band makes it the WIDE kernel for all, which takes any band
+  // one wide band makes it the WIDE kernel for all, which takes any band, and
+  // one cluster size serves all (48 systems of 11 tiles a block column 0.93 ms,
+  // two of 121 tiles 0.80, all in one launch of two CTAs a system 3.55)
   int maxP = 0, J = 0, Wmax = 0;
   for (const Job &j : hjobs) {
     maxP = std::max(maxP, j.P);
@@ -715,7 +717,8 @@ int prepare_band_kernels() {
 int default_lead(int C, int) {
   // the leader's j <= NEAR tiles are its share in clusters of four or more;
   // in smaller ones the ranks would have most of the band to themselves (64
-  // systems, C = 2: half 16.6 ms, a third 17.8, none 20.7; 12 systems, C = 9:
+  // systems, C = 2: half 16.6 ms, a third 17.8, none 20.7; 12 systems of that
+  // band, C = 3: a quarter 8.27, a third 8.89, a fifth 8.81, none 10.0; C = 9:
   // none 3.97, a sixth 6.0)
   return C == 2 ? 2 : C == 3 ? 4 : 0;
 }
@@ -752,8 +755,10 @@ int band_active_clusters(int C, int J, int smax) {
 // with four tiles in flight keeps up with its share of HBM, and shallower
 // rings are slower before they let a larger cluster in (32 systems, 4 CTAs
 // each: depth 4 0.78 ms, 3 0.84, 2 0.96; 5 CTAs at depth 2, in two waves,
-// 1.63).  Where not even one CTA a
-// system is resident, C = 1 at the depth with the most CTAs on the chip.
+// 1.63).  Where not even one CTA a system is resident, which is from 149
+// systems on (the registers allow one CTA an SM), C = 1 at the depth with the
+// most CTAs on the chip: 148 systems of 236 block columns 3.0 ms, 149 4.7, 240
+// 5.2.
 // stages_forced > 0 fixes the depth.
 int pick_cluster(int nj, int cmax, int J, int *stages_out, int stages_forced) {
   int bestC = 0, bestS = BAND_STAGES_MAX, mostS = BAND_STAGES_MAX, most = 0;

@@ -319,13 +319,14 @@ int cg_round_iters(double kratio, double hcon);
 //   factor: nsolve nband^2 flops at 3.9 TFLOP/s (config-2 set-up,
 //           measured), divided by `reuse`, the solves expected per factored
 //           system (0: already factored, no cost).
-// The two streaming rates are calibration constants: k_cg's and
-// k_band_sweep's rates when the rule was set up.  Both kernels are faster
-// now (about 2.7 and 2.8 TB/s); with those rates the rule sends more modes
-// of a serving request to the band, and a request's factorisation, whose
-// block-column steps are latency-bound, costs more than the flop estimate
-// above -- the serving stream ran slower (makespan 7.2-7.7 s against
-// 5.3-7.8 s in an A/B on one box), so the calibrated pair stays.
+// The rates are calibration constants, the kernels' when the rule was set up,
+// and the band is charged whole.  The sweeps now run at about 6 TB/s on the
+// envelope's tiles alone, k_cg at about 3: on a mesh of 32 x 32 elements of
+// order 8 the rule sends 32 mass-dominated modes (lambda2 1e6) to the
+// iterations, 1.8 ms, where the band takes 1.15.  Faster rates were tried when
+// the sweeps ran at 2.8 TB/s, and the serving stream got slower by them
+// (makespan 7.2-7.7 s against 5.3-7.8): a request's factorisation, whose
+// block-column steps are latency-bound, costs more than the flop estimate.
 // A mode whose rounds would exceed CG_ROUND_CAP iterations, or whose CG would
 // need more than max_refine rounds, goes to the band.  iter_floor_s is the
 // least time an FP32 iteration takes whatever its bytes (a launch and, when
