@@ -388,21 +388,23 @@ __global__ void __launch_bounds__(ZW * 32, 3) k_z_inv_s(double *__restrict__ dat
 }
 
 // A kernel's limit on dynamic shared memory is a setting of the current
-// device's copy of it, so every launch sets it (to the same value: callers do
-// not disturb one another).
+// device's copy of it, so every launch of more than the default limit allows
+// (48 KB, with up to 1 KB of tables) sets it, to the kernel's `most`: callers
+// do not disturb one another.
 template <typename K>
-static cudaError_t dynamic_smem(K *kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+static cudaError_t dynamic_smem(K *kernel, size_t bytes, size_t most) {
+  if (bytes <= 47 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
 template <int N>
 static int launch_smem(double *d, int npts, long long stride, int sign, cudaStream_t st) {
   const int grid = (npts + 31) / 32;
   if (sign == 1) {
-    SX_CUDA(dynamic_smem(k_z_fwd_s<N>, (int)zsmem(N)));
+    SX_CUDA(dynamic_smem(k_z_fwd_s<N>, zsmem(N), zsmem(N)));
     k_z_fwd_s<N><<<grid, ZW * 32, zsmem(N), st>>>(d, npts, stride, 1.0 / N);
   } else {
-    SX_CUDA(dynamic_smem(k_z_inv_s<N>, (int)zsmem(N)));
+    SX_CUDA(dynamic_smem(k_z_inv_s<N>, zsmem(N), zsmem(N)));
     k_z_inv_s<N><<<grid, ZW * 32, zsmem(N), st>>>(d, npts, stride);
   }
   return SX_OK;
@@ -851,10 +853,10 @@ static int launch_rows(const ZPlan235 &Z, int rows, double *d, int npts, long lo
   const int grid = (npts + 32 * Z.PG - 1) / (32 * Z.PG);
   const size_t smem = (size_t)Z.PG * Z.M * 512;
   if (sign == 1) {
-    SX_CUDA(dynamic_smem(k_z_fwd_any<NT, MINB, RMAX>, rows * 512));
+    SX_CUDA(dynamic_smem(k_z_fwd_any<NT, MINB, RMAX>, smem, (size_t)rows * 512));
     k_z_fwd_any<NT, MINB, RMAX><<<grid, NT, smem, st>>>(Z, d, npts, stride, 1.0 / Z.N);
   } else {
-    SX_CUDA(dynamic_smem(k_z_inv_any<NT, MINB, RMAX>, rows * 512));
+    SX_CUDA(dynamic_smem(k_z_inv_any<NT, MINB, RMAX>, smem, (size_t)rows * 512));
     k_z_inv_any<NT, MINB, RMAX><<<grid, NT, smem, st>>>(Z, d, npts, stride);
   }
   SX_CUDA(cudaGetLastError());
