@@ -8,7 +8,7 @@ mixed-precision channel: [0,2pi] x [0,1], 64 x 64 quads jittered +-20 %
 (seed 3), N = 10, nz = 128 planes (modes 0..63, 127 planes solved, Nyquist
 skipped), lambda2 log-uniform in [1e-2, 1e4] per mode, Dirichlet walls,
 periodic in x, manufactured solution u = sum_k a_k sin(pi y) cos(kz) cos(3x).
-Every mode is factored (121 GB of band factors, set-up).  A step is one solve
+Every mode is factored (119.5 GB of band factors, set-up).  A step is one solve
 of every plane of every mode.
 
 Metric: Helmholtz DoF-solves/s (unique nodes per plane x planes solved /
@@ -326,7 +326,7 @@ def run_ours(args, rank, world):
         f_work.copy_(f_src)  # the solve overwrites its forcing (src/field.cpp:525-526)
 
     # 256 MB written between timed steps: evicts the 126 MB L2 (the step's
-    # working set, 121 GB of factors, is far above L2 anyway)
+    # working set, 119.5 GB of factors, is far above L2 anyway)
     flush = torch.empty(64 << 20, dtype=torch.float32, device=dev)
 
     def timed(fn, k, wu):
@@ -1140,7 +1140,7 @@ def run_profile(args):
     band3: band sweeps of two config-3 systems (the full 64 x 64, N = 10
            mesh, modes 0 and 1: 2.9 GB of factors, the config-3 band)
     solve3: `steps` batched FP64 solves of config 3 at full size (every
-           mode factored, 121 GB), for a launch list (one-pass metrics only)
+           mode factored, 119.5 GB), for a launch list (one-pass metrics only)
     mixed: the mixed-precision batched form on the full config-2 workload
            with Jacobi systems only (no band factors, ~0.3 GB resident)
     transform: the z-direction transform of the config-2 field (nz = 64,

@@ -250,15 +250,14 @@ SX_API int sx_field_solve_batched_host(sx_modal modal, double *u, const double *
  *                         for every mode, 2 = band Cholesky for every
  *                         factored mode
  *   SX_TUNE_BAND_STAGES   band-sweep tiles in flight per CTA, 1..4 (auto:
- *                         4, or 2 or 1 when that lets a larger cluster
- *                         stay resident -- two CTAs then share an SM)
+ *                         the most with which every system's cluster is
+ *                         resident)
  *   SX_TUNE_BAND_LEAD     the cluster leader's share of the band tiles off
  *                         the critical path: K in 2..64 gives it the last of
  *                         every K such tiles of a block column (worked on
  *                         while it waits for the other CTAs' partial sums);
- *                         1 = none (it keeps only the tile next to the
- *                         diagonal and the diagonal block's inverse);
- *                         <= 0 = the default
+ *                         1 = none (it keeps only the two tiles next to
+ *                         the diagonal); <= 0 = the default
  *   SX_TUNE_HOST_CHUNK    Fourier modes per chunk of the host-buffer
  *                         pipeline of sx_field_solve_batched_host (each
  *                         chunk is copied up, solved and copied back on
@@ -434,8 +433,9 @@ SX_API int sx_numbering_write(const char *path, const char *fields, int nset, co
  *                  every member meets tol_rel;
  *   SX_FP64 (and the modes SX_MIXED_FP32 routes to the band Cholesky)
  *                  one band-sweep launch covers every member's systems.
- * The launch sequence is captured as CUDA graphs and replayed while the set
- * of members and their buffers stay the same.  A modal system may appear
+ * The launch sequence is captured as CUDA graphs (the FP64 one on the second
+ * call with given members and buffers) and replayed while the set of members
+ * and their buffers stay the same.  A modal system may appear
  * once per call.  stats, when non-null, has `count` entries.  The batch
  * object holds the tables and graphs; it does not own the modal systems. */
 typedef struct sx_batch_s *sx_batch;
