@@ -119,7 +119,7 @@ static bool same_constants(const System &S, double lambda2, double betak2, int m
 namespace sx {
 
 // What a band system may take of the pool beyond POOL_KEEP (modal_populate).
-constexpr uint64_t POOL_SPARE = uint64_t(128) << 20;
+constexpr uint64_t POOL_SPARE = uint64_t(192) << 20;
 
 // Device memory of one band system on a mesh.
 static size_t direct_bytes(const sx_mesh_s &M) {
@@ -181,10 +181,10 @@ int modal_populate(sx_modal_s &M, const double *lam, const double *bk2, const Sy
   // Band systems live in the pool while that is the cheaper way to make and
   // drop them.  From the pool, what is above POOL_KEEP is unmapped at the next
   // wait and mapped again for the next systems, some 14 ms a GB; by cudaMalloc
-  // and cudaFree a system's five buffers take about 2 ms whatever their size.
-  // Built and dropped (pool / cudaMalloc): 32 systems of 0.17 GB 35 / 98 ms;
-  // 4 of 1.6 GB 100 / 78; 12 of 1.6 GB 340 / 190; 48 of 1.6 GB 1610 / 696; 16
-  // of 6.6 GB 2660 / 1480; at the line, 129 of 0.17 GB, 270 / 271.
+  // and cudaFree a system's five buffers take 2 to 3 ms whatever their size.
+  // Built and dropped (pool / cudaMalloc): 32 systems of 0.17 GB 35 / 98 ms, 129
+  // of them 270 / 271; 12 of 0.49 GB 104 / 119; 4 of 1.6 GB 100 / 78, 12 of them
+  // 340 / 190, 48 of them 1610 / 696; 16 of 6.6 GB 2660 / 1480.
   if (direct.size() * direct_bytes(*M.mesh) <= POOL_KEEP + direct.size() * POOL_SPARE)
     for (System *S : direct) SX_TRY(device_pool(M.mesh->device, &S->pool));
   SX_TRY(systems_build_direct(direct, st));

@@ -9,6 +9,7 @@
 #include <cstdarg>
 #include <cstring>
 #include <algorithm>
+#include <chrono>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -296,6 +297,7 @@ int mesh_kratio(const sx_mesh_desc *d, double *out) {
 // POOL_KEEP bytes of freed memory stay mapped for the next ones.
 static std::mutex pool_mu;
 static std::map<int, cudaMemPool_t> pools;
+static std::map<int, std::chrono::steady_clock::time_point> looked;  // device_pool_release's last look
 
 int sx::device_pool(int device, cudaMemPool_t *out) {
   std::lock_guard<std::mutex> lk(pool_mu);
@@ -326,7 +328,10 @@ void sx::device_pool_trim() {
 }
 
 void sx::device_pool_release(int device) {
-  constexpr uint64_t WORTH = uint64_t(64) << 20;  // idle memory below this is not looked at
+  // idle memory below this is not looked at, nor the device twice in this time
+  // (the look takes 65 us, as much as a small system's buffers)
+  constexpr uint64_t WORTH = uint64_t(64) << 20;
+  constexpr std::chrono::milliseconds AGAIN(20);
   std::lock_guard<std::mutex> lk(pool_mu);
   auto it = pools.find(device);
   if (it == pools.end()) return;
@@ -335,6 +340,10 @@ void sx::device_pool_release(int device) {
       cudaMemPoolGetAttribute(it->second, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
       reserved < used + WORTH)
     return;
+  const auto now = std::chrono::steady_clock::now();
+  auto last = looked.find(device);
+  if (last != looked.end() && now - last->second < AGAIN) return;
+  looked[device] = now;
   size_t fr = 0, tot = 0;
   if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr < 2 * POOL_KEEP) cudaMemPoolTrimTo(it->second, 0);
 }
