@@ -86,33 +86,37 @@ bool factors_235(int n) {
 
 }  // namespace
 
-// exp(-2 pi i t / TWN), t = 0 .. TWN/2, from the host's cos / sin in FP64;
-// a length-L stage uses t = j * (TWN / L).
+// exp(-2 pi i t / TWN), t = 0 .. TWN/2; a length-L stage uses t = j * (TWN / L).
+// Part of the module's image, so that every device and context has it and the
+// first call may be a captured one.  (As a kernel parameter, which the mixed-
+// radix kernels' table of any length has to be, 4 KB cost a short launch 2.5
+// us.)
 constexpr int TWN = 256;
-__constant__ double c_twr[TWN / 2 + 1], c_twi[TWN / 2 + 1];
-
-static int ensure_twiddles() {
-  static std::mutex mu;
-  static std::vector<char> done(256, 0);
-  int dev = 0;
-  SX_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  if (dev < 256 && done[dev]) return SX_OK;
-  double wr[TWN / 2 + 1], wi[TWN / 2 + 1];
-  for (int t = 0; t <= TWN / 2; t++) {
-    const double a = 2.0 * M_PI * t / TWN;
-    wr[t] = std::cos(a);
-    wi[t] = -std::sin(a);
+// cos(2 pi t / 256), t = 0 .. 64, correctly rounded
+constexpr double QUARTER[TWN / 4 + 1] = {
+    1.0, 0.9996988186962042, 0.9987954562051724, 0.9972904566786902, 0.9951847266721969,
+    0.99247953459871, 0.989176509964781, 0.9852776423889412, 0.9807852804032304, 0.9757021300385286,
+    0.970031253194544, 0.9637760657954398, 0.9569403357322088, 0.9495281805930367, 0.9415440651830208,
+    0.9329927988347388, 0.9238795325112867, 0.9142097557035307, 0.9039892931234433, 0.8932243011955153,
+    0.881921264348355, 0.8700869911087115, 0.8577286100002721, 0.8448535652497071, 0.8314696123025452,
+    0.8175848131515837, 0.8032075314806449, 0.7883464276266062, 0.773010453362737, 0.7572088465064846,
+    0.7409511253549591, 0.7242470829514669, 0.7071067811865476, 0.6895405447370669, 0.6715589548470184,
+    0.6531728429537768, 0.6343932841636455, 0.6152315905806268, 0.5956993044924334, 0.5758081914178453,
+    0.5555702330196022, 0.5349976198870973, 0.5141027441932218, 0.49289819222978404, 0.47139673682599764,
+    0.4496113296546066, 0.4275550934302821, 0.40524131400498986, 0.3826834323650898, 0.35989503653498817,
+    0.33688985339222005, 0.31368174039889146, 0.2902846772544624, 0.26671275747489837, 0.2429801799032639,
+    0.2191012401568698, 0.19509032201612828, 0.17096188876030122, 0.14673047445536175, 0.1224106751992162,
+    0.0980171403295606, 0.07356456359966743, 0.049067674327418015, 0.024541228522912288, 0.0};
+struct Twiddles {
+  double c[TWN / 2 + 1], s[TWN / 2 + 1];
+  constexpr Twiddles() : c(), s() {
+    for (int t = 0; t <= TWN / 2; t++) {
+      c[t] = t <= TWN / 4 ? QUARTER[t] : -QUARTER[TWN / 2 - t];
+      s[t] = t <= TWN / 4 ? -QUARTER[TWN / 4 - t] : -QUARTER[t - TWN / 4];
+    }
   }
-  wr[TWN / 4] = 0.0;  // exact at the quarter and half turns
-  wi[TWN / 4] = -1.0;
-  wr[TWN / 2] = -1.0;
-  wi[TWN / 2] = 0.0;
-  SX_CUDA(cudaMemcpyToSymbol(c_twr, wr, sizeof(wr)));
-  SX_CUDA(cudaMemcpyToSymbol(c_twi, wi, sizeof(wi)));
-  if (dev < 256) done[dev] = 1;
-  return SX_OK;
-}
+};
+__constant__ Twiddles c_tw;  // constant-initialised
 
 constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n / 2); }
 constexpr int bitrev(int v, int bits) {
@@ -136,7 +140,7 @@ struct FftStage {
 #pragma unroll
       for (int j = 0; j < LEN / 2; j++) {
         const int t = j * (TWN / LEN);
-        const double wr = c_twr[t], wi = INV ? -c_twi[t] : c_twi[t];
+        const double wr = c_tw.c[t], wi = INV ? -c_tw.s[t] : c_tw.s[t];
         const int a = i + j, b = i + j + LEN / 2;
         const double vr = re[b] * wr - im[b] * wi, vi = re[b] * wi + im[b] * wr;
         re[b] = re[a] - vr;
@@ -181,7 +185,7 @@ __global__ void __launch_bounds__(128) k_z_fwd(double *__restrict__ data, int np
     const double er = 0.5 * (re[k] + yr), ei = 0.5 * (im[k] + yi);
     const double orr = 0.5 * (im[k] - yi), oi = -0.5 * (re[k] - yr);  // (Z_k - conj Z_{M-k}) / 2i
     const int t = k * (TWN / N);
-    const double wr = c_twr[t], wi = c_twi[t];
+    const double wr = c_tw.c[t], wi = c_tw.s[t];
     data[(2 * k) * stride + p] = (er + (orr * wr - oi * wi)) * scale;
     data[(2 * k + 1) * stride + p] = (ei + (orr * wi + oi * wr)) * scale;
   }
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(128) k_z_inv(double *__restrict__ data, int np
       const double er = 0.5 * (xr + cr), ei = 0.5 * (xi + ci);
       const double dr = 0.5 * (xr - cr), di = 0.5 * (xi - ci);
       const int t = q * (TWN / N);
-      const double wr = c_twr[t], wi = -c_twi[t];  // conj W^q
+      const double wr = c_tw.c[t], wi = -c_tw.s[t];  // conj W^q
       const double orr = dr * wr - di * wi, oi = dr * wi + di * wr;
       re[bitrev(q, LB)] = er - oi;  // E + i O
       im[bitrev(q, LB)] = ei + orr;
@@ -254,8 +258,8 @@ __device__ __forceinline__ void twiddle(int e, bool inv, double &wr, double &wi)
   e &= M - 1;
   const bool neg = e >= M / 2;
   const int t = (neg ? e - M / 2 : e) * (TWN / M);
-  wr = neg ? -c_twr[t] : c_twr[t];
-  wi = neg ? -c_twi[t] : c_twi[t];
+  wr = neg ? -c_tw.c[t] : c_tw.c[t];
+  wi = neg ? -c_tw.s[t] : c_tw.s[t];
   if (inv) wi = -wi;
 }
 
@@ -336,7 +340,7 @@ __global__ void __launch_bounds__(ZW * 32, 3) k_z_fwd_s(double *__restrict__ dat
       const double er = 0.5 * (ar + yr), ei = 0.5 * (ai + yi);
       const double orr = 0.5 * (ai - yi), oi = -0.5 * (ar - yr);
       const int t = q * (TWN / N);
-      const double wr = c_twr[t], wi = c_twi[t];
+      const double wr = c_tw.c[t], wi = c_tw.s[t];
       data[(2 * q) * stride + p] = (er + (orr * wr - oi * wi)) * scale;
       data[(2 * q + 1) * stride + p] = (ei + (orr * wi + oi * wr)) * scale;
     }
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(ZW * 32, 3) k_z_inv_s(double *__restrict__ dat
       const double er = 0.5 * (xr + cr), ei = 0.5 * (xi + ci);
       const double dr = 0.5 * (xr - cr), di = 0.5 * (xi - ci);
       const int t = q * (TWN / N);
-      const double wr = c_twr[t], wi = -c_twi[t];
+      const double wr = c_tw.c[t], wi = -c_tw.s[t];
       const double orr = dr * wr - di * wi, oi = dr * wi + di * wr;
       Zr[q * 32 + lane] = er - oi;
       Zi[q * 32 + lane] = ei + orr;
@@ -879,10 +883,10 @@ static int launch_any(double *d, int nz, int npts, long long stride, int sign, c
 // transform; before that the four-step ones' straight loads come back sooner.
 // Forward / inverse, us, four-step against mixed-radix:
 //   128: 10,000 points 13.1/13.3 and 15.2/15.2, 41,472 25.6/27.5 and 27.8/28.1,
-//        82,944 47.6/50.0 and 47.5/50.0, 200,000 112/124 and 106/119
+//        82,944 48.7/51.6 and 51.6/54.0, 200,000 112/124 and 106/119
 //   256: 10,000 points 17.6/19.2 and 24.4/28.7, 82,944 85/98 and 114/142,
 //        200,000 184/221 and 246/318
-static bool four_step_faster(int nz, int npts) { return nz == 256 || (nz == 128 && npts < 80000); }
+static bool four_step_faster(int nz, int npts) { return nz == 256 || (nz == 128 && npts < 100000); }
 
 template <int N>
 static void launch_reg(double *d, int npts, long long stride, int sign, cudaStream_t st) {
@@ -945,7 +949,6 @@ extern "C" int sx_transform_z(double *d_data, int nz, int plane_stride, int npts
   }
   if (nz <= 64 && (nz & (nz - 1)) == 0) {
     // one pass in registers, enqueued without waiting (no workspace)
-    SX_TRY(ensure_twiddles());
     cudaStream_t st = (cudaStream_t)stream;
     switch (nz) {
       case 2: launch_reg<2>(d_data, npts, plane_stride, sign, st); break;
@@ -961,8 +964,7 @@ extern "C" int sx_transform_z(double *d_data, int nz, int plane_stride, int npts
   if (nz <= ZN_MAX) {
     // one pass through shared memory, enqueued without waiting
     if (four_step_faster(nz, npts)) {
-      SX_TRY(ensure_twiddles());
-      if (nz == 256)
+        if (nz == 256)
         SX_TRY(launch_smem<256>(d_data, npts, plane_stride, sign, (cudaStream_t)stream));
       else
         SX_TRY(launch_smem<128>(d_data, npts, plane_stride, sign, (cudaStream_t)stream));

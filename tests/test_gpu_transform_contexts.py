@@ -45,7 +45,7 @@ for a, b in ((X, want), (Y, want), (Z, x)):
 """
 
 
-@pytest.mark.parametrize("nz", [24, 96, 240, 512])  # one length of each kernel variant
+@pytest.mark.parametrize("nz", [24, 96, 128, 240, 256, 512])  # one length of each kernel variant
 def test_second_context(nz):
     r = subprocess.run([sys.executable, "-c", SCRIPT, str(nz)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]

@@ -42,9 +42,9 @@ def test_transform_every_length(nz):
         assert np.array_equal(back[:, npts:], x[:, npts:])
 
 
-@pytest.mark.parametrize("npts", [79_999, 80_000, 80_033])
+@pytest.mark.parametrize("npts", [99_999, 100_000, 100_033])
 def test_transform_128_on_both_sides_of_its_line(npts):
-    """Length 128 takes other kernels from 80,000 points on."""
+    """Length 128 takes other kernels from 100,000 points on."""
     import torch
     import semtex_b200 as sx
     nz = 128
@@ -62,3 +62,30 @@ def test_transform_128_on_both_sides_of_its_line(npts):
     sx.transform_z(d.data_ptr(), nz, npts + 6, npts, -1)
     torch.cuda.synchronize()
     assert float((d - x).abs().max()) <= 1e-14 * float(x.abs().max())
+
+
+@pytest.mark.parametrize("nz", [96, 128, 256])
+def test_first_transform_inside_a_capture(nz):
+    """Nothing is set up on the device before a length's first call, so that it
+    may be a captured one.  In a process of its own: it is the first."""
+    import subprocess
+    import sys
+    script = f"""
+import numpy as np, torch
+import semtex_b200 as sx
+nz, n = {nz}, 500
+x = torch.randn(nz, n, dtype=torch.float64, device="cuda")
+d, st, g = x.clone(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+torch.cuda.synchronize()
+with torch.cuda.graph(g, stream=st, capture_error_mode="thread_local"):
+    sx.transform_z(d.data_ptr(), nz, n, n, 1, stream=st.cuda_stream)
+g.replay()
+torch.cuda.synchronize()
+F = np.fft.rfft(x.cpu().numpy(), axis=0) / nz
+X = d.cpu().numpy()
+assert np.abs(X[0] - F[0].real).max() <= 1e-14 * np.abs(F).max()
+assert np.abs(X[2::2] - F[1:-1].real).max() <= 1e-14 * np.abs(F).max()
+assert np.abs(X[3::2] - F[1:-1].imag).max() <= 1e-14 * np.abs(F).max()
+"""
+    r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
